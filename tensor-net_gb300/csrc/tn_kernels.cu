@@ -1,8 +1,6 @@
 // tn_kernels.cu -- kernels of the trajectory engine and their launchers.
 //
-//  k_run        persistent executor: CTAs pull work items (one trajectory's
-//               instruction list each) from an atomic counter and run them with
-//               the device routines of tn_device.cuh.
+//  (k_run, the persistent executor, is in tn_run.cuh)
 //  k_compile    builds every trajectory's instruction list for one brickwork
 //               layer on the device (apply_bilayer, circuit.rs:624-659 ->
 //               apply_meas_prob_layer control flow, mps.rs:2206-2252).
@@ -10,144 +8,9 @@
 //               mps.rs:370-391).
 #include "tn_device.cuh"
 #include "tn_internal.h"
-#include "tn_tc.cuh"
+#include "tn_queue.cuh"
 
 namespace tn {
-
-__device__ __forceinline__ unsigned long long global_ns() { return tc::global_ns(); }
-
-__device__ __forceinline__ int load_acquire(const int *p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void store_release(int *p, int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Appends the sweep item of listed trajectory i to the pushed queue (one thread).
-__device__ void push_sweep(Item *dyn, int *tail, const Item *sweeps, int i) {
-  const int slot = atomicAdd(tail, 1);
-  const Item s = sweeps[i];
-  dyn[slot].traj = s.traj;
-  dyn[slot].off = s.off;
-  dyn[slot].len = s.len;
-  store_release(&dyn[slot].aux, 1);
-}
-
-// Static schedule (la.rem == nullptr): items[0, count) in counter order.
-// Dependency-driven schedule: a CTA takes a pushed sweep item when one is
-// ready (claimed by compare-and-swap on the sweep head below the push tail),
-// else the next gate item; once the gate items are gone it claims the next
-// sweep slot and waits (bounded by kQueueWaitNs) for its push.  Every pushed
-// item depends only on gate items already taken by running CTAs, so the
-// waits end; a wait that runs out sets qerr and the CTA moves on.
-template <typename T, int NT, int W>
-__global__ void __launch_bounds__(NT, 1) k_run(LaunchArgs la, int sortP, int ws_cap) {
-  extern __shared__ __align__(256) unsigned char smem[];
-  __shared__ Item s_item;
-  __shared__ int s_kind;  // 0 done, 1 gate / static item, 2 pushed sweep item, 3 skip
-  __shared__ uint64_t s_bar;
-  __shared__ uint32_t s_tmem;
-  Smem<T, W> sm(smem, sortP);
-  Work<T> wk = make_work<T>(reinterpret_cast<unsigned char *>(la.ws) + size_t(blockIdx.x) * la.ws_stride, ws_cap);
-  const bool dd = la.rem != nullptr;
-  // float: one 128 x 256 FP32 accumulator tile (theta and recovery GEMMs);
-  // double-float: eight 128 x 64 level accumulators of the tensor-core update
-  constexpr bool kTC = sizeof(T) == 4 || std::is_same<T, ::tn::dd>::value;
-  constexpr uint32_t kTmemCols = sizeof(T) == 4 ? 256 : 512;
-  if constexpr (kTC) {
-    // the executor owns kTmemCols tensor-memory columns for its whole
-    // life (one CTA per SM); released below on the kernel's only exit path
-    if ((threadIdx.x >> 5) == 0) {
-      tc::tmem_alloc(&s_tmem, kTmemCols);
-      tc::tmem_relinquish();
-    }
-    if (threadIdx.x == 0) {
-      tc::mbar_init(&s_bar, 1);
-      tc::mbar_fence_init();
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    sm.tmem = s_tmem;
-    sm.bar = &s_bar;
-    sm.phase = 0;
-    sm.tc = la.theta_simt == 0;
-  }
-  for (;;) {
-    if (threadIdx.x == 0) {
-      const int G = la.nitems_dev ? *la.nitems_dev : la.nitems;
-      int kind = 0, slot_i = -1;
-      if (dd) {
-        // A pushed sweep item that is already there goes first: the sweeps
-        // are the serial chains that bound the launch, the gate items are
-        // independent filler.
-        int h = *reinterpret_cast<volatile int *>(la.dyn_head);
-        while (h < *reinterpret_cast<volatile int *>(la.dyn_tail)) {
-          const int prev = atomicCAS(la.dyn_head, h, h + 1);
-          if (prev == h) {
-            slot_i = h;
-            break;
-          }
-          h = prev;
-        }
-      }
-      if (slot_i < 0) {
-        const int it = atomicAdd(la.counter, 1);
-        if (it < G) {
-          s_item = la.items[it];
-          kind = 1;
-        } else if (dd) {
-          // no gate left: claim the next sweep slot and wait for its push
-          const int h = atomicAdd(la.dyn_head, 1);
-          if (h < la.nsweeps) slot_i = h;
-        }
-      }
-      if (slot_i >= 0) {
-        Item *slot = la.dyn + slot_i;
-        const unsigned long long t0 = global_ns();
-        const unsigned long long limit = la.queue_wait_ns ? la.queue_wait_ns : kQueueWaitNs;
-        kind = 2;
-        while (load_acquire(&slot->aux) == 0) {
-          if (global_ns() - t0 > limit) {
-            atomicExch(la.qerr, 1);
-            kind = 3;
-            break;
-          }
-          __nanosleep(200);
-        }
-        if (kind == 2) s_item = Item{slot->traj, slot->off, slot->len, 0};
-      }
-      s_kind = kind;
-    }
-    __syncthreads();
-    const int kind = s_kind;
-    const Item item = s_item;
-    __syncthreads();
-    if (kind == 0) break;
-    if (kind == 3) continue;
-    if (kind == 2) __threadfence();  // acquire side for every thread of the CTA
-    run_program<T, NT, W>(la, (dd && kind == 1) ? la.gprog : la.prog, item, wk, sm);
-    if (dd && kind == 1) {
-      __threadfence();  // this thread's writes of the gate's result, visible device-wide
-      __syncthreads();
-      if (threadIdx.x == 0 && atomicSub(la.rem + item.aux, 1) == 1) {
-        __threadfence();
-        push_sweep(la.dyn, la.dyn_tail, la.sweeps, item.aux);
-      }
-    }
-  }
-  if constexpr (kTC) {
-    tc::fence_before_sync();
-    __syncthreads();
-    if ((threadIdx.x >> 5) == 0) {
-      tc::fence_after_sync();
-      tc::tmem_dealloc(sm.tmem, kTmemCols);
-    }
-  }
-}
 
 __global__ void k_reset(TrajDev *trajs, const int *list, int count, int prec) {
   const int t = list[blockIdx.x];
@@ -401,66 +264,31 @@ __global__ void k_compile_dd(const TrajDev *trajs, const int *list, int nt, cons
 }
 
 // ------------------------------------------------------------- launchers
-// Dynamic shared memory limit configured for k_run<T> on the current
-// device (raised on demand; set when a handle or batch is created, so that
-// a stream capture of a launch finds it already in place).
-template <typename T, int NT, int W>
-static cudaError_t ensure_run_smem(size_t smem) {
-  static int configured[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int &have = configured[dev & 63];
-  if (int(smem) > have) {
-    cudaError_t e = cudaFuncSetAttribute(k_run<T, NT, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e != cudaSuccess) return e;
-    have = int(smem);
-  }
-  return cudaSuccess;
-}
-
-template <typename T, int NT, int W>
-static cudaError_t launch_run_t(const LaunchArgs &la, int grid, int sortP, int ws_cap, cudaStream_t st) {
-  const size_t smem = SmemLayout<T, W>::total(sortP);
-  cudaError_t e = ensure_run_smem<T, NT, W>(smem);
-  if (e != cudaSuccess) return e;
-  k_run<T, NT, W><<<grid, NT, smem, st>>>(la, sortP, ws_cap);
-  return cudaGetLastError();
-}
+#define TN_DECLARE_RUN(SUFFIX)                                                                              \
+  cudaError_t launch_run_##SUFFIX(const LaunchArgs &la, int grid, int sortP, int ws_cap, cudaStream_t st);  \
+  size_t run_smem_##SUFFIX(int sortP);                                                                      \
+  size_t run_work_##SUFFIX(int cap);                                                                        \
+  int run_blocks_##SUFFIX(int sortP);
+TN_DECLARE_RUN(f32)
+TN_DECLARE_RUN(f64)
+TN_DECLARE_RUN(df)
 
 cudaError_t launch_run(int prec, const LaunchArgs &la, int grid, int sortP, int ws_cap, cudaStream_t st) {
-  if (prec == 0) return launch_run_t<double, kThreads, kBlockW>(la, grid, sortP, ws_cap, st);
-  if (prec == 2) return launch_run_t<dd, kThreads, kBlockW>(la, grid, sortP, ws_cap, st);
-  return launch_run_t<float, kThreads, kBlockW>(la, grid, sortP, ws_cap, st);
+  if (prec == 0) return launch_run_f64(la, grid, sortP, ws_cap, st);
+  if (prec == 2) return launch_run_df(la, grid, sortP, ws_cap, st);
+  return launch_run_f32(la, grid, sortP, ws_cap, st);
 }
 
 size_t run_smem_bytes(int prec, int sortP) {
-  if (prec == 0) return SmemLayout<double, kBlockW>::total(sortP);
-  if (prec == 2) return SmemLayout<dd, kBlockW>::total(sortP);
-  return SmemLayout<float, kBlockW>::total(sortP);
+  return prec == 0 ? run_smem_f64(sortP) : (prec == 2 ? run_smem_df(sortP) : run_smem_f32(sortP));
 }
 
 size_t run_work_bytes(int prec, int cap) {
-  if (prec == 0) return work_bytes<double>(cap);
-  if (prec == 2) return work_bytes<dd>(cap);
-  return work_bytes<float>(cap);
+  return prec == 0 ? run_work_f64(cap) : (prec == 2 ? run_work_df(cap) : run_work_f32(cap));
 }
 
 int run_blocks_per_sm(int prec, int sortP) {
-  int nb = 0;
-  const size_t smem = run_smem_bytes(prec, sortP);
-  cudaError_t e;
-  if (prec == 0) {
-    ensure_run_smem<double, kThreads, kBlockW>(smem);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_run<double, kThreads, kBlockW>, kThreads, smem);
-  } else if (prec == 2) {
-    ensure_run_smem<dd, kThreads, kBlockW>(smem);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_run<dd, kThreads, kBlockW>, kThreads, smem);
-  } else {
-    ensure_run_smem<float, kThreads, kBlockW>(smem);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_run<float, kThreads, kBlockW>, kThreads, smem);
-  }
-  if (e != cudaSuccess || nb < 1) nb = 1;
-  return nb;
+  return prec == 0 ? run_blocks_f64(sortP) : (prec == 2 ? run_blocks_df(sortP) : run_blocks_f32(sortP));
 }
 
 cudaError_t launch_reset(TrajDev *trajs, const int *list, int count, int prec, cudaStream_t st) {
