@@ -182,6 +182,17 @@ __device__ __forceinline__ cpx<dd> acc_fin<dd>(const cdacc &acc) {
   return mkc<dd>(dd_norm(acc.x.hi, acc.x.lo), dd_norm(acc.y.hi, acc.y.lo));
 }
 
+// Renormalises a raw double-float accumulator: its low part collects the
+// errors of the terms so far and rounds relative to itself, so long sums bring
+// it back below half an ulp of the high part every few terms (n terms then err
+// by about sqrt(n) 2^-50 of the largest instead of n 2^-50).
+template <typename A>
+__device__ __forceinline__ void acc_renorm(A &) {}
+__device__ __forceinline__ void acc_renorm(cdacc &a) {
+  fast_two_sum(a.x.hi, a.x.lo, a.x.hi, a.x.lo);
+  fast_two_sum(a.y.hi, a.y.lo, a.y.hi, a.y.lo);
+}
+
 // --------------------------------------------------------- block helpers
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double *red) {
@@ -256,6 +267,9 @@ __device__ __forceinline__ int block_min_int(int v, int *red) {
 // the block pair resident in shared memory when vectors have at most
 // RES_ROWS elements; otherwise (and for float64) it is streamed from L2 in
 // 32-row chunks.
+// least size of that arena (float64, whose block Jacobi needs less)
+constexpr size_t kLocalArena = 212 * 1024;
+
 template <typename T, int W>
 struct SmemLayout {
   static constexpr int TU = 16;
@@ -287,10 +301,13 @@ struct SmemLayout {
                                          ? OZ_DIGITS * (oz_a_plane + oz_b_plane) + 4 * OZ_MT * sizeof(float) +
                                                (OZ_MT + OZ_N + W) * sizeof(int)
                                          : 0;
-  __host__ __device__ static size_t total(int P) {
-    return region0(P) + ab_bytes + 2 * g_bytes + ts_bytes + 128 * sizeof(double) + 256 * sizeof(int) + 512 +
-           (oz_bytes ? oz_bytes + 1024 : 0);
+  static constexpr size_t head_bytes = 128 * sizeof(double) + 256 * sizeof(int);  // reductions, column lists
+  // the block Jacobi's areas, which bond_local uses as one arena
+  __host__ __device__ static size_t arena_bytes(int P) {
+    const size_t a = region0(P) + ab_bytes + 2 * g_bytes + ts_bytes + 512 + (oz_bytes ? oz_bytes + 1024 : 0);
+    return a > kLocalArena ? a : kLocalArena;
   }
+  __host__ __device__ static size_t total(int P) { return head_bytes + arena_bytes(P); }
 };
 
 template <typename T, int W>
@@ -306,13 +323,16 @@ struct Smem {
   bool tc = false;
   bool tc_fail = false;  // an MMA wait ran past its limit during the current bond op
   unsigned char *oz = nullptr;  // double-float executor: tensor-core update staging (1024-byte aligned)
+  size_t arena;                 // bytes from r0 on
   __device__ Smem(unsigned char *base, int P) {
     using L = SmemLayout<T, W>;
-    auto al = [](unsigned char *q) {
-      return reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(q) + 15) & ~uintptr_t(15));
-    };
     unsigned char *p = base;
+    red = reinterpret_cast<double *>(p);
+    p += 128 * sizeof(double);
+    ired = reinterpret_cast<int *>(p);
+    p += 256 * sizeof(int);
     r0 = p;
+    arena = L::arena_bytes(P);
     p += L::region0(P);
     Ab = reinterpret_cast<cpx<T> *>(p);
     p += L::ab_bytes;
@@ -322,11 +342,6 @@ struct Smem {
     p += L::g_bytes;
     Ts = reinterpret_cast<cpx<T> *>(p);
     p += L::ts_bytes;
-    p = al(p);
-    red = reinterpret_cast<double *>(p);
-    p += 128 * sizeof(double);
-    ired = reinterpret_cast<int *>(p);
-    p += 256 * sizeof(int);
     if (L::oz_bytes) oz = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
   }
 };
@@ -396,6 +411,10 @@ __device__ __forceinline__ void rr_pair(int r, int t, int &p, int &q) {
   p = a < b ? a : b;
   q = a < b ? b : a;
 }
+
+}  // namespace tn
+#include "tn_local.cuh"
+namespace tn {
 
 // =======================================================================
 // Phase 1: theta = Lambda_{k-1} Gamma_k Lambda_k Gamma_{k+1} Lambda_{k+1},
@@ -1518,6 +1537,11 @@ __device__ int jacobi_svd(cpx<T> *__restrict__ A, int ell, int c, int max_sweeps
   bool guided = kDD;
   const float tol_f = 4.f * sqrtf(float(ell)) * Eps<float>::v;
   constexpr float kGuidedDone = 1e-4f, kFinishDone = 1e-9f;
+  // Float: a sweep whose pairs were all below 3e-5 leaves ~1e-9 / gap, under
+  // the threshold (7e-7 to 1e-5) for relative gaps down to 1e-3, and is the last
+  // one.  Besides the confirming Gram pass this removes the sweep-limit hits:
+  // pairs whose rounding noise hovers about the threshold.
+  constexpr bool kFar = kDD || sizeof(T) == 4;
   // Columns with |a|^2 <= eps^2 ||A||_F^2 are rounding noise: rotating them
   // changes nothing above rounding and their relative off-diagonals never
   // settle, so they are neither rotated nor counted for convergence.
@@ -1696,6 +1720,9 @@ __device__ int jacobi_svd(cpx<T> *__restrict__ A, int ell, int c, int max_sweeps
             } else {
               act = pair_active<T>(sm.G[p * (W + 1) + p].x, sm.G[q * (W + 1) + q].x, sm.G[p * (W + 1) + q], tol,
                                    tiny2);
+              if constexpr (sizeof(T) == 4)
+                farS |= int(pair_active<T>(sm.G[p * (W + 1) + p].x, sm.G[q * (W + 1) + q].x, sm.G[p * (W + 1) + q],
+                                           kFloatDone, tiny2));
             }
           }
           if (act) {
@@ -1708,7 +1735,7 @@ __device__ int jacobi_svd(cpx<T> *__restrict__ A, int ell, int c, int max_sweeps
       }
       needW = __syncthreads_or(needW);
       needC = __syncthreads_or(needC);
-      if constexpr (kDD) far |= __syncthreads_or(farS);
+      if constexpr (kFar) far |= __syncthreads_or(farS);
       const int need = needW | needC;
       if (mode == 0 && !(needW && needC)) mode = needC ? 1 : 2;
       long long t1 = clock64();
@@ -1779,7 +1806,7 @@ __device__ int jacobi_svd(cpx<T> *__restrict__ A, int ell, int c, int max_sweeps
         cyc[2] += clock64() - t1;
       }
     }
-    if (!rotated || (kDD && !far)) {
+    if (!rotated || (kFar && !far)) {
       if (guided) {  // float-converged: the remaining sweeps in double-float
         guided = false;
         continue;
@@ -2194,6 +2221,278 @@ __device__ bool refactor_lq(const cpx<T> *__restrict__ gk, const cpx<T> *__restr
   return true;
 }
 
+// A bond operation held in shared memory from theta to the new Gammas (plan
+// pl).  Same steps and rules as bond_op's general path: theta and the gate,
+// LQ reduction of refactors, SVD, process_svd, Gamma rebuild, renormalisation.
+template <typename T, int NT, int W>
+__device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, const double *gate, const LocalBond<T> &pl, bool try_lq,
+                                  int max_sweeps, Work<T> &wk, Smem<T, W> &sm, long long *cyc) {
+  using R = typename RedType<T>::type;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int cL = tr.chi[k], cM = tr.chi[k + 1], cR = tr.chi[k + 2], m = 2 * cL, nc = 2 * cR;
+  cpx<T> *gk = gamma_slot<T>(tr, k), *gk1 = gamma_slot<T>(tr, k + 1);
+  unsigned char *at = sm.r0;
+  __builtin_assume(__isShared(at));
+  cpx<T> *T0 = reinterpret_cast<cpx<T> *>(at);
+  at += pl.theta;
+  cpx<T> *A = reinterpret_cast<cpx<T> *>(at);
+  at += pl.vec;
+  unsigned char *scratch = at;
+  at += pl.svd;
+  T *lL = reinterpret_cast<T *>(at), *lM = lL + cL, *lR = lM + cM, *sL = lR + cR, *sR = sL + cL;
+  at += pl.lam;
+  double *key = reinterpret_cast<double *>(at);
+  const int cmax = min(m, nc);
+  double *skey = key + cmax, *s2 = skey + cmax;
+  T *isig = reinterpret_cast<T *>(s2 + cmax), *isig2 = isig + cmax, *w2 = isig2 + cmax;
+  int *perm = reinterpret_cast<int *>(w2 + cmax);
+  const double *lamL = lam_slot(tr, k), *lamR = lam_slot(tr, k + 2);
+  double *lamM = lam_slot(tr, k + 1);
+  LocalResult res;
+  for (int v = tid; v < cL; v += NT) lL[v] = T(lamL[v]);
+  for (int u = tid; u < cM; u += NT) lM[u] = T(lamM[u]);
+  for (int w = tid; w < cR; w += NT) lR[w] = T(lamR[w]);
+  __syncthreads();
+  // theta, one (v, w) with its four (s1, s2) a thread; dst2 gets the copy that the sweeps work on
+  auto theta = [&](bool colmode, cpx<T> *dst2) {
+    const int ld = (colmode ? m : nc) | 1;
+    for (int o = tid; o < cL * cR; o += NT) {
+      const int v = o / cR, w = o - v * cR;
+      typename CAcc<T>::type acc[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = acc_zero<T>();
+      const cpx<T> *x = gk + size_t(2 * v) * cM, *y = gk1 + w;
+#pragma unroll 2
+      for (int u = 0; u < cM; ++u) {
+        if ((u & 3) == 0) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) acc_renorm(acc[q]);
+        }
+        const cpx<T> x0 = cscale(x[u], lM[u]), x1 = cscale(x[cM + u], lM[u]);
+        const cpx<T> y0 = y[size_t(2 * u) * cR], y1 = y[size_t(2 * u + 1) * cR];
+        acc_fma<T>(acc[0], x0, y0);
+        acc_fma<T>(acc[1], x0, y1);
+        acc_fma<T>(acc[2], x1, y0);
+        acc_fma<T>(acc[3], x1, y1);
+      }
+      cpx<T> th[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) th[q] = cscale(cscale(acc_fin<T>(acc[q]), lL[v]), lR[w]);
+      if (gate) {
+        cpx<T> t2[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          cpx<T> s = czero<T>();
+#pragma unroll
+          for (int b = 0; b < 4; ++b)
+            s = cfma(mkc<T>(T(gate[8 * a + 2 * b]), T(gate[8 * a + 2 * b + 1])), th[b], s);
+          t2[a] = s;
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a) th[a] = t2[a];
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const int i = 2 * v + (a >> 1), j = (a & 1) * cR + w;
+        const int at2 = colmode ? j * ld + i : i * ld + j;
+        T0[at2] = th[a];
+        if (dst2) dst2[at2] = th[a];
+      }
+    }
+    __syncthreads();
+  };
+  const long long c0 = clock64();
+  bool colmode = m > nc;
+  int ell = colmode ? m : nc, c = colmode ? nc : m;
+  bool lq = false;
+  if (try_lq) {  // as refactor_lq
+    cpx<T> *S = reinterpret_cast<cpx<T> *>(scratch);
+    const int ps = cM | 1;
+    T *diag0 = reinterpret_cast<T *>(scratch + LocalBond<T>::al(size_t(cM) * ps * sizeof(cpx<T>)));
+    for (int e = tid; e < cM * (cM + 1) / 2; e += NT) {
+      int p, q;
+      tri_entry(e, cM, p, q);
+      typename CAcc<T>::type acc = acc_zero<T>();
+      const cpx<T> *bp = gk1 + size_t(p) * nc, *bq = gk1 + size_t(q) * nc;
+#pragma unroll 2
+      for (int col = 0; col < nc; ++col) {
+        const T l = lR[col < cR ? col : col - cR];
+        acc_jfma<T>(acc, cscale(bp[col], l), cscale(bq[col], l));
+      }
+      S[q * ps + p] = acc_fin<T>(acc);  // S_qp = sum B_q conj(B_p)
+    }
+    __syncthreads();
+    if (cholesky_local<T, NT>(S, ps, cM, sizeof(T) == 4 ? 0.1f : 1e-3f, diag0)) {
+      lq = true;
+      const int ld = m | 1;
+      gemm_exact_from<T, NT>(
+          m, cM, [](int, int j) { return j; }, cM,
+          [&](int i, int u) { return cscale(gk[size_t(i) * cM + u], lL[i >> 1] * lM[u]); },
+          [&](int j, int u) { return S[u * ps + j]; }, [&](int i, int j, cpx<T> v) { A[j * ld + i] = v; });
+      colmode = true;
+      ell = m;
+      c = cM;
+    } else {
+      __syncthreads();
+    }
+  }
+  theta(colmode, lq ? nullptr : A);
+  const int ld = ell | 1;
+  const long long c1 = clock64();
+  const int sw = c > 1 ? svd_local<T, NT>(A, ld, ell, c, max_sweeps, scratch, sm.red) : 1;
+  const long long c2 = clock64();
+  cyc[0] = c1 - c0;
+  cyc[1] = c2 - c1;
+  res.lq = lq;
+  res.colmode = colmode;
+  res.ell = ell;
+  res.c = c;
+  res.sweeps = sw;
+  if (sw < 0) {  // go on in the global workspace
+    __syncthreads();
+    const int nv = colmode ? nc : m;
+    for (int idx = tid; idx < c * ell; idx += NT) wk.A[idx] = A[(idx / ell) * ld + idx % ell];
+    for (int idx = tid; idx < nv * ell; idx += NT) wk.T0[idx] = T0[(idx / ell) * ld + idx % ell];
+    for (int v = tid; v < cL; v += NT) wk.lam3[v] = lL[v];
+    for (int u = tid; u < cM; u += NT) wk.lam3[tr.cap + u] = lM[u];
+    for (int w = tid; w < cR; w += NT) wk.lam3[2 * tr.cap + w] = lR[w];
+    __syncthreads();
+    return res;
+  }
+  // process_svd: norms (working-precision terms, summed in R), order, rank
+  // rule and factors.  Square roots and divisions in float64 run in the few
+  // threads that own a value: repeated by every warp they would cost more
+  // than the products.
+  R *sq = reinterpret_cast<R *>(skey);
+  for (int j = warp; j < c; j += NT / 32) {
+    T part = T(0);
+    for (int i = lane; i < ell; i += 32) part += cabs2(A[j * ld + i]);
+    R s = R(part);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s = s + shfl_xor(s, o);
+    if (lane == 0) sq[j] = s;
+  }
+  __syncthreads();
+  for (int j = tid; j < c; j += NT) key[j] = sqrt(double(sq[j]));
+  __syncthreads();
+  for (int j = tid; j < c; j += NT) {
+    const double x = key[j];
+    int rk = 0;
+    for (int i = 0; i < c; ++i) rk += (key[i] > x || (key[i] == x && i < j)) ? 1 : 0;
+    rk = min(rk, c - 1);
+    skey[rk] = x;
+    perm[rk] = j;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    double n1 = 0.0;
+    for (int j = lane; j < c; j += 32) n1 += skey[j] * skey[j];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n1 += __shfl_xor_sync(0xffffffffu, n1, o);
+    n1 = sqrt(n1);
+    const int mode = tr.trunc_mode;
+    const double eps = fmax((mode == 2 || mode == 3) ? fabs(tr.cutoff) : 2.220446049250313e-16, rank_floor<T>(ell));
+    int bad = c;
+    for (int j = lane; j < c; j += 32)
+      if (!is_normal_pos(skey[j] / n1, eps)) bad = min(bad, j);
+    const int nlead = __reduce_min_sync(0xffffffffu, bad);
+    int rank = mode == 1 ? max(1, min(max(tr.chi_max, 1), nlead))
+                         : (mode == 3 ? max(1, min(tr.chi_max, nlead)) : max(nlead, 1));
+    if (rank > tr.cap) {
+      if (lane == 0) atomicOr(tr.status, ST_CAPACITY);
+      rank = tr.cap;
+    }
+    double n2 = 0.0;
+    for (int j = lane; j < rank; j += 32) {
+      const double s = skey[j] / n1;
+      n2 += s * s;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+    n2 = sqrt(n2);
+    for (int j = lane; j < rank; j += 32) s2[j] = (skey[j] / n1) / n2;
+    if (lane == 0) {
+      sm.red[126] = n2;
+      sm.ired[0] = rank;
+    }
+  }
+  __syncthreads();
+  const int rank = sm.ired[0];
+  const R n2 = R(sm.red[126]);
+  for (int j = tid; j < rank; j += NT) {
+    const R x = R(skey[j]), y = R(s2[j]), ix = R(1) / x;
+    isig[j] = T(ix);
+    isig2[j] = T(ix * ix);
+    w2[j] = T(y * y);
+  }
+  for (int v = tid; v < cL; v += NT) sL[v] = T(R(1) / R(lamL[v]));
+  for (int w = tid; w < cR; w += NT) sR[w] = T(n2 / R(lamR[w]));
+  __syncthreads();
+  // Gamma_k and Gamma_{k+1} (one side from the vectors, the other recovered
+  // from theta), with the sums of local_renormalize on the way
+  T pk = T(0), pk1 = T(0);
+  auto put0 = [&](int i, int j, cpx<T> u) {
+    const cpx<T> v = cscale(u, sL[i >> 1]);
+    gk[size_t(i) * rank + j] = v;
+    const T l = lL[i >> 1];
+    pk += cabs2(v) * (l * l) * w2[j];
+  };
+  auto put1 = [&](int j, int col, cpx<T> u) {
+    const int w = col < cR ? col : col - cR;
+    const cpx<T> v = cscale(u, sR[w]);
+    gk1[size_t(j) * nc + col] = v;
+    pk1 += cabs2(v) * w2[j] * (lR[w] * lR[w]);
+  };
+  if (colmode) {
+    for (int o = tid; o < m * rank; o += NT) {
+      const int i = o / rank, j = o - i * rank;
+      put0(i, j, cscale(A[perm[j] * ld + i], isig[j]));
+    }
+    gemm_exact<T, NT>(
+        rank, nc, m,
+        [&](int j, int i) {
+          const cpx<T> a = A[perm[j] * ld + i];
+          return mkc<T>(a.x, -a.y);
+        },
+        [&](int col, int i) { return T0[col * ld + i]; },
+        [&](int j, int col, cpx<T> v) { put1(j, col, cscale(v, isig2[j])); });
+  } else {
+    for (int o = tid; o < rank * nc; o += NT) {
+      const int j = o / nc, col = o - j * nc;
+      put1(j, col, cscale(A[perm[j] * ld + col], isig[j]));
+    }
+    gemm_exact<T, NT>(
+        m, rank, nc, [&](int i, int col) { return T0[i * ld + col]; },
+        [&](int j, int col) {
+          const cpx<T> a = A[perm[j] * ld + col];
+          return mkc<T>(a.x, -a.y);
+        },
+        [&](int i, int j, cpx<T> v) { put0(i, j, cscale(v, isig2[j])); });
+  }
+  R nk = R(pk), nk1 = R(pk1);
+  block_sum2_in<R, NT>(nk, nk1, sm.red);
+  if (tid < 32) {
+    const R a = R(1) / sqrt(nk), b = R(1) / sqrt(nk1);
+    __syncwarp();
+    T *f = reinterpret_cast<T *>(sm.red + 100);
+    if (tid == 0) {
+      f[0] = T(a);
+      f[1] = T(b);
+    }
+  }
+  __syncthreads();
+  const T ik = reinterpret_cast<T *>(sm.red + 100)[0], ik1 = reinterpret_cast<T *>(sm.red + 100)[1];
+  // each thread rescales what it wrote (the loops above run over the same elements)
+  for (int o = tid; o < m * rank; o += NT) gk[o] = cscale(gk[o], ik);
+  for (int o = tid; o < rank * nc; o += NT) gk1[o] = cscale(gk1[o], ik1);
+  for (int j = tid; j < rank; j += NT) lamM[j] = s2[j];
+  if (tid == 0) tr.chi[k + 1] = rank;
+  __syncthreads();
+  cyc[2] = clock64() - c2;
+  res.done = true;
+  return res;
+}
+
 // One bond operation on (k, k+1): gate != nullptr -> apply_unitary2, else local_refactor.
 template <typename T, int NT, int W>
 __device__ void bond_op(const TrajDev &tr, int k, const double *gate, Work<T> &wk, int max_sweeps, int scheme,
@@ -2204,13 +2503,23 @@ __device__ void bond_op(const TrajDev &tr, int k, const double *gate, Work<T> &w
   const double *lamL = lam_slot(tr, k), *lamR = lam_slot(tr, k + 2);
   double *lamM = lam_slot(tr, k + 1);
   long long c0 = clock64();
+  const bool try_lq = !gate && cM < nc && cM <= m;
+  LocalBond<T> pl;
+  LocalResult loc;
+  long long lcyc[3] = {0, 0, 0};
+  // Small bonds stay in shared memory throughout; MIXED takes them below the
+  // tensor-core theta's sizes.
+  const bool local = pl.plan(cL, cM, cR, try_lq, sm.arena, NT);
+  if (local) loc = bond_local<T, NT, W>(tr, k, gate, pl, try_lq, max_sweeps, wk, sm, lcyc);
   // Lambda_{k-1}, Lambda_k, Lambda_{k+1} in the working precision (the state
   // keeps them in float64; the contraction multiplies in T)
   T *lLt = wk.lam3, *lMt = wk.lam3 + tr.cap, *lRt = wk.lam3 + 2 * tr.cap;
-  for (int v = threadIdx.x; v < cL; v += NT) lLt[v] = T(lamL[v]);
-  for (int u = threadIdx.x; u < cM; u += NT) lMt[u] = T(lamM[u]);
-  for (int w = threadIdx.x; w < cR; w += NT) lRt[w] = T(lamR[w]);
-  __syncthreads();
+  if (!local) {
+    for (int v = threadIdx.x; v < cL; v += NT) lLt[v] = T(lamL[v]);
+    for (int u = threadIdx.x; u < cM; u += NT) lMt[u] = T(lamM[u]);
+    for (int w = threadIdx.x; w < cR; w += NT) lRt[w] = T(lamR[w]);
+    __syncthreads();
+  }
   // Refactors of a bond whose theta has more columns than its rank bound
   // chiM go through the LQ-reduced matrix M (m x chiM); gates and small
   // bonds take the direct path on theta.
@@ -2226,13 +2535,18 @@ __device__ void bond_op(const TrajDev &tr, int k, const double *gate, Work<T> &w
     }
     build_theta<T, NT, W>(gk, gk1, lLt, lMt, lRt, cL, cM, cR, g, dst, copy, cm, sm);
   };
-  if (!gate && cM < nc && cM <= m) {
+  if (!local && try_lq) {
     theta(nullptr, wk.T0, wk.T0, true);
     lq = refactor_lq<T, NT, W>(gk, gk1, lLt, lMt, lRt, cL, cM, cR, tr.cap, wk, sm);
   }
   bool colmode;
   int ell, c;
-  if (lq) {
+  if (local) {
+    lq = loc.lq;
+    colmode = loc.colmode;
+    ell = loc.ell;
+    c = loc.c;
+  } else if (lq) {
     colmode = true;
     ell = m;
     c = cM;
@@ -2244,7 +2558,19 @@ __device__ void bond_op(const TrajDev &tr, int k, const double *gate, Work<T> &w
   }
   long long c1 = clock64();
   long long cyc[4] = {0, 0, 0, 0};
-  int sw = jacobi_svd<T, NT, W>(wk.A, ell, c, max_sweeps, sm, cyc, wk.sig, wk.perm, scheme);
+  int sw = loc.sweeps;
+  // The vectors of a wider theta still fit svd_local's scratch up to c = 64
+  // (float64 classes) or 128 x 128 (float); the block Jacobi takes the rest and
+  // what svd_local could not separate.
+  if (!local && c > 1 && c <= LocalSvd<T>::max_c(NT) && LocalSvd<T>::bytes(ell, c) <= sm.arena) {
+    const long long t0 = clock64();
+    sw = svd_local<T, NT>(wk.A, ell, ell, c, max_sweeps, sm.r0, sm.red);
+    __syncthreads();
+    cyc[1] += clock64() - t0;
+    loc.svd_done = sw >= 0;
+  }
+  if (!loc.done && !loc.svd_done)
+    sw = jacobi_svd<T, NT, W>(wk.A, ell, c, max_sweeps, sm, cyc, wk.sig, wk.perm, scheme);
   long long c2 = clock64();
   if (threadIdx.x == 0) {
     if (sw < 0) {
@@ -2256,29 +2582,32 @@ __device__ void bond_op(const TrajDev &tr, int k, const double *gate, Work<T> &w
     }
     if (tr.stats) {
       if (lq) atomicAdd(tr.stats + STAT_LQ_OPS, 1.0);
-      const double a = double(m > nc ? m : nc), b = double(m > nc ? nc : m);
-      double ft = 8.0 * m * double(cM) * nc + (gate ? 128.0 * cL * cR : 0.0);
-      atomicAdd(tr.stats + STAT_FLOP_THETA, ft);
-      atomicAdd(tr.stats + STAT_FLOP_SVD, 4.0 * (4.0 * a * a * b + 8.0 * a * b * b + 9.0 * b * b * b));
+      // (whole numbers below 2^53: integer arithmetic spares this thread a chain of float64 operations)
+      const long long a = m > nc ? m : nc, b = m > nc ? nc : m;
+      atomicAdd(tr.stats + STAT_FLOP_THETA, double(8ll * m * cM * nc + (gate ? 128ll * cL * cR : 0ll)));
+      atomicAdd(tr.stats + STAT_FLOP_SVD, double(4ll * (4 * a * a * b + 8 * a * b * b + 9 * b * b * b)));
       atomicAdd(tr.stats + STAT_BOND_OPS, 1.0);
       atomicAdd(tr.stats + STAT_SWEEPS, double(sw < 0 ? max_sweeps : sw));
       // read the Gamma pair + Lambdas, write the new Gamma pair
-      const double eb = double(sizeof(cpx<T>));
-      atomicAdd(tr.stats + STAT_BYTES, eb * (2.0 * cL * cM + 2.0 * cM * cR) * 2.0 + 8.0 * (cL + cM + cR));
+      const long long eb = sizeof(cpx<T>);
+      atomicAdd(tr.stats + STAT_BYTES, double(eb * 4 * (1ll * cL * cM + 1ll * cM * cR) + 8ll * (cL + cM + cR)));
     }
   }
-  finalize_bond<T, NT, W>(tr, k, gk, gk1, lamL, lamM, lamR, cL, cR, colmode, ell, c, wk, sm);
+  if (!loc.done) finalize_bond<T, NT, W>(tr, k, gk, gk1, lamL, lamM, lamR, cL, cR, colmode, ell, c, wk, sm);
   if (sm.tc_fail) {  // a tensor-core wait gave up: the op's result is not trustworthy
     if (threadIdx.x == 0) atomicOr(tr.status, ST_BAD_INSTR);
     sm.tc_fail = false;
   }
   if (threadIdx.x == 0 && tr.stats) {
-    atomicAdd(tr.stats + STAT_CYC_THETA, double(c1 - c0));
-    atomicAdd(tr.stats + STAT_CYC_GRAM, double(cyc[0]));
-    atomicAdd(tr.stats + STAT_CYC_ROT, double(cyc[1]));
-    atomicAdd(tr.stats + STAT_CYC_UPDATE, double(cyc[2]));
-    atomicAdd(tr.stats + STAT_CYC_FINAL, double(clock64() - c2));
-    atomicAdd(tr.stats + STAT_BLOCK_STEPS, double(cyc[3]));
+    // in shared memory the whole SVD counts as rotations
+    atomicAdd(tr.stats + STAT_CYC_THETA, double(local ? lcyc[0] : c1 - c0));
+    atomicAdd(tr.stats + STAT_CYC_ROT, double(cyc[1] + lcyc[1]));
+    atomicAdd(tr.stats + STAT_CYC_FINAL, double(loc.done ? lcyc[2] : clock64() - c2));
+    if (!loc.done) {
+      atomicAdd(tr.stats + STAT_CYC_GRAM, double(cyc[0]));
+      atomicAdd(tr.stats + STAT_CYC_UPDATE, double(cyc[2]));
+      atomicAdd(tr.stats + STAT_BLOCK_STEPS, double(cyc[3]));
+    }
   }
 }
 

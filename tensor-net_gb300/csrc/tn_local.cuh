@@ -1,0 +1,728 @@
+// tn_local.cuh -- bond operations that fit the CTA's shared memory.
+//
+// Most bond operations of a trajectory are small (chain ends, early layers,
+// strongly measured circuits), and their time is latency: barriers, scalar
+// chains and round trips to global scratch, not arithmetic.  Here theta, the
+// Jacobi vectors and every per-value array stay in shared memory, products
+// have exactly as many terms as the bond has (no tile padding), and the SVD is
+// split by precision:
+//
+//  1. float one-sided (Hestenes) Jacobi on a float copy of the vectors, the
+//     rotations accumulated in V (hestenes): one barrier a round, no Gram matrix;
+//  2. V made unitary to the working precision by a Newton-Schulz step
+//     (unitarise), and A <- A Q in the working precision (apply_unitary): exact
+//     to its rounding, so the float angles cost no accuracy;
+//  3. refinement: the Gram matrix of A in the working precision gives every
+//     remaining rotation at once, tan(theta) = t for each pair as in a Jacobi
+//     rotation; I + K with K_qp = -t e, K_pq = t conj(e) is made unitary by the
+//     same step and applied.  The off-diagonals fall quadratically; two steps
+//     usually reach the working precision's threshold.
+//
+// The sweeps of 1 are the many, cheap ones; the working precision pays for two
+// or three products instead of every rotation of every sweep.  Pairs that are
+// degenerate to the float rounding cannot be separated by 3 (K would not be
+// small); svd_local then reports so and the caller goes on with the block
+// Jacobi on the (already unitarily transformed) vectors.
+#pragma once
+
+namespace tn {
+
+// Float sweeps end after one whose pairs were all below this (see jacobi_svd).
+constexpr float kFloatDone = 3e-5f;
+
+// ------------------------------------------------------------- arithmetic
+// Arithmetic of the sums that need more than float but not float64's
+// throughput cost (float64 issues at 1/64 of the float rate): double-float
+// for float and dd, float64 only where the working precision is float64.
+template <typename T>
+struct RedType {
+  using type = dd;
+};
+template <>
+struct RedType<double> {
+  using type = double;
+};
+__device__ __forceinline__ float lead(float x) { return x; }
+__device__ __forceinline__ float lead(double x) { return float(x); }
+__device__ __forceinline__ float lead(dd x) { return x.hi; }
+template <typename T>
+__device__ __forceinline__ T from_dd(dd x) {
+  return T(x);
+}
+template <>
+__device__ __forceinline__ double from_dd<double>(dd x) {
+  return double(x.hi) + double(x.lo);
+}
+
+// Sum of products of floats, every product exact, the sum in three floats
+// (about 2^-60 of its largest term: V^H V - I cancels to 1e-6 and its own
+// error is what V's unitarity is held to, in float64 too).
+struct tacc {
+  float hi, mid, lo;
+};
+__device__ __forceinline__ void tacc_add_prod(tacc &s, float a, float b) {
+  float p, e, h, t, u;
+  two_prod(a, b, p, e);
+  two_sum(s.hi, p, h, t);
+  s.hi = h;
+  two_sum(s.mid, t, h, u);
+  s.mid = h;
+  s.lo = __fadd_rn(s.lo, __fadd_rn(u, e));
+}
+__device__ __forceinline__ dd tacc_fin(const tacc &s) {
+  float h, e, m, f;
+  two_sum(s.hi, s.mid, h, e);
+  two_sum(e, s.lo, m, f);
+  return dd_norm(h, m);
+}
+// acc + a w with w double-float
+__device__ __forceinline__ void dacc_add_fdprod(dacc &s, float a, dd w) {
+  float p, e, h, t;
+  two_prod(a, w.hi, p, e);
+  e = __fmaf_rn(a, w.lo, e);
+  two_sum(s.hi, p, h, t);
+  s.hi = h;
+  s.lo = __fadd_rn(s.lo, __fadd_rn(t, e));
+}
+
+// Largest of the threads' non-negative values (uniform result).
+template <int NT>
+__device__ __forceinline__ float block_max(float v, double *red) {
+  unsigned int *r = reinterpret_cast<unsigned int *>(red);
+  // NaN compares above every number here (its bit pattern does), so a bad
+  // value is seen by the caller's upper limits
+  unsigned int m = __reduce_max_sync(0xffffffffu, __float_as_uint(v) & 0x7fffffffu);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) r[threadIdx.x >> 5] = m;
+  __syncthreads();
+  m = r[threadIdx.x & (NT / 32 - 1)];
+  m = __reduce_max_sync(0xffffffffu, m);
+  return __uint_as_float(m);
+}
+
+// Upper-triangle entry e -> (p, q), p <= q < c, row by row.
+__device__ __forceinline__ void tri_entry(int e, int c, int &p, int &q) {
+  const float b = float(2 * c + 1);
+  int r = int((b - sqrtf(fmaxf(b * b - 8.f * float(e), 0.f))) * 0.5f);
+  r = max(0, min(r, c - 1));
+  auto start = [&](int x) { return x * c - x * (x - 1) / 2; };
+  while (r > 0 && start(r) > e) --r;
+  while (r + 1 < c && start(r + 1) <= e) ++r;
+  p = r;
+  q = r + (e - start(r));
+}
+
+// C[x][y] = sum_k P(x, k) Q(y, k), one output a thread, exactly M N K terms.
+// Faster than the 64 x 64 tiles of gemm_nt while the outputs are at most a
+// few per thread: a 16 x 16 x 16 double-float product is one pass of 16 terms
+// here and a whole padded tile there.
+template <typename T, int NT, class FP, class FQ, class FE>
+__device__ void gemm_exact(int M, int N, int K, FP P, FQ Q, FE E) {
+  for (int o = threadIdx.x; o < M * N; o += NT) {
+    const int x = o / N, y = o - x * N;
+    typename CAcc<T>::type acc = acc_zero<T>();
+#pragma unroll 4
+    for (int k = 0; k < K; ++k) {
+      if ((k & 3) == 0) acc_renorm(acc);
+      acc_fma<T>(acc, P(x, k), Q(y, k));
+    }
+    E(x, y, acc_fin<T>(acc));
+  }
+}
+
+// The same with the terms k < from(x, y) of an output left out (a triangular factor).
+template <typename T, int NT, class FK, class FP, class FQ, class FE>
+__device__ void gemm_exact_from(int M, int N, FK from, int K, FP P, FQ Q, FE E) {
+  for (int o = threadIdx.x; o < M * N; o += NT) {
+    const int x = o / N, y = o - x * N;
+    typename CAcc<T>::type acc = acc_zero<T>();
+#pragma unroll 2
+    for (int k = from(x, y); k < K; ++k) acc_fma<T>(acc, P(x, k), Q(y, k));
+    E(x, y, acc_fin<T>(acc));
+  }
+  __syncthreads();
+}
+
+// ------------------------------------------------- 1. float Hestenes Jacobi
+// One-sided Jacobi of the c float vectors As[j * pa + i] (length ell, in
+// shared memory), rotations accumulated in the columns Vs[j * pv + i] (when
+// Vs is set).  Round-robin ordering over the vectors sorted by decreasing norm
+// (de Rijk); a pair belongs to LG lanes, which form the inner product and
+// apply the rotation to their elements.  Norms are carried by a' = a - t |g|,
+// b' = b + t |g| and recomputed each sweep.  Stops after a sweep without a
+// pair above `done` (before its rotation).  Returns the sweeps, -1 at the limit.
+template <int NT>
+__device__ int hestenes(cpx<float> *As, int pa, int ell, cpx<float> *Vs, int pv, int c, float *nrm, int *ord,
+                        float floor_, float tol, float done, int max_sweeps) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int cp = c + (c & 1), np = cp >> 1, ring = cp - 1;
+  int LG = 32;
+  while (LG > 4 && np * LG > NT) LG >>= 1;
+  const int l = tid & (LG - 1), grp = tid / LG, ngrp = NT / LG;
+  const int active = min(NT, ((np * LG + 31) >> 5) << 5);  // threads that own a pair (whole warps)
+  const float tol2 = tol * tol, done2 = done * done;
+  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    for (int j = warp; j < c; j += NT / 32) {
+      float s = 0.f;
+      for (int i = lane; i < ell; i += 32) s += cabs2(As[j * pa + i]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) nrm[j] = s;
+    }
+    __syncthreads();
+    float fro = 0.f;
+    for (int j = tid; j < c; j += NT) {
+      const float x = nrm[j];
+      int rk = 0;
+      for (int i = 0; i < c; ++i) {
+        const float y = nrm[i];
+        rk += (y > x || (y == x && i < j)) ? 1 : 0;
+      }
+      ord[min(rk, c - 1)] = j;
+    }
+    for (int i = 0; i < c; ++i) fro += nrm[i];
+    const float tiny2 = fmaxf(fro * floor_ * floor_, 1e-37f);
+    __syncthreads();
+    int far = 0;
+    if (tid < active) {
+      for (int r = 0; r < ring; ++r) {
+        for (int t0 = 0; t0 < np; t0 += ngrp) {
+          const int t = t0 + grp;
+          int a_ = t == 0 ? 0 : t + r, b_ = cp - 1 - t + r;  // circle positions t and cp - 1 - t
+          if (a_ > ring) a_ -= ring;
+          if (b_ > ring) b_ -= ring;
+          const int lo = min(a_, b_), hi = max(a_, b_);
+          const bool valid = t < np && hi < c;
+          const int P = valid ? ord[lo] : 0, Q = valid ? ord[hi] : 0;
+          cpx<float> *ap = As + P * pa, *aq = As + Q * pa;
+          float gx = 0.f, gy = 0.f;
+          for (int i = l; i < ell; i += LG) {
+            const cpx<float> x = ap[i], y = aq[i];
+            gx = fmaf(x.x, y.x, fmaf(x.y, y.y, gx));
+            gy = fmaf(x.x, y.y, fmaf(-x.y, y.x, gy));
+          }
+          for (int o = LG >> 1; o > 0; o >>= 1) {
+            gx += __shfl_xor_sync(0xffffffffu, gx, o);
+            gy += __shfl_xor_sync(0xffffffffu, gy, o);
+          }
+          const float a = nrm[P], b = nrm[Q];
+          __syncwarp();
+          if (valid && a > tiny2 && b > tiny2) {
+            // scaled by the norms: g / (|a_p| |a_q|) stays in range for vectors of any size
+            const float ra = rsqrtf(a), rb = rsqrtf(b), sc = ra * rb;
+            const float hx = gx * sc, hy = gy * sc, r2 = fmaf(hx, hx, hy * hy);
+            far |= int(r2 > done2);
+            if (r2 > tol2) {
+              const float rr = rsqrtf(r2);
+              const float z = 0.5f * ((b - a) * sc) * rr;
+              const float z1 = fmaf(z, z, 1.f);
+              const float tt = fabsf(z) > 1e15f ? __fdividef(0.5f, z)
+                                                : copysignf(__fdividef(1.f, fabsf(z) + z1 * rsqrtf(z1)), z);
+              const float cs = rsqrtf(fmaf(tt, tt, 1.f)), sn = tt * cs;
+              const cpx<float> e = mkc<float>(hx * rr, -hy * rr);
+              for (int i = l; i < ell; i += LG) {
+                const cpx<float> x = ap[i], y = cmul(e, aq[i]);
+                ap[i] = mkc<float>(cs * x.x - sn * y.x, cs * x.y - sn * y.y);
+                aq[i] = mkc<float>(sn * x.x + cs * y.x, sn * x.y + cs * y.y);
+              }
+              if (Vs) {
+                cpx<float> *vp = Vs + P * pv, *vq = Vs + Q * pv;
+                for (int i = l; i < c; i += LG) {
+                  const cpx<float> x = vp[i], y = cmul(e, vq[i]);
+                  vp[i] = mkc<float>(cs * x.x - sn * y.x, cs * x.y - sn * y.y);
+                  vq[i] = mkc<float>(sn * x.x + cs * y.x, sn * x.y + cs * y.y);
+                }
+              }
+              if (l == 0) {
+                const float d = tt * (r2 * rr) * (a * ra) * (b * rb);
+                nrm[P] = a - d;
+                nrm[Q] = b + d;
+              }
+            }
+          }
+        }
+        if (active == 32)
+          __syncwarp();
+        else
+          asm volatile("bar.sync 1, %0;" ::"r"(active) : "memory");
+      }
+    }
+    if (!__syncthreads_or(far)) return sweep + 1;
+  }
+  return -1;
+}
+
+// ------------------------------------------------ 2. unitary to working precision
+// Q (c x c, row-major with pitch pq) <- the unitary factor of V (float,
+// columns Vs[k * pv + r]), V unitary to a few float roundings or I + K.
+// S = V^H V - I is formed from exact float products; float Newton-Schulz
+// steps bring |S| below 1e-5 first where it is larger (I + K with a t near 1);
+// then Q = V (I - S/2 + 3/8 S^2), whose error is of the order |S|^3 < 1e-15.
+// The correction V W is accumulated in double-float in every mode (W < 1e-5,
+// so its error is below 1e-16).  Returns false (Q not written) when V is too
+// far from unitary.
+template <typename T, int NT>
+__device__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S, int ps, cpx<T> *Q, int pq, double *red) {
+  constexpr int OPT = NT >= 512 ? 8 : 8;  // outputs per thread: c <= 64 at 512 threads, c <= 32 at 128
+  const int tid = threadIdx.x;
+  const int ntri = c * (c + 1) / 2;
+  for (int it = 0;; ++it) {
+    float smax = 0.f;
+    for (int e = tid; e < ntri; e += NT) {
+      int p, q;
+      tri_entry(e, c, p, q);
+      const cpx<float> *vp = Vs + p * pv, *vq = Vs + q * pv;
+      tacc ax, ay;
+      ax.mid = ax.lo = ay.hi = ay.mid = ay.lo = 0.f;
+      ax.hi = p == q ? -1.f : 0.f;
+#pragma unroll 2
+      for (int k = 0; k < c; ++k) {
+        const cpx<float> x = vp[k], y = vq[k];
+        tacc_add_prod(ax, x.x, y.x);
+        tacc_add_prod(ax, x.y, y.y);
+        tacc_add_prod(ay, x.x, y.y);
+        tacc_add_prod(ay, -x.y, y.x);
+      }
+      const dd sx = tacc_fin(ax), sy = tacc_fin(ay);
+      S[p * ps + q] = mkc<dd>(sx, sy);
+      if (p != q) S[q * ps + p] = mkc<dd>(sx, -sy);
+      smax = fmaxf(smax, fmaxf(fabsf(sx.hi), fabsf(sy.hi)));
+      if (!(sx.hi == sx.hi && sy.hi == sy.hi)) smax = __int_as_float(0x7f800000);
+    }
+    smax = block_max<NT>(smax, red);  // (ends with S visible: its barriers follow the stores)
+    if (smax <= 1e-5f) break;
+    if (!(smax <= 0.5f) || it >= 6) return false;
+    cpx<float> out[OPT];
+#pragma unroll
+    for (int u = 0; u < OPT; ++u) {
+      const int o = tid + u * NT;
+      if (o < c * c) {
+        const int y = o / c, r = o - y * c;
+        cpx<float> a = czero<float>();
+        for (int k = 0; k < c; ++k) {
+          const cpx<dd> s = S[k * ps + y];
+          a = cfma(Vs[k * pv + r], mkc<float>(s.x.hi, s.y.hi), a);
+        }
+        const cpx<float> v = Vs[y * pv + r];
+        out[u] = mkc<float>(fmaf(-0.5f, a.x, v.x), fmaf(-0.5f, a.y, v.y));
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < OPT; ++u) {
+      const int o = tid + u * NT;
+      if (o < c * c) Vs[(o / c) * pv + o % c] = out[u];
+    }
+    __syncthreads();
+  }
+  // W = -S/2 + 3/8 S^2 (the square in float), in place of S
+  {
+    cpx<float> sq[OPT];
+#pragma unroll
+    for (int u = 0; u < OPT; ++u) {
+      const int o = tid + u * NT;
+      if (o < c * c) {
+        const int y = o / c, x = o - y * c;
+        cpx<float> a = czero<float>();
+        for (int k = 0; k < c; ++k) {
+          const cpx<dd> s = S[x * ps + k], t = S[k * ps + y];
+          a = cfma(mkc<float>(s.x.hi, s.y.hi), mkc<float>(t.x.hi, t.y.hi), a);
+        }
+        sq[u] = a;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < OPT; ++u) {
+      const int o = tid + u * NT;
+      if (o < c * c) {
+        const int y = o / c, x = o - y * c;
+        const cpx<dd> s = S[x * ps + y];
+        S[x * ps + y] = mkc<dd>(dd(-0.5f * s.x.hi, -0.5f * s.x.lo) + dd(0.375f * sq[u].x),
+                                dd(-0.5f * s.y.hi, -0.5f * s.y.lo) + dd(0.375f * sq[u].y));
+      }
+    }
+    __syncthreads();
+  }
+  for (int o = tid; o < c * c; o += NT) {
+    const int y = o / c, r = o - y * c;
+    dacc ax, ay;
+    ax.hi = ax.lo = ay.hi = ay.lo = 0.f;
+#pragma unroll 2
+    for (int k = 0; k < c; ++k) {
+      const cpx<float> v = Vs[k * pv + r];
+      const cpx<dd> w = S[k * ps + y];
+      dacc_add_fdprod(ax, v.x, w.x);
+      dacc_add_fdprod(ax, -v.y, w.y);
+      dacc_add_fdprod(ay, v.x, w.y);
+      dacc_add_fdprod(ay, v.y, w.x);
+    }
+    const cpx<float> v = Vs[y * pv + r];
+    Q[r * pq + y] = mkc<T>(T(v.x) + from_dd<T>(dd_norm(ax.hi, ax.lo)), T(v.y) + from_dd<T>(dd_norm(ay.hi, ay.lo)));
+  }
+  __syncthreads();
+  return true;
+}
+
+// 32 rows [i0, i0 + 32) of the vectors A[j * ld + i] as stage[r * pt + j].
+template <typename T, int NT>
+__device__ __forceinline__ void stage_rows(const cpx<T> *A, int ld, int ell, int c, int i0, cpx<T> *stage, int pt) {
+  for (int idx = threadIdx.x; idx < 32 * c; idx += NT) {
+    const int r = idx & 31, p = idx >> 5;
+    stage[r * pt + p] = i0 + r < ell ? A[size_t(p) * ld + i0 + r] : czero<T>();
+  }
+}
+
+// A <- A Q, 32 rows at a time.
+template <typename T, int NT>
+__device__ void apply_unitary(cpx<T> *A, int ld, int ell, int c, const cpx<T> *Q, int pq, cpx<T> *stage, int pt) {
+  for (int i0 = 0; i0 < ell; i0 += 32) {
+    stage_rows<T, NT>(A, ld, ell, c, i0, stage, pt);
+    __syncthreads();
+    const int rows = min(32, ell - i0);
+    for (int o = threadIdx.x; o < 32 * c; o += NT) {
+      const int r = o & 31, y = o >> 5;
+      if (r < rows) {
+        typename CAcc<T>::type acc = acc_zero<T>();
+#pragma unroll 4
+        for (int p = 0; p < c; ++p) {
+          if ((p & 3) == 0) acc_renorm(acc);
+          acc_fma<T>(acc, stage[r * pt + p], Q[p * pq + y]);
+        }
+        A[size_t(y) * ld + i0 + r] = acc_fin<T>(acc);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// A <- A + A K for K (float, off-diagonal, K[p][y] = Ks[y * pk + p]) so small
+// that the float correction of the leading parts is exact to the working
+// precision (limit at the call).
+template <typename T, int NT>
+__device__ void apply_small(cpx<T> *A, int ld, int ell, int c, const cpx<float> *Ks, int pk, cpx<float> *stage,
+                            int pt) {
+  for (int i0 = 0; i0 < ell; i0 += 32) {
+    for (int idx = threadIdx.x; idx < 32 * c; idx += NT) {
+      const int r = idx & 31, p = idx >> 5;
+      cpx<float> v = czero<float>();
+      if (i0 + r < ell) {
+        const cpx<T> x = A[size_t(p) * ld + i0 + r];
+        v = mkc<float>(lead(x.x), lead(x.y));
+      }
+      stage[r * pt + p] = v;
+    }
+    __syncthreads();
+    const int rows = min(32, ell - i0);
+    for (int o = threadIdx.x; o < 32 * c; o += NT) {
+      const int r = o & 31, y = o >> 5;
+      if (r < rows) {
+        cpx<float> a = czero<float>();
+        for (int p = 0; p < c; ++p)
+          if (p != y) a = cfma(stage[r * pt + p], Ks[y * pk + p], a);
+        cpx<T> &x = A[size_t(y) * ld + i0 + r];
+        const cpx<T> v = x;
+        x = mkc<T>(v.x + T(a.x), v.y + T(a.y));
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// G = A^H A (upper triangle G[p * pg + q], p <= q) in the working precision.
+template <typename T, int NT>
+__device__ void gram_local(const cpx<T> *A, int ld, int ell, int c, cpx<T> *G, int pg, cpx<T> *stage, int pt) {
+  constexpr int PER = 5;  // c (c + 1) / 2 entries: c <= 64 at 512 threads, c <= 32 at 128
+  const int ntri = c * (c + 1) / 2;
+  typename CAcc<T>::type acc[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) acc[u] = acc_zero<T>();
+  for (int i0 = 0; i0 < ell; i0 += 32) {
+    stage_rows<T, NT>(A, ld, ell, c, i0, stage, pt);
+    __syncthreads();
+    const int rows = min(32, ell - i0);
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int e = threadIdx.x + u * NT;
+      if (e < ntri) {
+        int p, q;
+        tri_entry(e, c, p, q);
+        typename CAcc<T>::type a = acc[u];
+#pragma unroll 4
+        for (int r = 0; r < rows; ++r) {
+          if ((r & 3) == 0) acc_renorm(a);
+          acc_jfma<T>(a, stage[r * pt + p], stage[r * pt + q]);
+        }
+        acc[u] = a;
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = threadIdx.x + u * NT;
+    if (e < ntri) {
+      int p, q;
+      tri_entry(e, c, p, q);
+      G[p * pg + q] = acc_fin<T>(acc[u]);
+    }
+  }
+  __syncthreads();
+}
+
+// ------------------------------------------------------------- the SVD
+// Scratch of svd_local in bytes: the float vectors (or, later, a stage of 32
+// rows and Q), the Gram matrix / S, V, norms and order.
+template <typename T>
+struct LocalSvd {
+  static constexpr int MAXC = sizeof(T) == 4 ? 128 : 64;
+  __host__ __device__ static constexpr size_t al(size_t x) { return (x + 15) & ~size_t(15); }
+  __host__ __device__ static constexpr int odd(int x) { return x | 1; }
+  __host__ __device__ static size_t as_bytes(int ell, int c) { return al(size_t(c) * odd(ell) * sizeof(cpx<float>)); }
+  __host__ __device__ static size_t first_bytes(int ell, int c) {
+    const size_t a = as_bytes(ell, c);
+    const size_t b = sizeof(T) == 4 ? 0 : al(size_t(32) * odd(c) * sizeof(cpx<T>)) + al(size_t(c) * odd(c) * 16);
+    return a > b ? a : b;
+  }
+  __host__ __device__ static size_t bytes(int ell, int c) {
+    const size_t tail = al(size_t(c) * 8);
+    if (sizeof(T) == 4) return first_bytes(ell, c) + tail;
+    return first_bytes(ell, c) + al(size_t(c) * odd(c) * 16) + al(size_t(c) * odd(c) * 8) + tail;
+  }
+  // largest c of the refinement's fixed outputs per thread
+  __host__ __device__ static int max_c(int nt) { return sizeof(T) == 4 ? MAXC : (nt >= 512 ? 64 : 32); }
+};
+
+// Orthogonalises the c vectors A[j * ld + i] (length ell; any address space)
+// by unitary column operations.  scratch: LocalSvd<T>::bytes of shared memory,
+// 16-byte aligned.  Returns the number of sweeps and refinement steps, or -1:
+// A is then a unitary transform of the input that has not converged (a
+// degenerate spectrum, or the sweep limit), for the caller's block Jacobi.
+template <typename T, int NT>
+__device__ int svd_local(cpx<T> *A, int ld, int ell, int c, int max_sweeps, unsigned char *scratch, double *red) {
+  using L = LocalSvd<T>;
+  const int tid = threadIdx.x;
+  const int pa = L::odd(ell), pc = L::odd(c);
+  unsigned char *at = scratch;
+  cpx<float> *As = reinterpret_cast<cpx<float> *>(at);
+  at += L::first_bytes(ell, c);
+  const float tolf = 4.f * sqrtf(float(ell)) * Eps<float>::v;
+  auto load = [&]() {
+    for (int idx = tid; idx < c * ell; idx += NT) {
+      const int j = idx / ell, i = idx - j * ell;
+      const cpx<T> x = A[size_t(j) * ld + i];
+      As[j * pa + i] = mkc<float>(lead(x.x), lead(x.y));
+    }
+  };
+  if constexpr (sizeof(T) == 4) {
+    float *nrm = reinterpret_cast<float *>(at);
+    int *ord = reinterpret_cast<int *>(nrm + c);
+    load();
+    __syncthreads();
+    const int sw = hestenes<NT>(As, pa, ell, nullptr, 0, c, nrm, ord, float(sweep_floor<float>(ell)), tolf,
+                                fmaxf(tolf, kFloatDone), max_sweeps);
+    for (int idx = tid; idx < c * ell; idx += NT) {
+      const int j = idx / ell, i = idx - j * ell;
+      A[size_t(j) * ld + i] = As[j * pa + i];
+    }
+    __syncthreads();
+    return sw;
+  } else {
+    cpx<T> *stage = reinterpret_cast<cpx<T> *>(scratch);
+    cpx<T> *Q = reinterpret_cast<cpx<T> *>(scratch + L::al(size_t(32) * pc * sizeof(cpx<T>)));
+    cpx<dd> *S = reinterpret_cast<cpx<dd> *>(at);
+    cpx<T> *G = reinterpret_cast<cpx<T> *>(at);
+    at += L::al(size_t(c) * pc * 16);
+    cpx<float> *Vs = reinterpret_cast<cpx<float> *>(at);
+    at += L::al(size_t(c) * pc * 8);
+    float *nrm = reinterpret_cast<float *>(at);
+    int *ord = reinterpret_cast<int *>(nrm + c);
+    const float floor_t = float(sweep_floor<T>(ell));
+    const float tol = float(4.0 * sqrt(double(ell)) * double(Eps<T>::v));
+    // a correction formed in float is exact to the working precision below this angle
+    constexpr float kFloatApply = std::is_same<T, double>::value ? 1e-9f : 1e-7f;
+    constexpr int kMaxStages = 3, kMaxSteps = 10;
+    int sweeps = 0, stages = 0;
+    bool bulk = true;  // a float stage is due
+    for (int step = 0; step < kMaxSteps; ++step) {
+      if (bulk) {
+        load();
+        for (int idx = tid; idx < c * c; idx += NT) {
+          const int y = idx / c, r = idx - y * c;
+          Vs[y * pc + r] = mkc<float>(y == r ? 1.f : 0.f, 0.f);
+        }
+        __syncthreads();
+        // the first stage leaves vectors at the float noise level alone; once A
+        // holds them to its own precision the next one resolves them too
+        const int sw = hestenes<NT>(As, pa, ell, Vs, pc, c, nrm, ord, stages == 0 ? Eps<float>::v : floor_t, tolf,
+                                    1e-4f, min(max_sweeps, 20));
+        sweeps += sw < 0 ? min(max_sweeps, 20) : sw;
+        ++stages;
+        if (!unitarise<T, NT>(Vs, pc, c, S, pc, Q, pc, red)) return -1;
+        apply_unitary<T, NT>(A, ld, ell, c, Q, pc, stage, pc);
+        bulk = false;
+      }
+      gram_local<T, NT>(A, ld, ell, c, G, pc, stage, pc);
+      float fro = 0.f;
+      for (int j = 0; j < c; ++j) fro += lead(G[j * pc + j].x);
+      const float tiny2 = fmaxf(fro * floor_t * floor_t, 1e-37f);
+      // K of every pair above the threshold, r = |g| / (|a_p| |a_q|) and |t|
+      float rmax = 0.f, kmax = 0.f;
+      for (int e = tid; e < c * (c + 1) / 2; e += NT) {
+        int p, q;
+        tri_entry(e, c, p, q);
+        if (p == q) {
+          Vs[p * pc + p] = mkc<float>(1.f, 0.f);
+          continue;
+        }
+        cpx<float> vpq = czero<float>(), vqp = czero<float>();
+        const T at_ = G[p * pc + p].x, bt_ = G[q * pc + q].x;
+        const float a = lead(at_), b = lead(bt_);
+        if (a > tiny2 && b > tiny2) {
+          const cpx<T> g = G[p * pc + q];
+          const float sc = rsqrtf(a) * rsqrtf(b);
+          const float hx = lead(g.x) * sc, hy = lead(g.y) * sc, r2 = fmaf(hx, hx, hy * hy), r = sqrtf(r2);
+          rmax = fmaxf(rmax, r);
+          if (r > tol) {
+            const float rr = 1.f / r;
+            const float z = 0.5f * (lead(bt_ - at_) * sc) * rr;
+            const float z1 = fmaf(z, z, 1.f);
+            const float t = fabsf(z) > 1e15f ? 0.5f / z : copysignf(1.f / (fabsf(z) + sqrtf(z1)), z);
+            kmax = fmaxf(kmax, fabsf(t));
+            const float ex = hx * rr, ey = -hy * rr;
+            vqp = mkc<float>(-t * ex, -t * ey);
+            vpq = mkc<float>(t * ex, -t * ey);
+          }
+        }
+        Vs[p * pc + q] = vqp;  // column p, row q
+        Vs[q * pc + p] = vpq;  // column q, row p
+      }
+      rmax = block_max<NT>(rmax, red);
+      kmax = block_max<NT>(kmax, red);
+      if (!(rmax < 2.f)) return -1;  // not a number
+      if (rmax <= tol) return sweeps + 1;
+      ++sweeps;
+      // the pairs left after this step are of order r times the largest angle
+      const bool last = rmax * kmax * 8.f <= tol;
+      if (kmax <= kFloatApply) {
+        apply_small<T, NT>(A, ld, ell, c, Vs, pc, reinterpret_cast<cpx<float> *>(stage), pc);
+      } else if (rmax > 1e-3f && kmax > 0.3f && stages < kMaxStages) {
+        bulk = true;  // far from converged: vectors that the float stage had left alone
+        __syncthreads();
+        continue;
+      } else {
+        if (!unitarise<T, NT>(Vs, pc, c, S, pc, Q, pc, red)) return -1;
+        apply_unitary<T, NT>(A, ld, ell, c, Q, pc, stage, pc);
+      }
+      if (last) return sweeps + 1;
+    }
+    return -1;
+  }
+}
+
+// In-place Cholesky S = L L^H of an n x n Hermitian matrix in shared memory
+// (pitch ps; the lower triangle becomes L).  Same rule as cholesky_lower: false
+// when a pivot falls below `rel` times its original diagonal.
+template <typename T, int NT>
+__device__ bool cholesky_local(cpx<T> *S, int ps, int n, float rel, T *diag0) {
+  for (int i = threadIdx.x; i < n; i += NT) diag0[i] = S[i * ps + i].x;
+  __syncthreads();
+  for (int k = 0; k < n; ++k) {
+    const T d = S[k * ps + k].x;
+    if (!(lead(d) > rel * lead(diag0[k])) || !(lead(d) > 0.f)) return false;  // uniform: every thread read the same
+    __syncthreads();
+    if (threadIdx.x < 32 || int(threadIdx.x) < n) {  // whole warps that hold a row below the pivot
+      const T l = sqrt(d), il = T(1) / l;
+      for (int i = k + 1 + threadIdx.x; i < n; i += NT) S[i * ps + k] = cscale(S[i * ps + k], il);
+      if (threadIdx.x == 0) S[k * ps + k] = mkc<T>(l, T(0));
+    }
+    __syncthreads();
+    const int rem = n - k - 1;
+    for (int idx = threadIdx.x; idx < rem * rem; idx += NT) {
+      const int i = k + 1 + idx / rem, j = k + 1 + idx % rem;
+      if (j > i) continue;
+      const cpx<T> li = S[i * ps + k], lj = S[j * ps + k];
+      cpx<T> v = S[i * ps + j];
+      v.x -= li.x * lj.x + li.y * lj.y;
+      v.y -= li.y * lj.x - li.x * lj.y;
+      S[i * ps + j] = v;
+    }
+    __syncthreads();
+  }
+  return true;
+}
+
+// ------------------------------------------------------------- bond operation
+// Shared-memory plan of bond_local.  theta (T0) and the vectors (A) are
+// vector-contiguous with an odd pitch, so that lanes that walk over vectors
+// hit different banks.  Taken when theta is at most 64 x 64 (chi <= 32: beyond,
+// the products want register tiles) and everything fits.
+template <typename T>
+struct LocalBond {
+  static constexpr int MAXM = 64;
+  size_t theta, vec, svd, lam, vals, total;
+  __host__ __device__ static size_t al(size_t x) { return (x + 15) & ~size_t(15); }
+  __host__ __device__ static size_t most(size_t a, size_t b) { return a > b ? a : b; }
+  __host__ __device__ bool plan(int cL, int cM, int cR, bool lq, size_t room, int nt) {
+    const int m = 2 * cL, nc = 2 * cR, c = m < nc ? m : nc, ell = m < nc ? nc : m;
+    if (ell > MAXM || cM > MAXM || c > LocalSvd<T>::max_c(nt)) return false;
+    const size_t e = sizeof(cpx<T>);
+    theta = al(size_t(c) * (ell | 1) * e);
+    vec = theta;
+    svd = LocalSvd<T>::bytes(ell, c);
+    if (lq) {  // cM vectors of length m, theta as columns; and room for the direct path if it falls back
+      theta = most(theta, al(size_t(nc) * (m | 1) * e));
+      vec = most(vec, al(size_t(cM) * (m | 1) * e));
+      svd = most(svd, LocalSvd<T>::bytes(m, cM));
+      svd = most(svd, al(size_t(cM) * (cM | 1) * e) + al(size_t(cM) * sizeof(T)));
+    }
+    lam = al(size_t(2) * (cL + cM + cR) * sizeof(T));
+    vals = al(size_t(c) * (3 * sizeof(double) + 3 * sizeof(T) + sizeof(int))) + 128;
+    total = theta + vec + svd + lam + vals;
+    return total <= room;
+  }
+};
+
+// Sums of two values over the CTA in the arithmetic R (uniform result).
+template <typename R, int NT>
+__device__ __forceinline__ void block_sum2_in(R &a, R &b, double *red) {
+  R *r = reinterpret_cast<R *>(red);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a = a + shfl_xor(a, o);
+    b = b + shfl_xor(b, o);
+  }
+  __syncthreads();
+  if (lane == 0) {
+    r[warp] = a;
+    r[NT / 32 + warp] = b;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    a = lane < NT / 32 ? r[lane] : R(0);
+    b = lane < NT / 32 ? r[NT / 32 + lane] : R(0);
+#pragma unroll
+    for (int o = NT / 64; o > 0; o >>= 1) {
+      a = a + shfl_xor(a, o);
+      b = b + shfl_xor(b, o);
+    }
+    if (lane == 0) {
+      r[2 * (NT / 32)] = a;
+      r[2 * (NT / 32) + 1] = b;
+    }
+  }
+  __syncthreads();
+  a = r[2 * (NT / 32)];
+  b = r[2 * (NT / 32) + 1];
+}
+
+// What bond_local leaves behind.
+struct LocalResult {
+  bool done = false;  // the bond is finished; else theta and the vectors are in the global workspace
+  bool svd_done = false;  // (general path) svd_local has orthogonalised the vectors
+  bool lq = false, colmode = false;
+  int ell = 0, c = 0, sweeps = 0;
+};
+
+}  // namespace tn
