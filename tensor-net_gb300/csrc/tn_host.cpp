@@ -240,7 +240,7 @@ int mps_alloc(tn_mps *m) {
   CK(m->chi.ensure(sizeof(int) * (m->n + 1)));
   CK(m->status.ensure(sizeof(int)));
   CK(m->dtraj.ensure(sizeof(TrajDev)));
-  CK(m->stats.ensure(sizeof(double) * STAT_N));
+  CK(m->stats.ensure(sizeof(double) * (STAT_N + 2)));  // counters, then two values of an observable
   CK(cudaMemsetAsync(m->stats.p, 0, sizeof(double) * STAT_N, m->st));
   TrajDev &d = m->h;
   d.stats = m->stats.as<double>();
@@ -367,6 +367,21 @@ int mps_run(tn_mps *m, const std::vector<Instr> &prog, const std::vector<double>
     sync = true;
   }
   if (sync) CK(cudaStreamSynchronize(m->st));
+  return TN_OK;
+}
+
+// Observable of the state (launch_observe) into nout host values; `instr` is
+// the same read for the executor, where the bond capacity is too large for it.
+int mps_observe(tn_mps *m, const Instr &instr, double alpha, int nout, double *out) {
+  if (!observe_fits(m->prec, int(m->cap))) {
+    if (instr.op == OP_PROBS)
+      return mps_run(m, {instr}, {}, {}, 0, nullptr, nullptr, 0, nullptr, 1, out);
+    return mps_run(m, {instr}, {}, {alpha}, 0, nullptr, nullptr, 1, out, 0, nullptr);
+  }
+  double *dout = m->stats.as<double>() + STAT_N;
+  CK(launch_observe(m->prec, m->dtraj.as<TrajDev>(), int(m->cap), instr.op, instr.k, alpha, dout, m->st));
+  CK(cudaMemcpyAsync(out, dout, sizeof(double) * nout, cudaMemcpyDeviceToHost, m->st));
+  CK(cudaStreamSynchronize(m->st));
   return TN_OK;
 }
 
@@ -596,9 +611,8 @@ int tn_mps_apply_unitary1(tn_mps *m, uint32_t k, const double *op, uint32_t rows
   if (k >= m->n) return TN_OK;
   if (!gate_shape_ok(rows, cols, 2)) return TN_ERR_OPERATOR_SHAPE;
   if (!all_finite(op, 8)) return TN_ERR_INVALID_ARG;
-  std::vector<double> g(32, 0.0);
-  std::memcpy(g.data(), op, 8 * sizeof(double));
-  return mps_run(m, {Instr{OP_UNI1, int(k), 0, 0}}, g, {}, 0, nullptr, nullptr, 0, nullptr, 0, nullptr);
+  CK(launch_unitary1(m->prec, m->dtraj.as<TrajDev>(), int(m->cap), int(k), op, m->st));
+  return TN_OK;
 }
 
 int tn_mps_apply_unitary2(tn_mps *m, uint32_t k, const double *op, uint32_t rows, uint32_t cols) {
@@ -614,7 +628,7 @@ int tn_mps_probs(const tn_mps *cm, uint32_t k, double out[2]) {
   tn_mps *m = const_cast<tn_mps *>(cm);
   if (!m || !out) return TN_ERR_INVALID_ARG;
   if (k >= m->n) return TN_NONE;
-  return mps_run(m, {Instr{OP_PROBS, int(k), 0, 0}}, {}, {}, 0, nullptr, nullptr, 0, nullptr, 1, out);
+  return mps_observe(m, Instr{OP_PROBS, int(k), 0, 0}, 0.0, 2, out);
 }
 
 int tn_mps_prob(const tn_mps *m, uint32_t k, uint32_t p, double *out) {
@@ -750,7 +764,7 @@ int tn_mps_entropy_vn(const tn_mps *cm, uint32_t b, double *out) {
   tn_mps *m = const_cast<tn_mps *>(cm);
   if (!m || !out) return TN_ERR_INVALID_ARG;
   if (m->n < 2 || b >= m->n - 1) return TN_NONE;
-  return mps_run(m, {Instr{OP_ENTROPY, int(b), 0, 0}}, {}, {}, 0, nullptr, nullptr, 1, out, 0, nullptr);
+  return mps_observe(m, Instr{OP_ENTROPY, int(b), 0, 0}, 1.0, 1, out);
 }
 
 int tn_mps_entropy_ry_schmidt(const tn_mps *cm, double a, uint32_t b, double *out) {
@@ -758,7 +772,7 @@ int tn_mps_entropy_ry_schmidt(const tn_mps *cm, double a, uint32_t b, double *ou
   if (!m || !out) return TN_ERR_INVALID_ARG;
   if (a == 1.0) return tn_mps_entropy_vn(cm, b, out);
   if (m->n < 2 || b >= m->n - 1) return TN_NONE;
-  return mps_run(m, {Instr{OP_RENYI, int(b), 0, 0}}, {}, {a}, 0, nullptr, nullptr, 1, out, 0, nullptr);
+  return mps_observe(m, Instr{OP_RENYI, int(b), 0, 0}, a, 1, out);
 }
 
 int tn_mps_bond_dim(const tn_mps *m, uint32_t b, uint32_t *out) {

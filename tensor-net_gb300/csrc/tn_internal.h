@@ -119,6 +119,12 @@ cudaError_t launch_run(int prec, const LaunchArgs &la, int grid, int sortP, int 
 size_t run_smem_bytes(int prec, int sortP);
 size_t run_work_bytes(int prec, int cap);
 int run_blocks_per_sm(int prec, int sortP);
+// Observables of one state, outside the executor: op = OP_PROBS (k = site,
+// two values), OP_ENTROPY or OP_RENYI (k = bond, alpha; one value) into out.
+bool observe_fits(int prec, int cap);  // the bond capacity is within its shared memory
+cudaError_t launch_observe(int prec, const TrajDev *traj, int cap, int op, int k, double alpha, double *out,
+                           cudaStream_t st);
+cudaError_t launch_unitary1(int prec, const TrajDev *traj, int cap, int k, const double *op, cudaStream_t st);
 cudaError_t launch_reset(TrajDev *trajs, const int *list, int count, int prec, cudaStream_t st);
 // posts (may be null): per measurement, 0 / 1 = post-selected outcome (Meas::Proj), else sampled
 cudaError_t launch_compile(const TrajDev *trajs, const int *list, int nt, const int *order, const int *gate_off,

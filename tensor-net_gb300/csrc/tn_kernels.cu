@@ -291,6 +291,85 @@ int run_blocks_per_sm(int prec, int sortP) {
   return prec == 0 ? run_blocks_f64(sortP) : (prec == 2 ? run_blocks_df(sortP) : run_blocks_f32(sortP));
 }
 
+// Observables (and one-site gates) of a single state without the executor:
+// its arguments arrive by value, so a read is one launch and one copy back
+// instead of four copies in, a launch of the whole executor and a copy back
+// (read of an entropy, a Renyi entropy and site probabilities at n = 16,
+// chi = 64: 100 us before, see k_observe's caller).  Bound by launch latency.
+constexpr int kObserveThreads = 256;
+
+template <typename T>
+__global__ void __launch_bounds__(kObserveThreads) k_observe(const TrajDev *traj, int op, int k, double alpha,
+                                                             double *out) {
+  extern __shared__ __align__(256) unsigned char osm[];
+  Smem<T, kBlockW> sm(osm, 1);
+  const TrajDev tr = *traj;
+  if (op == OP_PROBS) {
+    double p0, p1;
+    site_probs<T, kObserveThreads, kBlockW>(tr, k, p0, p1, sm);
+    if (threadIdx.x == 0) {
+      out[0] = p0;
+      out[1] = p1;
+    }
+  } else {
+    const double e = bond_entropy<kObserveThreads>(tr, k, alpha, sm.red);
+    if (threadIdx.x == 0) out[0] = e;
+  }
+}
+
+struct Op1 {
+  double v[8];
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kObserveThreads) k_unitary1(const TrajDev *traj, int k, Op1 op) {
+  const TrajDev tr = *traj;
+  const int cL = tr.chi[k], cR = tr.chi[k + 1];
+  cpx<T> *g = gamma_slot<T>(tr, k);
+  const cpx<T> o00 = mkc<T>(T(op.v[0]), T(op.v[1])), o01 = mkc<T>(T(op.v[2]), T(op.v[3]));
+  const cpx<T> o10 = mkc<T>(T(op.v[4]), T(op.v[5])), o11 = mkc<T>(T(op.v[6]), T(op.v[7]));
+  for (size_t idx = blockIdx.x * size_t(blockDim.x) + threadIdx.x; idx < size_t(cL) * cR;
+       idx += size_t(gridDim.x) * blockDim.x) {
+    const size_t v = idx / cR, u = idx % cR;
+    const cpx<T> a = g[(v * 2 + 0) * cR + u], b = g[(v * 2 + 1) * cR + u];
+    g[(v * 2 + 0) * cR + u] = cfma(o01, b, cmul(o00, a));
+    g[(v * 2 + 1) * cR + u] = cfma(o11, b, cmul(o10, a));
+  }
+}
+
+template <typename T>
+static cudaError_t launch_observe_t(const TrajDev *traj, int cap, int op, int k, double alpha, double *out,
+                                    cudaStream_t st) {
+  // site_probs keeps the squared Lambdas of both bonds in shared memory
+  const size_t smem = SmemLayout<T, kBlockW>::head_bytes + 2 * size_t(cap) * sizeof(T);
+  if (smem > 48 * 1024) return cudaErrorInvalidValue;
+  k_observe<T><<<1, kObserveThreads, smem, st>>>(traj, op, k, alpha, out);
+  return cudaGetLastError();
+}
+
+bool observe_fits(int prec, int cap) { return 2048 + 2 * size_t(cap) * (prec == 1 ? 4 : 8) <= 48 * 1024; }
+
+cudaError_t launch_observe(int prec, const TrajDev *traj, int cap, int op, int k, double alpha, double *out,
+                           cudaStream_t st) {
+  if (prec == 0) return launch_observe_t<double>(traj, cap, op, k, alpha, out, st);
+  if (prec == 2) return launch_observe_t<dd>(traj, cap, op, k, alpha, out, st);
+  return launch_observe_t<float>(traj, cap, op, k, alpha, out, st);
+}
+
+cudaError_t launch_unitary1(int prec, const TrajDev *traj, int cap, int k, const double *op, cudaStream_t st) {
+  Op1 o;
+  for (int i = 0; i < 8; ++i) o.v[i] = op[i];
+  const size_t blocks = (size_t(cap) * cap + kObserveThreads - 1) / kObserveThreads;
+  const int grid = int(blocks < 64 ? blocks : 64);
+  if (prec == 0)
+    k_unitary1<double><<<grid, kObserveThreads, 0, st>>>(traj, k, o);
+  else if (prec == 2)
+    k_unitary1<dd><<<grid, kObserveThreads, 0, st>>>(traj, k, o);
+  else
+    k_unitary1<float><<<grid, kObserveThreads, 0, st>>>(traj, k, o);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_reset(TrajDev *trajs, const int *list, int count, int prec, cudaStream_t st) {
   if (count <= 0) return cudaSuccess;
   k_reset<<<count, 128, 0, st>>>(trajs, list, count, prec);
