@@ -71,6 +71,7 @@ struct tn_batch {
   double *dstats = nullptr;
   void *ws = nullptr;
   size_t ws_stride = 0;
+  bool ws_team = false;
   // step buffers: one packed device block + one pinned host block
   void *dstep = nullptr, *hstep = nullptr;
   size_t step_bytes = 0;
@@ -277,6 +278,7 @@ int launch_step(tn_batch *b, uint32_t nt, const StepPtrs &P0, bool timed = true)
   la.pout = P.probs;
   la.ws = b->ws;
   la.ws_stride = b->ws_stride;
+  la.ws_team = b->ws_team;
   la.max_sweeps = b->max_sweeps;
   la.jacobi_scheme = b->scheme;
   la.theta_simt = b->theta_simt;
@@ -444,8 +446,7 @@ int tn_batch_create(uint32_t ntraj, const uint32_t *ns, const tn_trunc *truncs, 
   b->bps = run_blocks_per_sm(precision, b->sortP);
   b->grid_max = std::max(1, b->sms * b->bps);
   b->grid_max = std::min<int>(b->grid_max, int(std::max<uint32_t>(ntraj, b->sum_n / 2)));
-  b->ws_stride = run_work_bytes(precision, b->maxcap);
-  e = cudaMalloc(&b->ws, b->ws_stride * b->grid_max);
+  e = alloc_work(precision, b->maxcap, b->grid_max, &b->ws, &b->ws_stride, &b->ws_team);
   if (e != cudaSuccess) return bail(fail(e, "cudaMalloc(workspace)"));
   b->pcap = 4 * b->maxn + 8;
   // reset all slots to |0...0>
@@ -966,8 +967,7 @@ tn_batch *batch_engine_create(uint32_t slots, int prec, int ws_cap, int max_n, i
   b->bps = run_blocks_per_sm(prec, b->sortP);
   b->grid_max = std::max(1, b->sms * b->bps);
   if (grid_limit > 0) b->grid_max = std::min(b->grid_max, grid_limit);
-  b->ws_stride = run_work_bytes(prec, b->maxcap);
-  e = cudaMalloc(&b->ws, b->ws_stride * b->grid_max);
+  e = alloc_work(prec, b->maxcap, b->grid_max, &b->ws, &b->ws_stride, &b->ws_team);
   if (e != cudaSuccess) return bail(fail(e, "cudaMalloc(workspace)"));
   b->pcap = 4 * max_n + 8;
   e = cudaStreamSynchronize(b->st);

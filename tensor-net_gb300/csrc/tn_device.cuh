@@ -310,6 +310,9 @@ struct SmemLayout {
   __host__ __device__ static size_t total(int P) { return head_bytes + arena_bytes(P); }
 };
 
+template <typename T>
+size_t __host__ __device__ team_bytes(int cap);
+
 template <typename T, int W>
 struct Smem {
   unsigned char *r0;
@@ -319,12 +322,14 @@ struct Smem {
   // tensor-core state of the CTA (float executor): accumulator columns in
   // tensor memory, the MMA-completion mbarrier and its phase
   uint64_t *bar = nullptr;
-  uint32_t tmem = 0, phase = 0;
+  uint64_t *gbar = nullptr;  // two more mbarriers: the stages of oz_gemm
+  uint32_t tmem = 0, phase = 0, gphase = 0;
   bool tc = false;
   bool tc_fail = false;  // an MMA wait ran past its limit during the current bond op
   unsigned char *oz = nullptr;  // double-float executor: tensor-core update staging (1024-byte aligned)
   size_t arena;                 // bytes from r0 on
-  __device__ Smem(unsigned char *base, int P) {
+  unsigned char *base;
+  __device__ Smem(unsigned char *base_, int P) : base(base_) {
     using L = SmemLayout<T, W>;
     unsigned char *p = base;
     red = reinterpret_cast<double *>(p);
@@ -360,6 +365,7 @@ struct Work {
   T *isig;       // 2*cap: 1/sigma_j and (after cap*2) 1/sigma_j^2 of the kept values
   T *isig2;
   T *w2;         // 2*cap: s2_j^2 in the working precision
+  void *team = nullptr;  // workspace of svd_team (team_work), or none
 };
 
 template <typename T>
@@ -371,8 +377,9 @@ __host__ __device__ inline size_t work_bytes(int cap) {
 }
 
 template <typename T>
-__device__ inline Work<T> make_work(void *base, int cap) {
+__device__ inline Work<T> make_work(void *base, int cap, bool team) {
   Work<T> w;
+  w.team = team && team_bytes<T>(cap) ? reinterpret_cast<unsigned char *>(base) + work_bytes<T>(cap) : nullptr;
   unsigned char *p = reinterpret_cast<unsigned char *>(base);
   size_t n4 = size_t(4) * cap * cap;
   w.A = reinterpret_cast<cpx<T> *>(p);
@@ -412,6 +419,14 @@ __device__ __forceinline__ void rr_pair(int r, int t, int &p, int &q) {
   q = a < b ? b : a;
 }
 
+// 1 / sqrt(x) with one Newton step: the hardware's approximation is biased, and
+// rotations scaled by it shrink a column a little more each time (3e-5 over the
+// sweeps of 80 vectors).
+__device__ __forceinline__ float rsqrt_near(float x) {
+  const float r = rsqrtf(x);
+  return fmaf(r, fmaf(-0.5f * x * r, r, 0.5f), r);
+}
+
 }  // namespace tn
 #include "tn_local.cuh"
 namespace tn {
@@ -424,7 +439,7 @@ namespace tn {
 // theta[i][j] (vectors = columns, m > nc), else A[i*nc + j] = theta[i][j].
 // =======================================================================
 template <typename T, int NT, int W>
-__device__ void build_theta(const cpx<T> *__restrict__ gk, const cpx<T> *__restrict__ gk1,
+__device__ __noinline__ void build_theta(const cpx<T> *__restrict__ gk, const cpx<T> *__restrict__ gk1,
                             const T *__restrict__ lamL, const T *__restrict__ lamM,
                             const T *__restrict__ lamR, int cL, int cM, int cR,
                             const double *__restrict__ gate, cpx<T> *__restrict__ A, cpx<T> *__restrict__ T0,
@@ -552,7 +567,7 @@ __device__ bool wait_mma(Smem<T, W> &sm) {
 template <int NT, int W>
 __device__ bool build_theta_tc(const cpx<float> *gk, const cpx<float> *gk1, const float *lamL, const float *lamM,
                                const float *lamR, int cL, int cM, int cR, const double *gate, cpx<float> *A,
-                               cpx<float> *T0, bool colmode, Smem<float, W> &sm) {
+                               cpx<float> *T0, bool colmode, Smem<float, W> &sm, int rank = 0, int size = 1) {
   constexpr int MT = 128, NTL = 256, KC = 32, WT = NTL / 4;
   constexpr uint32_t IDESC = tc::idesc_tf32(MT, NTL);
   constexpr uint32_t LBO = 128, SBO = KC * 32;
@@ -568,8 +583,10 @@ __device__ bool build_theta_tc(const cpx<float> *gk, const cpx<float> *gk1, cons
   }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   bool ok = true;
+  int tile = 0;
   for (int i0 = 0; i0 < m; i0 += MT) {
     for (int w0 = 0; w0 < cR; w0 += WT) {
+      if (tile++ % size != rank) continue;  // another member's tile
       int chunk = 0;
       for (int k0 = 0; k0 < K2; k0 += KC, ++chunk) {
         if (chunk > 0) ok = wait_mma<float, W>(sm) && ok;  // the staging tiles are free again
@@ -1511,7 +1528,7 @@ template <typename T, int NT, int W>
 __device__ void bitonic_desc(double *key, int *idx, int P);
 
 template <typename T, int NT, int W>
-__device__ int jacobi_svd(cpx<T> *__restrict__ A, int ell, int c, int max_sweeps, Smem<T, W> &sm,
+__device__ __noinline__ int jacobi_svd(cpx<T> *__restrict__ A, int ell, int c, int max_sweeps, Smem<T, W> &sm,
                           long long *cyc, double *__restrict__ nrm, int *__restrict__ ord, int scheme) {
   using L = SmemLayout<T, W>;
   constexpr int B = W / 2;
@@ -1906,7 +1923,7 @@ __device__ void gemm_nt(int M, int N, int K, FP P, FQ Q, FE E, Smem<T, W> &sm) {
 // stores.  Staging tiles in the resident Jacobi block's shared memory, which
 // is idle outside the Jacobi.
 template <int NT, int W, class FP, class FQ, class FE>
-__device__ bool gemm_nt_tc(int M, int N, int K, FP P, FQ Q, FE E, Smem<float, W> &sm) {
+__device__ bool gemm_nt_tc(int M, int N, int K, FP P, FQ Q, FE E, Smem<float, W> &sm, int rank = 0, int size = 1) {
   constexpr int MT = 128, NTL = 256, KC = 32, YT = NTL / 2;
   constexpr uint32_t IDESC = tc::idesc_tf32(MT, NTL);
   constexpr uint32_t LBO = 128, SBO = KC * 32;
@@ -1914,8 +1931,10 @@ __device__ bool gemm_nt_tc(int M, int N, int K, FP P, FQ Q, FE E, Smem<float, W>
   const int K2 = 2 * K;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   bool ok = true;
+  int tile = 0;
   for (int i0 = 0; i0 < M; i0 += MT) {
     for (int y0 = 0; y0 < N; y0 += YT) {
+      if (tile++ % size != rank) continue;  // another member's tile
       int chunk = 0;
       for (int k0 = 0; k0 < K2; k0 += KC, ++chunk) {
         if (chunk > 0) ok = wait_mma<float, W>(sm) && ok;
@@ -1999,8 +2018,13 @@ __device__ bool gemm_nt_auto(int M, int N, int K, FP P, FQ Q, FE E, Smem<T, W> &
   return true;
 }
 
+}  // namespace tn
+#include "tn_oz.cuh"
+#include "tn_team.cuh"
+namespace tn {
+
 template <typename T, int NT, int W>
-__device__ void finalize_bond(const TrajDev &tr, int k, cpx<T> *__restrict__ gk, cpx<T> *__restrict__ gk1,
+__device__ __noinline__ void finalize_bond(const TrajDev &tr, int k, cpx<T> *__restrict__ gk, cpx<T> *__restrict__ gk1,
                               const double *__restrict__ lamL, double *__restrict__ lamM,
                               const double *__restrict__ lamR, int cL, int cR, bool colmode, int ell, int c,
                               Work<T> &wk, Smem<T, W> &sm) {
@@ -2156,17 +2180,24 @@ __device__ __forceinline__ double *lam_slot(const TrajDev &tr, int s) { return t
 // a pivot falls below `rel` times the original diagonal entry, i.e. when the
 // rows behind S are far from orthonormal.
 template <typename T, int NT, int W>
-__device__ bool cholesky_lower(cpx<T> *__restrict__ S, int n, double rel, double *__restrict__ diag0,
+__device__ __noinline__ bool cholesky_lower(cpx<T> *__restrict__ S, int n, double rel, double *__restrict__ diag0,
                                Smem<T, W> &sm) {
+  // The pivot's square root and reciprocal are worked out by the warps that
+  // scale its column, in double-float unless the precision is float64: float64
+  // ones repeated by 16 warps cost 10 000 cycles a pivot.
+  using R = typename RedType<T>::type;
   for (int i = threadIdx.x; i < n; i += NT) diag0[i] = double(S[size_t(i) * n + i].x);
   __syncthreads();
   for (int k = 0; k < n; ++k) {
-    const double d = double(S[size_t(k) * n + k].x);
-    if (!(d > rel * diag0[k]) || !(d > 0.0)) return false;  // uniform: every thread read the same value
-    const T l = T(sqrt(d)), il = T(1.0 / sqrt(d));
+    const T d = S[size_t(k) * n + k].x;
+    const float df = lead(d);
+    if (!(df > float(rel) * float(diag0[k])) || !(df > 0.f)) return false;  // uniform: every thread read the same value
     __syncthreads();
-    for (int i = k + 1 + threadIdx.x; i < n; i += NT) S[size_t(i) * n + k] = cscale(S[size_t(i) * n + k], il);
-    if (threadIdx.x == 0) S[size_t(k) * n + k] = mkc<T>(l, T(0));
+    if (threadIdx.x < 32 || int(threadIdx.x & ~31u) < n - k - 1) {
+      const R l = sqrt(R(d)), il = R(1) / l;
+      for (int i = k + 1 + threadIdx.x; i < n; i += NT) S[size_t(i) * n + k] = cscale(S[size_t(i) * n + k], T(il));
+      if (threadIdx.x == 0) S[size_t(k) * n + k] = mkc<T>(T(l), T(0));
+    }
     __syncthreads();
     const int rem = n - k - 1;
     for (int idx = threadIdx.x; idx < rem * rem; idx += NT) {
@@ -2195,7 +2226,7 @@ __device__ bool cholesky_lower(cpx<T> *__restrict__ S, int n, double rel, double
 // passes.  Returns false (and leaves theta in wk.T0 untouched) when B is too
 // far from orthonormal rows for the factorisation to be accurate.
 template <typename T, int NT, int W>
-__device__ bool refactor_lq(const cpx<T> *__restrict__ gk, const cpx<T> *__restrict__ gk1,
+__device__ __noinline__ bool refactor_lq(const cpx<T> *__restrict__ gk, const cpx<T> *__restrict__ gk1,
                             const T *__restrict__ lamL, const T *__restrict__ lamM,
                             const T *__restrict__ lamR, int cL, int cM, int cR, int cap, Work<T> &wk,
                             Smem<T, W> &sm) {
@@ -2224,13 +2255,16 @@ __device__ bool refactor_lq(const cpx<T> *__restrict__ gk, const cpx<T> *__restr
 // A bond operation held in shared memory from theta to the new Gammas (plan
 // pl).  Same steps and rules as bond_op's general path: theta and the gate,
 // LQ reduction of refactors, SVD, process_svd, Gamma rebuild, renormalisation.
-template <typename T, int NT, int W>
-__device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, const double *gate, const LocalBond<T> &pl, bool try_lq,
-                                  int max_sweeps, Work<T> &wk, Smem<T, W> &sm, long long *cyc) {
+template <typename TS, int NT, int W>
+__device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL, int cM, int cR, const double *gate,
+                                               const LocalBond<typename LocalType<TS>::type> &pl, bool try_lq,
+                                               int max_sweeps, Work<TS> &wk, Smem<TS, W> &sm, long long *cyc) {
+  using T = typename LocalType<TS>::type;  // of the arithmetic; TS: of the state
   using R = typename RedType<T>::type;
+  constexpr bool kExact = std::is_same<T, TS>::value;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int cL = tr.chi[k], cM = tr.chi[k + 1], cR = tr.chi[k + 2], m = 2 * cL, nc = 2 * cR;
-  cpx<T> *gk = gamma_slot<T>(tr, k), *gk1 = gamma_slot<T>(tr, k + 1);
+  const int m = 2 * cL, nc = 2 * cR;
+  cpx<TS> *gk = gamma_slot<TS>(tr, k), *gk1 = gamma_slot<TS>(tr, k + 1);
   unsigned char *at = sm.r0;
   __builtin_assume(__isShared(at));
   cpx<T> *T0 = reinterpret_cast<cpx<T> *>(at);
@@ -2241,9 +2275,9 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, const d
   at += pl.svd;
   T *lL = reinterpret_cast<T *>(at), *lM = lL + cL, *lR = lM + cM, *sL = lR + cR, *sR = sL + cL;
   at += pl.lam;
-  double *key = reinterpret_cast<double *>(at);
   const int cmax = min(m, nc);
-  double *skey = key + cmax, *s2 = skey + cmax;
+  R *sq = reinterpret_cast<R *>(at), *ssq = sq + cmax;
+  double *s2 = reinterpret_cast<double *>(ssq + cmax);
   T *isig = reinterpret_cast<T *>(s2 + cmax), *isig2 = isig + cmax, *w2 = isig2 + cmax;
   int *perm = reinterpret_cast<int *>(w2 + cmax);
   const double *lamL = lam_slot(tr, k), *lamR = lam_slot(tr, k + 2);
@@ -2261,15 +2295,15 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, const d
       typename CAcc<T>::type acc[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[q] = acc_zero<T>();
-      const cpx<T> *x = gk + size_t(2 * v) * cM, *y = gk1 + w;
+      const cpx<TS> *x = gk + size_t(2 * v) * cM, *y = gk1 + w;
 #pragma unroll 2
       for (int u = 0; u < cM; ++u) {
         if ((u & 3) == 0) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) acc_renorm(acc[q]);
         }
-        const cpx<T> x0 = cscale(x[u], lM[u]), x1 = cscale(x[cM + u], lM[u]);
-        const cpx<T> y0 = y[size_t(2 * u) * cR], y1 = y[size_t(2 * u + 1) * cR];
+        const cpx<T> x0 = cscale(widen(x[u]), lM[u]), x1 = cscale(widen(x[cM + u]), lM[u]);
+        const cpx<T> y0 = widen(y[size_t(2 * u) * cR]), y1 = widen(y[size_t(2 * u + 1) * cR]);
         acc_fma<T>(acc[0], x0, y0);
         acc_fma<T>(acc[1], x0, y1);
         acc_fma<T>(acc[2], x1, y0);
@@ -2313,33 +2347,35 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, const d
       int p, q;
       tri_entry(e, cM, p, q);
       typename CAcc<T>::type acc = acc_zero<T>();
-      const cpx<T> *bp = gk1 + size_t(p) * nc, *bq = gk1 + size_t(q) * nc;
+      const cpx<TS> *bp = gk1 + size_t(p) * nc, *bq = gk1 + size_t(q) * nc;
 #pragma unroll 2
       for (int col = 0; col < nc; ++col) {
         const T l = lR[col < cR ? col : col - cR];
-        acc_jfma<T>(acc, cscale(bp[col], l), cscale(bq[col], l));
+        acc_jfma<T>(acc, cscale(widen(bp[col]), l), cscale(widen(bq[col]), l));
       }
       S[q * ps + p] = acc_fin<T>(acc);  // S_qp = sum B_q conj(B_p)
     }
     __syncthreads();
-    if (cholesky_local<T, NT>(S, ps, cM, sizeof(T) == 4 ? 0.1f : 1e-3f, diag0)) {
+    if (cholesky_local<T, NT>(S, ps, cM, sizeof(TS) == 4 ? 0.1f : 1e-3f, diag0)) {
       lq = true;
       const int ld = m | 1;
       gemm_exact_from<T, NT>(
           m, cM, [](int, int j) { return j; }, cM,
-          [&](int i, int u) { return cscale(gk[size_t(i) * cM + u], lL[i >> 1] * lM[u]); },
+          [&](int i, int u) { return cscale(widen(gk[size_t(i) * cM + u]), lL[i >> 1] * lM[u]); },
           [&](int j, int u) { return S[u * ps + j]; }, [&](int i, int j, cpx<T> v) { A[j * ld + i] = v; });
       colmode = true;
       ell = m;
       c = cM;
     } else {
       __syncthreads();
+      res.declined = true;
+      return res;
     }
   }
   theta(colmode, lq ? nullptr : A);
   const int ld = ell | 1;
   const long long c1 = clock64();
-  const int sw = c > 1 ? svd_local<T, NT>(A, ld, ell, c, max_sweeps, scratch, sm.red) : 1;
+  const int sw = c > 1 ? svd_local<T, NT>(A, ld, ell, c, max_sweeps, scratch, sm.red, kExact ? svd_tolerance<T>(ell) : 1e-8f) : 1;
   const long long c2 = clock64();
   cyc[0] = c1 - c0;
   cyc[1] = c2 - c1;
@@ -2351,19 +2387,18 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, const d
   if (sw < 0) {  // go on in the global workspace
     __syncthreads();
     const int nv = colmode ? nc : m;
-    for (int idx = tid; idx < c * ell; idx += NT) wk.A[idx] = A[(idx / ell) * ld + idx % ell];
-    for (int idx = tid; idx < nv * ell; idx += NT) wk.T0[idx] = T0[(idx / ell) * ld + idx % ell];
-    for (int v = tid; v < cL; v += NT) wk.lam3[v] = lL[v];
-    for (int u = tid; u < cM; u += NT) wk.lam3[tr.cap + u] = lM[u];
-    for (int w = tid; w < cR; w += NT) wk.lam3[2 * tr.cap + w] = lR[w];
+    for (int idx = tid; idx < c * ell; idx += NT) wk.A[idx] = narrow<TS>(A[(idx / ell) * ld + idx % ell]);
+    for (int idx = tid; idx < nv * ell; idx += NT) wk.T0[idx] = narrow<TS>(T0[(idx / ell) * ld + idx % ell]);
+    for (int v = tid; v < cL; v += NT) wk.lam3[v] = TS(lL[v]);
+    for (int u = tid; u < cM; u += NT) wk.lam3[tr.cap + u] = TS(lM[u]);
+    for (int w = tid; w < cR; w += NT) wk.lam3[2 * tr.cap + w] = TS(lR[w]);
     __syncthreads();
     return res;
   }
-  // process_svd: norms (working-precision terms, summed in R), order, rank
-  // rule and factors.  Square roots and divisions in float64 run in the few
-  // threads that own a value: repeated by every warp they would cost more
-  // than the products.
-  R *sq = reinterpret_cast<R *>(skey);
+  // process_svd on the squared norms (working-precision terms, summed in R):
+  // order, rank rule s_j / ||s|| > eps, kept values.  float64 square roots and
+  // divisions only where a stored Lambda needs one, in one warp: repeated by
+  // every warp, or chained, they would cost more than the products.
   for (int j = warp; j < c; j += NT / 32) {
     T part = T(0);
     for (int i = lane; i < ell; i += 32) part += cabs2(A[j * ld + i]);
@@ -2373,28 +2408,28 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, const d
     if (lane == 0) sq[j] = s;
   }
   __syncthreads();
-  for (int j = tid; j < c; j += NT) key[j] = sqrt(double(sq[j]));
-  __syncthreads();
   for (int j = tid; j < c; j += NT) {
-    const double x = key[j];
+    const R x = sq[j];
     int rk = 0;
-    for (int i = 0; i < c; ++i) rk += (key[i] > x || (key[i] == x && i < j)) ? 1 : 0;
+    for (int i = 0; i < c; ++i) rk += (sq[i] > x || (sq[i] == x && i < j)) ? 1 : 0;
     rk = min(rk, c - 1);
-    skey[rk] = x;
+    ssq[rk] = x;
     perm[rk] = j;
   }
   __syncthreads();
   if (warp == 0) {
-    double n1 = 0.0;
-    for (int j = lane; j < c; j += 32) n1 += skey[j] * skey[j];
+    R tot = R(0);
+    for (int j = lane; j < c; j += 32) tot = tot + ssq[j];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) n1 += __shfl_xor_sync(0xffffffffu, n1, o);
-    n1 = sqrt(n1);
+    for (int o = 16; o > 0; o >>= 1) tot = tot + shfl_xor(tot, o);
     const int mode = tr.trunc_mode;
-    const double eps = fmax((mode == 2 || mode == 3) ? fabs(tr.cutoff) : 2.220446049250313e-16, rank_floor<T>(ell));
+    const double eps = fmax((mode == 2 || mode == 3) ? fabs(tr.cutoff) : 2.220446049250313e-16, rank_floor<TS>(ell));
+    const double least = eps * eps * double(tot);
     int bad = c;
-    for (int j = lane; j < c; j += 32)
-      if (!is_normal_pos(skey[j] / n1, eps)) bad = min(bad, j);
+    for (int j = lane; j < c; j += 32) {
+      const double x = double(ssq[j]);
+      if (!(isfinite(x) && x > least && x > 0.0)) bad = min(bad, j);
+    }
     const int nlead = __reduce_min_sync(0xffffffffu, bad);
     int rank = mode == 1 ? max(1, min(max(tr.chi_max, 1), nlead))
                          : (mode == 3 ? max(1, min(tr.chi_max, nlead)) : max(nlead, 1));
@@ -2402,25 +2437,23 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, const d
       if (lane == 0) atomicOr(tr.status, ST_CAPACITY);
       rank = tr.cap;
     }
-    double n2 = 0.0;
-    for (int j = lane; j < rank; j += 32) {
-      const double s = skey[j] / n1;
-      n2 += s * s;
-    }
+    R kept = R(0);
+    for (int j = lane; j < rank; j += 32) kept = kept + ssq[j];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
-    n2 = sqrt(n2);
-    for (int j = lane; j < rank; j += 32) s2[j] = (skey[j] / n1) / n2;
+    for (int o = 16; o > 0; o >>= 1) kept = kept + shfl_xor(kept, o);
+    const double dk = double(kept);
+    for (int j = lane; j < rank; j += 32) s2[j] = sqrt(double(ssq[j]) / dk);
     if (lane == 0) {
-      sm.red[126] = n2;
+      // norm of the kept values relative to all of them
+      reinterpret_cast<R *>(sm.red)[127] = sqrt(kept / tot);
       sm.ired[0] = rank;
     }
   }
   __syncthreads();
   const int rank = sm.ired[0];
-  const R n2 = R(sm.red[126]);
+  const R n2 = reinterpret_cast<R *>(sm.red)[127];
   for (int j = tid; j < rank; j += NT) {
-    const R x = R(skey[j]), y = R(s2[j]), ix = R(1) / x;
+    const R x = sqrt(ssq[j]), y = R(s2[j]), ix = R(1) / x;
     isig[j] = T(ix);
     isig2[j] = T(ix * ix);
     w2[j] = T(y * y);
@@ -2428,26 +2461,25 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, const d
   for (int v = tid; v < cL; v += NT) sL[v] = T(R(1) / R(lamL[v]));
   for (int w = tid; w < cR; w += NT) sR[w] = T(n2 / R(lamR[w]));
   __syncthreads();
-  // Gamma_k and Gamma_{k+1} (one side from the vectors, the other recovered
-  // from theta), with the sums of local_renormalize on the way
+  // Gamma_k and Gamma_{k+1}: one side from the vectors, the other recovered
+  // from theta into the scratch; first the sums of local_renormalize, then
+  // both written once, scaled.
+  cpx<T> *rec = reinterpret_cast<cpx<T> *>(scratch);
   T pk = T(0), pk1 = T(0);
-  auto put0 = [&](int i, int j, cpx<T> u) {
-    const cpx<T> v = cscale(u, sL[i >> 1]);
-    gk[size_t(i) * rank + j] = v;
+  auto side0 = [&](int i, int j, cpx<T> u) { return cscale(u, sL[i >> 1]); };
+  auto side1 = [&](int col, cpx<T> u) { return cscale(u, sR[col < cR ? col : col - cR]); };
+  auto add0 = [&](int i, int j, cpx<T> v) {
     const T l = lL[i >> 1];
     pk += cabs2(v) * (l * l) * w2[j];
   };
-  auto put1 = [&](int j, int col, cpx<T> u) {
-    const int w = col < cR ? col : col - cR;
-    const cpx<T> v = cscale(u, sR[w]);
-    gk1[size_t(j) * nc + col] = v;
-    pk1 += cabs2(v) * w2[j] * (lR[w] * lR[w]);
+  auto add1 = [&](int j, int col, cpx<T> v) {
+    const T l = lR[col < cR ? col : col - cR];
+    pk1 += cabs2(v) * w2[j] * (l * l);
   };
+  auto direct0 = [&](int i, int j) { return side0(i, j, cscale(A[perm[j] * ld + i], isig[j])); };
+  auto direct1 = [&](int j, int col) { return side1(col, cscale(A[perm[j] * ld + col], isig[j])); };
   if (colmode) {
-    for (int o = tid; o < m * rank; o += NT) {
-      const int i = o / rank, j = o - i * rank;
-      put0(i, j, cscale(A[perm[j] * ld + i], isig[j]));
-    }
+    for (int o = tid; o < m * rank; o += NT) add0(o / rank, o % rank, direct0(o / rank, o % rank));
     gemm_exact<T, NT>(
         rank, nc, m,
         [&](int j, int i) {
@@ -2455,19 +2487,24 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, const d
           return mkc<T>(a.x, -a.y);
         },
         [&](int col, int i) { return T0[col * ld + i]; },
-        [&](int j, int col, cpx<T> v) { put1(j, col, cscale(v, isig2[j])); });
+        [&](int j, int col, cpx<T> v) {
+          v = side1(col, cscale(v, isig2[j]));
+          rec[j * nc + col] = v;
+          add1(j, col, v);
+        });
   } else {
-    for (int o = tid; o < rank * nc; o += NT) {
-      const int j = o / nc, col = o - j * nc;
-      put1(j, col, cscale(A[perm[j] * ld + col], isig[j]));
-    }
+    for (int o = tid; o < rank * nc; o += NT) add1(o / nc, o % nc, direct1(o / nc, o % nc));
     gemm_exact<T, NT>(
         m, rank, nc, [&](int i, int col) { return T0[i * ld + col]; },
         [&](int j, int col) {
           const cpx<T> a = A[perm[j] * ld + col];
           return mkc<T>(a.x, -a.y);
         },
-        [&](int i, int j, cpx<T> v) { put0(i, j, cscale(v, isig2[j])); });
+        [&](int i, int j, cpx<T> v) {
+          v = side0(i, j, cscale(v, isig2[j]));
+          rec[i * rank + j] = v;
+          add0(i, j, v);
+        });
   }
   R nk = R(pk), nk1 = R(pk1);
   block_sum2_in<R, NT>(nk, nk1, sm.red);
@@ -2482,9 +2519,8 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, const d
   }
   __syncthreads();
   const T ik = reinterpret_cast<T *>(sm.red + 100)[0], ik1 = reinterpret_cast<T *>(sm.red + 100)[1];
-  // each thread rescales what it wrote (the loops above run over the same elements)
-  for (int o = tid; o < m * rank; o += NT) gk[o] = cscale(gk[o], ik);
-  for (int o = tid; o < rank * nc; o += NT) gk1[o] = cscale(gk1[o], ik1);
+  for (int o = tid; o < m * rank; o += NT) gk[o] = narrow<TS>(cscale(colmode ? direct0(o / rank, o % rank) : rec[o], ik));
+  for (int o = tid; o < rank * nc; o += NT) gk1[o] = narrow<TS>(cscale(colmode ? rec[o] : direct1(o / nc, o % nc), ik1));
   for (int j = tid; j < rank; j += NT) lamM[j] = s2[j];
   if (tid == 0) tr.chi[k + 1] = rank;
   __syncthreads();
@@ -2493,24 +2529,40 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, const d
   return res;
 }
 
+// Work counters of one bond operation (one thread; whole numbers below 2^53,
+// in integer arithmetic to spare the thread a chain of float64 operations).
+template <typename T>
+__device__ void bond_stats(const TrajDev &tr, int cL, int cM, int cR, bool gate, bool lq, int sweeps) {
+  const long long m = 2 * cL, nc = 2 * cR, a = m > nc ? m : nc, b = m > nc ? nc : m;
+  if (lq) atomicAdd(tr.stats + STAT_LQ_OPS, 1.0);
+  atomicAdd(tr.stats + STAT_FLOP_THETA, double(8 * m * cM * nc + (gate ? 128ll * cL * cR : 0ll)));
+  atomicAdd(tr.stats + STAT_FLOP_SVD, double(4 * (4 * a * a * b + 8 * a * b * b + 9 * b * b * b)));
+  atomicAdd(tr.stats + STAT_BOND_OPS, 1.0);
+  atomicAdd(tr.stats + STAT_SWEEPS, double(sweeps));
+  // read the Gamma pair + Lambdas, write the new Gamma pair
+  const long long eb = sizeof(cpx<T>);
+  atomicAdd(tr.stats + STAT_BYTES, double(eb * 4 * (1ll * cL * cM + 1ll * cM * cR) + 8ll * (cL + cM + cR)));
+}
+
 // One bond operation on (k, k+1): gate != nullptr -> apply_unitary2, else local_refactor.
 template <typename T, int NT, int W>
-__device__ void bond_op(const TrajDev &tr, int k, const double *gate, Work<T> &wk, int max_sweeps, int scheme,
-                        Smem<T, W> &sm) {
-  const int cL = tr.chi[k], cM = tr.chi[k + 1], cR = tr.chi[k + 2];
+__device__ void bond_op(const TrajDev &tr, int k, int cL, int cM, int cR, const double *gate, Work<T> &wk,
+                        int max_sweeps, int scheme, Smem<T, W> &sm) {
   const int m = 2 * cL, nc = 2 * cR;
   cpx<T> *gk = gamma_slot<T>(tr, k), *gk1 = gamma_slot<T>(tr, k + 1);
   const double *lamL = lam_slot(tr, k), *lamR = lam_slot(tr, k + 2);
   double *lamM = lam_slot(tr, k + 1);
   long long c0 = clock64();
   const bool try_lq = !gate && cM < nc && cM <= m;
-  LocalBond<T> pl;
+  LocalBond<typename LocalType<T>::type> pl;
   LocalResult loc;
   long long lcyc[3] = {0, 0, 0};
-  // Small bonds stay in shared memory throughout; MIXED takes them below the
-  // tensor-core theta's sizes.
-  const bool local = pl.plan(cL, cM, cR, try_lq, sm.arena, NT);
-  if (local) loc = bond_local<T, NT, W>(tr, k, gate, pl, try_lq, max_sweeps, wk, sm, lcyc);
+  bool local = pl.plan(cL, cM, cR, try_lq, sm.arena, NT);  // small bonds stay in shared memory throughout
+  for (bool lq_turn = try_lq; local; lq_turn = false) {
+    loc = bond_local<T, NT, W>(tr, k, cL, cM, cR, gate, pl, lq_turn, max_sweeps, wk, sm, lcyc);
+    if (!loc.declined) break;
+    local = pl.plan(cL, cM, cR, false, sm.arena, NT);  // theta itself instead of its LQ factor
+  }
   // Lambda_{k-1}, Lambda_k, Lambda_{k+1} in the working precision (the state
   // keeps them in float64; the contraction multiplies in T)
   T *lLt = wk.lam3, *lMt = wk.lam3 + tr.cap, *lRt = wk.lam3 + 2 * tr.cap;
@@ -2535,7 +2587,7 @@ __device__ void bond_op(const TrajDev &tr, int k, const double *gate, Work<T> &w
     }
     build_theta<T, NT, W>(gk, gk1, lLt, lMt, lRt, cL, cM, cR, g, dst, copy, cm, sm);
   };
-  if (!local && try_lq) {
+  if (!local && try_lq && !loc.declined) {
     theta(nullptr, wk.T0, wk.T0, true);
     lq = refactor_lq<T, NT, W>(gk, gk1, lLt, lMt, lRt, cL, cM, cR, tr.cap, wk, sm);
   }
@@ -2564,7 +2616,7 @@ __device__ void bond_op(const TrajDev &tr, int k, const double *gate, Work<T> &w
   // what svd_local could not separate.
   if (!local && c > 1 && c <= LocalSvd<T>::max_c(NT) && LocalSvd<T>::bytes(ell, c) <= sm.arena) {
     const long long t0 = clock64();
-    sw = svd_local<T, NT>(wk.A, ell, ell, c, max_sweeps, sm.r0, sm.red);
+    sw = svd_local_global<T, NT>(wk.A, ell, c, max_sweeps, sm.r0, sm.red);
     __syncthreads();
     cyc[1] += clock64() - t0;
     loc.svd_done = sw >= 0;
@@ -2580,18 +2632,7 @@ __device__ void bond_op(const TrajDev &tr, int k, const double *gate, Work<T> &w
         atomicAdd(tr.stats + (lq ? STAT_NONCONV_LQ : STAT_NONCONV_DIRECT), double(c));
       }
     }
-    if (tr.stats) {
-      if (lq) atomicAdd(tr.stats + STAT_LQ_OPS, 1.0);
-      // (whole numbers below 2^53: integer arithmetic spares this thread a chain of float64 operations)
-      const long long a = m > nc ? m : nc, b = m > nc ? nc : m;
-      atomicAdd(tr.stats + STAT_FLOP_THETA, double(8ll * m * cM * nc + (gate ? 128ll * cL * cR : 0ll)));
-      atomicAdd(tr.stats + STAT_FLOP_SVD, double(4ll * (4 * a * a * b + 8 * a * b * b + 9 * b * b * b)));
-      atomicAdd(tr.stats + STAT_BOND_OPS, 1.0);
-      atomicAdd(tr.stats + STAT_SWEEPS, double(sw < 0 ? max_sweeps : sw));
-      // read the Gamma pair + Lambdas, write the new Gamma pair
-      const long long eb = sizeof(cpx<T>);
-      atomicAdd(tr.stats + STAT_BYTES, double(eb * 4 * (1ll * cL * cM + 1ll * cM * cR) + 8ll * (cL + cM + cR)));
-    }
+    if (tr.stats) bond_stats<T>(tr, cL, cM, cR, gate != nullptr, lq, sw < 0 ? max_sweeps : sw);
   }
   if (!loc.done) finalize_bond<T, NT, W>(tr, k, gk, gk1, lamL, lamM, lamR, cL, cR, colmode, ell, c, wk, sm);
   if (sm.tc_fail) {  // a tensor-core wait gave up: the op's result is not trustworthy
@@ -2609,6 +2650,340 @@ __device__ void bond_op(const TrajDev &tr, int k, const double *gate, Work<T> &w
       atomicAdd(tr.stats + STAT_BLOCK_STEPS, double(cyc[3]));
     }
   }
+}
+
+// Whether bond_team takes the bond, in the modes that have a float bulk and
+// tensor-core products.  Double-float: every bond whose theta is wider than
+// bond_local's (its products alone take a third of the operation on the FP32
+// pipes, chi = 50), the SVD by svd_local while the vectors fit.
+template <typename T, int NT, int W>
+__device__ __forceinline__ bool team_takes(const Team &tm, int cL, int cM, int cR, bool try_lq, const Work<T> &wk,
+                                           const Smem<T, W> &sm) {
+  if (sizeof(T) == 8 && !std::is_same<T, dd>::value) return false;
+  if (!wk.team || !sm.tc) return false;
+  const int m = 2 * cL, nc = 2 * cR, c = try_lq ? cM : min(m, nc);
+  if (std::is_same<T, dd>::value) return max(m, nc) > LocalBond<T>::MAXM && sm.arena >= kOzSmem;
+  // float: the single CTA's block Jacobi keeps a half-block resident from step to step; the team's does not
+  return tm.size > 1 && c > 64;
+}
+
+// A large bond operation on the team: theta, LQ reduction, products and the
+// rebuild as double-float (dd) or 3xTF32 (float) tensor-core products over the
+// members' tiles, svd_team / float_sweeps between them.  Same steps and rules
+// as bond_op.  Every member calls it; team-uniform.
+template <typename T, int NT, int W>
+__device__ __noinline__ void bond_team(const Team &tm, const TrajDev &tr, int k, const double *gate, int max_sweeps,
+                                       int scheme, Work<T> &wk, Smem<T, W> &sm) {
+  using R = typename RedType<T>::type;
+  constexpr bool kDD = std::is_same<T, dd>::value;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gthreads = tm.size * NT, gid = tm.rank * NT + tid;
+  const int cL = tr.chi[k], cM = tr.chi[k + 1], cR = tr.chi[k + 2], m = 2 * cL, nc = 2 * cR;
+  cpx<T> *gk = gamma_slot<T>(tr, k), *gk1 = gamma_slot<T>(tr, k + 1);
+  const double *lamL = lam_slot(tr, k), *lamR = lam_slot(tr, k + 2);
+  double *lamM = lam_slot(tr, k + 1);
+  TeamWork tw = team_work<T>(wk.team, tr.cap);
+  T *lL = wk.lam3, *lM = wk.lam3 + tr.cap, *lR = wk.lam3 + 2 * tr.cap;
+  const long long c0 = clock64();
+  long long cyc[4] = {0, 0, 0, 0};
+  if (tm.rank == 0) {
+    for (int v = tid; v < cL; v += NT) lL[v] = T(lamL[v]);
+    for (int u = tid; u < cM; u += NT) lM[u] = T(lamM[u]);
+    for (int w = tid; w < cR; w += NT) lR[w] = T(lamR[w]);
+  }
+  tm.sync();
+  // theta into T0 (and A unless the LQ path works on its own vectors)
+  auto theta = [&](bool colmode, bool copy) {
+    const int ell = colmode ? m : nc;
+    if constexpr (kDD) {
+      const OzPlanes x = oz_planes(tw.plP, tw.exP, m, cM, 8), y = oz_planes(tw.plQ, tw.exQ, nc, cM, 8);
+      oz_split<NT, 8>(tm, x, cM, [&](int i, int u) { return cscale(gk[size_t(i) * cM + u], lL[i >> 1] * lM[u]); });
+      oz_split<NT, 8>(tm, y, cM, [&](int j, int u) { return cscale(gk1[size_t(u) * nc + j], lR[j < cR ? j : j - cR]); });
+      tm.sync();
+      oz_gemm<NT>(tm, x, y, false, 8, colmode ? kOzTrans : kOzPlain, wk.T0, ell, nullptr, sm);
+      tm.sync();
+      if (!gate) {
+        if (copy)
+          for (int o = gid; o < m * nc; o += gthreads) wk.A[o] = wk.T0[o];
+      } else {
+        cpx<T> op[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) op[i] = mkc<T>(T(gate[2 * i]), T(gate[2 * i + 1]));
+        for (int o = gid; o < cL * cR; o += gthreads) {
+          const int v = colmode ? o % cL : o / cR, w = colmode ? o / cL : o % cR;
+          cpx<T> th[4];
+          size_t at[4];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            const int i = 2 * v + (a >> 1), j = (a & 1) * cR + w;
+            at[a] = colmode ? size_t(j) * ell + i : size_t(i) * ell + j;
+            th[a] = wk.T0[at[a]];
+          }
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            cpx<T> s = czero<T>();
+#pragma unroll
+            for (int b = 0; b < 4; ++b) s = cfma(op[a * 4 + b], th[b], s);
+            wk.T0[at[a]] = s;
+            if (copy) wk.A[at[a]] = s;
+          }
+        }
+      }
+    } else {
+      build_theta_tc<NT, W>(gk, gk1, lL, lM, lR, cL, cM, cR, gate, copy ? wk.A : wk.T0, wk.T0, colmode, sm, tm.rank,
+                            tm.size);
+    }
+    tm.sync();
+  };
+  bool lq = false, colmode = m > nc;
+  if (!gate && cM < nc && cM <= m) {
+    // as refactor_lq: S = B B^H = L L^H, vectors M = X diag(Lambda_k) L
+    cpx<T> *S = wk.A + size_t(2) * tr.cap * tr.cap;
+    if constexpr (kDD) {
+      const OzPlanes b = oz_planes(tw.plP, tw.exP, cM, nc, 8);
+      oz_split<NT, 8>(tm, b, nc, [&](int x, int j) { return cscale(gk1[size_t(x) * nc + j], lR[j < cR ? j : j - cR]); });
+      tm.sync();
+      oz_gemm<NT>(tm, b, b, true, 8, kOzHerm, S, cM, nullptr, sm);
+    } else {
+      gemm_nt_tc<NT, W>(
+          cM, cM, nc, [&](int x, int col) { return cscale(gk1[size_t(x) * nc + col], lR[col % cR]); },
+          [&](int y, int col) {
+            const cpx<T> b = cscale(gk1[size_t(y) * nc + col], lR[col % cR]);
+            return mkc<T>(b.x, -b.y);
+          },
+          [&](int x, int y, cpx<T> v) { S[size_t(x) * cM + y] = v; }, sm, tm.rank, tm.size);
+    }
+    tm.sync();
+    if (tm.rank == 0) {
+      const bool ok = cholesky_lower<T, NT, W>(S, cM, sizeof(T) == 4 ? 0.1 : 1e-3, wk.sig, sm);
+      __syncthreads();
+      if (tid == 0) tw.flag[0] = ok ? 1u : 0u;
+    }
+    tm.sync();
+    lq = *reinterpret_cast<volatile unsigned int *>(tw.flag) == 1u;
+    tm.sync();
+    if (lq) {
+      theta(true, false);
+      if constexpr (kDD) {
+        const OzPlanes x = oz_planes(tw.plP, tw.exP, m, cM, 8), y = oz_planes(tw.plQ, tw.exQ, cM, cM, 8);
+        oz_split<NT, 8>(tm, x, cM, [&](int i, int u) { return cscale(gk[size_t(i) * cM + u], lL[i >> 1] * lM[u]); });
+        oz_split<NT, 8>(tm, y, cM, [&](int j, int u) { return u >= j ? S[size_t(u) * cM + j] : czero<dd>(); });
+        tm.sync();
+        oz_gemm<NT>(tm, x, y, false, 8, kOzTrans, wk.A, m, nullptr, sm);
+      } else {
+        gemm_nt_tc<NT, W>(
+            m, cM, cM, [&](int i, int u) { return cscale(gk[size_t(i) * cM + u], lL[i >> 1] * lM[u]); },
+            [&](int j, int u) { return u >= j ? S[size_t(u) * cM + j] : czero<T>(); },
+            [&](int i, int j, cpx<T> v) { wk.A[size_t(j) * m + i] = v; }, sm, tm.rank, tm.size);
+      }
+      tm.sync();
+      colmode = true;
+    }
+  }
+  if (!lq) theta(colmode, true);
+  const int ell = colmode ? m : nc, c = lq ? cM : (colmode ? nc : m);
+  const long long c1 = clock64();
+  int sw;
+  if (kDD && c <= LocalSvd<T>::max_c(NT) && LocalSvd<T>::bytes(ell, c) <= sm.arena) {
+    if (tm.rank == 0) {
+      const long long t0 = clock64();
+      const int s1 = c > 1 ? svd_local_global<T, NT>(wk.A, ell, c, max_sweeps, sm.r0, sm.red) : 1;
+      cyc[1] += clock64() - t0;
+      __syncthreads();
+      if (tid == 0) tw.flag[0] = unsigned(s1 + 1);
+    }
+    tm.sync();
+    sw = int(*reinterpret_cast<volatile unsigned int *>(tw.flag)) - 1;
+  } else if constexpr (kDD) {
+    sw = svd_team<NT, W>(tm, wk.A, ell, c, max_sweeps, tw, sm, cyc);
+  } else {
+    int slot = 1;
+    if (tm.rank == 0)
+      for (int i = tid; i < kTeamFlags; i += NT) tw.flag[i] = 0u;
+    const long long t0 = clock64();
+    sw = float_sweeps<NT, W>(tm, wk.A, ell, nullptr, c, float(sweep_floor<float>(ell)), kFloatDone, max_sweeps, tw,
+                             slot, sm, cyc);
+    cyc[1] += clock64() - t0;
+  }
+  tm.sync();
+  if (sw < 0) {  // the block Jacobi on one CTA
+    if (tm.rank == 0) {
+      const int s2 = jacobi_svd<T, NT, W>(wk.A, ell, c, max_sweeps, sm, cyc, wk.sig, wk.perm, scheme);
+      __syncthreads();
+      if (tid == 0) tw.flag[0] = unsigned(s2 < 0 ? 0 : s2 + 1);
+    }
+    tm.sync();
+    sw = int(*reinterpret_cast<volatile unsigned int *>(tw.flag)) - 1;
+    tm.sync();
+  }
+  const long long c2 = clock64();
+  if (tid == 0 && tm.rank == 0) {
+    if (sw < 0) {
+      atomicOr(tr.status, ST_NOT_CONVERGED);
+      if (tr.stats) {
+        atomicAdd(tr.stats + STAT_NONCONV, 1.0);
+        atomicAdd(tr.stats + (lq ? STAT_NONCONV_LQ : STAT_NONCONV_DIRECT), double(c));
+      }
+    }
+    if (tr.stats) bond_stats<T>(tr, cL, cM, cR, gate != nullptr, lq, sw < 0 ? max_sweeps : sw);
+  }
+  // process_svd and the Gamma rebuild (finalize_bond); every member sorts for itself
+  for (int j = tm.rank * (NT / 32) + warp; j < c; j += tm.size * (NT / 32)) {
+    T part = T(0);
+    const cpx<T> *a = wk.A + size_t(j) * ell;
+    for (int i = lane; i < ell; i += 32) part += cabs2(a[i]);
+    R s = R(part);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s = s + shfl_xor(s, o);
+    if (lane == 0) wk.sig[j] = double(s);
+  }
+  tm.sync();
+  int P = 1;
+  while (P < c) P <<= 1;
+  double *key = reinterpret_cast<double *>(sm.r0);
+  int *pidx = reinterpret_cast<int *>(key + P);
+  for (int j = tid; j < P; j += NT) {
+    key[j] = j < c ? sqrt(wk.sig[j]) : -1.0;
+    pidx[j] = j;
+  }
+  __syncthreads();
+  bitonic_desc<T, NT, W>(key, pidx, P);
+  double part = 0.0;
+  for (int j = tid; j < c; j += NT) part += key[j] * key[j];
+  const double norm1 = sqrt(block_sum<NT>(part, sm.red));
+  const int mode = tr.trunc_mode;
+  const double eps = fmax((mode == 2 || mode == 3) ? fabs(tr.cutoff) : 2.220446049250313e-16, rank_floor<T>(ell));
+  int bad = c;
+  for (int j = tid; j < c; j += NT)
+    if (!is_normal_pos(key[j] / norm1, eps)) bad = min(bad, j);
+  const int nlead = block_min_int<NT>(bad, sm.ired);
+  int rank = mode == 1 ? max(1, min(max(tr.chi_max, 1), nlead))
+                       : (mode == 3 ? max(1, min(tr.chi_max, nlead)) : max(nlead, 1));
+  if (rank > tr.cap) {
+    if (tid == 0 && tm.rank == 0) atomicOr(tr.status, ST_CAPACITY);
+    rank = tr.cap;
+  }
+  double part2 = 0.0;
+  for (int j = tid; j < rank; j += NT) {
+    const double s = key[j] / norm1;
+    part2 += s * s;
+  }
+  const double norm2 = sqrt(block_sum<NT>(part2, sm.red));
+  tm.sync();  // the members have read sig
+  if (tm.rank == 0) {
+    for (int j = tid; j < rank; j += NT) {
+      const double s2 = (key[j] / norm1) / norm2;
+      wk.s2[j] = s2;
+      wk.perm[j] = pidx[j];
+      wk.isig[j] = T(1.0 / key[j]);
+      wk.isig2[j] = T(1.0 / (key[j] * key[j]));
+      wk.w2[j] = T(s2 * s2);
+    }
+    for (int v = tid; v < cL; v += NT) wk.scl[v] = T(1.0 / lamL[v]);
+    for (int w = tid; w < cR; w += NT) wk.scl[tr.cap + w] = T(norm2 / lamR[w]);
+  }
+  tm.sync();
+  const T *sL = wk.scl, *sR = wk.scl + tr.cap, *isig = wk.isig, *isig2 = wk.isig2, *w2 = wk.w2;
+  const int *perm = wk.perm;
+  T pk = T(0), pk1 = T(0);
+  auto put0 = [&](int i, int j, cpx<T> u) {
+    const cpx<T> v = cscale(u, sL[i >> 1]);
+    gk[size_t(i) * rank + j] = v;
+    const T l = lL[i >> 1];
+    pk += cabs2(v) * (l * l) * w2[j];
+  };
+  auto put1 = [&](int j, int col, cpx<T> u) {
+    const int w = col < cR ? col : col - cR;
+    const cpx<T> v = cscale(u, sR[w]);
+    gk1[size_t(j) * nc + col] = v;
+    pk1 += cabs2(v) * w2[j] * (lR[w] * lR[w]);
+  };
+  const cpx<T> *A = wk.A, *T0 = wk.T0;
+  if (colmode) {
+    for (int o = gid; o < m * rank; o += gthreads) {
+      const int i = o / rank, j = o - i * rank;
+      put0(i, j, cscale(A[size_t(perm[j]) * ell + i], isig[j]));
+    }
+  } else {
+    for (int o = gid; o < rank * nc; o += gthreads) {
+      const int j = o / nc, col = o - j * nc;
+      put1(j, col, cscale(A[size_t(perm[j]) * ell + col], isig[j]));
+    }
+  }
+  // the other side: rows j of A^H theta (colmode) or of A theta^H
+  if constexpr (kDD) {
+    const int N = colmode ? nc : m;
+    const OzPlanes a = oz_planes(tw.plP, tw.exP, rank, ell, 8), t = oz_planes(tw.plQ, tw.exQ, N, ell, 8);
+    oz_split<NT, 8>(tm, a, ell, [&](int j, int i) { return A[size_t(perm[j]) * ell + i]; });
+    oz_split<NT, 8>(tm, t, ell, [&](int x, int i) { return T0[size_t(x) * ell + i]; });
+    tm.sync();
+    oz_gemm<NT>(tm, a, t, true, 8, colmode ? kOzPlain : kOzTrans, tw.B, colmode ? N : rank, nullptr, sm);
+    tm.sync();
+    for (int o = gid; o < rank * N; o += gthreads) {  // B = sum_i a_j conj(t_x), as (j, x) or (x, j)
+      const int j = colmode ? o / N : o % rank, x = colmode ? o % N : o / rank;
+      const cpx<T> v = cscale(mkc<dd>(tw.B[o].x, -tw.B[o].y), isig2[j]);
+      if (colmode)
+        put1(j, x, v);
+      else
+        put0(x, j, v);
+    }
+  } else {
+    const int M = colmode ? rank : m, N = colmode ? nc : rank;
+    gemm_nt_tc<NT, W>(
+        M, N, ell,
+        [&](int x, int i) {
+          if (!colmode) return T0[size_t(x) * ell + i];
+          const cpx<T> a = A[size_t(perm[x]) * ell + i];
+          return mkc<T>(a.x, -a.y);
+        },
+        [&](int y, int i) {
+          if (colmode) return T0[size_t(y) * ell + i];
+          const cpx<T> a = A[size_t(perm[y]) * ell + i];
+          return mkc<T>(a.x, -a.y);
+        },
+        [&](int x, int y, cpx<T> v) {
+          if (colmode)
+            put1(x, y, cscale(v, isig2[x]));
+          else
+            put0(x, y, cscale(v, isig2[y]));
+        },
+        sm, tm.rank, tm.size);
+  }
+  // renormalisation: the members' sums in their order
+  R nk = R(pk), nk1 = R(pk1);
+  block_sum2_in<R, NT>(nk, nk1, sm.red);
+  R *part_sum = reinterpret_cast<R *>(wk.sig);
+  if (tid == 0) {
+    part_sum[2 * tm.rank] = nk;
+    part_sum[2 * tm.rank + 1] = nk1;
+  }
+  tm.sync();
+  nk = R(0);
+  nk1 = R(0);
+  for (int i = 0; i < tm.size; ++i) {
+    nk = nk + part_sum[2 * i];
+    nk1 = nk1 + part_sum[2 * i + 1];
+  }
+  const T ik = T(R(1) / sqrt(nk)), ik1 = T(R(1) / sqrt(nk1));
+  for (int o = gid; o < m * rank; o += gthreads) gk[o] = cscale(gk[o], ik);
+  for (int o = gid; o < rank * nc; o += gthreads) gk1[o] = cscale(gk1[o], ik1);
+  if (tm.rank == 0) {
+    for (int j = tid; j < rank; j += NT) lamM[j] = wk.s2[j];
+    if (tid == 0) tr.chi[k + 1] = rank;
+  }
+  if (sm.tc_fail) {
+    if (tid == 0) atomicOr(tr.status, ST_BAD_INSTR);
+    sm.tc_fail = false;
+  }
+  if (tid == 0 && tm.rank == 0 && tr.stats) {
+    atomicAdd(tr.stats + STAT_CYC_THETA, double(c1 - c0));
+    atomicAdd(tr.stats + STAT_CYC_GRAM, double(cyc[0]));
+    atomicAdd(tr.stats + STAT_CYC_ROT, double(cyc[1]));
+    atomicAdd(tr.stats + STAT_CYC_UPDATE, double(cyc[2]));
+    atomicAdd(tr.stats + STAT_CYC_FINAL, double(clock64() - c2));
+    atomicAdd(tr.stats + STAT_BLOCK_STEPS, double(cyc[3]));
+  }
+  tm.sync();
 }
 
 // local_probs (mps.rs:1079-1134): p_s = sum L_{k-1}[v]^2 |G[v,s,u]|^2 L_k[u]^2
@@ -2705,40 +3080,63 @@ __device__ double bond_entropy(const TrajDev &tr, int b, double alpha, double *r
   return log(tot) / (1.0 - alpha);
 }
 
+// A bond operation of the team: large ones on every member, the others on the
+// first while the rest wait at the barrier.
 template <typename T, int NT, int W>
-__device__ void run_program(const LaunchArgs &la, const Instr *prog, const Item &it, Work<T> &wk, Smem<T, W> &sm) {
+__device__ void bond(const Team &tm, const TrajDev &tr, int k, const double *gate, const LaunchArgs &la, Work<T> &wk,
+                     Smem<T, W> &sm) {
+  const int cL = tr.chi[k], cM = tr.chi[k + 1], cR = tr.chi[k + 2];
+  const bool try_lq = !gate && cM < 2 * cR && cM <= 2 * cL;
+  if constexpr (sizeof(T) == 4 || std::is_same<T, dd>::value) {
+    if (team_takes<T, NT, W>(tm, cL, cM, cR, try_lq, wk, sm)) {
+      if (tm.size > 1) tm.sync();  // (chi is read before the operation changes it)
+      bond_team<T, NT, W>(tm, tr, k, gate, la.max_sweeps, la.jacobi_scheme, wk, sm);
+      return;
+    }
+  }
+  if (tm.size > 1) tm.sync();
+  if (tm.rank == 0) bond_op<T, NT, W>(tr, k, cL, cM, cR, gate, wk, la.max_sweeps, la.jacobi_scheme, sm);
+  if (tm.size > 1) tm.sync();
+}
+
+template <typename T, int NT, int W>
+__device__ void run_program(const Team &tm, const LaunchArgs &la, const Instr *prog, const Item &it, Work<T> &wk,
+                            Smem<T, W> &sm) {
   const TrajDev tr = la.trajs[it.traj];
   for (int pc = 0; pc < it.len; ++pc) {
     const Instr in = prog[it.off + pc];
     switch (in.op) {
       case OP_GATE:
-        bond_op<T, NT, W>(tr, in.k, la.gates + size_t(in.a) * 32, wk, la.max_sweeps, la.jacobi_scheme, sm);
+        bond<T, NT, W>(tm, tr, in.k, la.gates + size_t(in.a) * 32, la, wk, sm);
         break;
       case OP_REFACTOR:
-        bond_op<T, NT, W>(tr, in.k, nullptr, wk, la.max_sweeps, la.jacobi_scheme, sm);
+        bond<T, NT, W>(tm, tr, in.k, nullptr, la, wk, sm);
         break;
       case OP_MEAS:
-        measure_site<T, NT, W>(tr, in.k, la.us[in.a], in.b, la.outcomes + in.a, la.probs + in.a, sm);
+        if (tm.rank == 0)
+          measure_site<T, NT, W>(tr, in.k, la.us[in.a], in.b, la.outcomes + in.a, la.probs + in.a, sm);
+        if (tm.size > 1) tm.sync();
         break;
       case OP_ENTROPY: {
         double e = bond_entropy<NT>(tr, in.k, 1.0, sm.red);
-        if (threadIdx.x == 0) la.ents[in.a] = e;
+        if (threadIdx.x == 0 && tm.rank == 0) la.ents[in.a] = e;
         __syncthreads();
         break;
       }
       case OP_RENYI: {
         double e = bond_entropy<NT>(tr, in.k, la.us[in.b], sm.red);
-        if (threadIdx.x == 0) la.ents[in.a] = e;
+        if (threadIdx.x == 0 && tm.rank == 0) la.ents[in.a] = e;
         __syncthreads();
         break;
       }
       case OP_UNI1:
-        unitary1<T, NT, W>(tr, in.k, la.gates + size_t(in.a) * 32);
+        if (tm.rank == 0) unitary1<T, NT, W>(tr, in.k, la.gates + size_t(in.a) * 32);
+        if (tm.size > 1) tm.sync();
         break;
       case OP_PROBS: {
         double p0, p1;
         site_probs<T, NT, W>(tr, in.k, p0, p1, sm);
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == 0 && tm.rank == 0) {
           la.pout[2 * in.a] = p0;
           la.pout[2 * in.a + 1] = p1;
         }
@@ -2748,7 +3146,7 @@ __device__ void run_program(const LaunchArgs &la, const Instr *prog, const Item 
       case OP_NOP:
         break;
       default:
-        if (threadIdx.x == 0) atomicOr(tr.status, ST_BAD_INSTR);
+        if (threadIdx.x == 0 && tm.rank == 0) atomicOr(tr.status, ST_BAD_INSTR);
         break;
     }
   }

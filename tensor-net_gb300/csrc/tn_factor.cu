@@ -376,6 +376,7 @@ int tn_mps_from_vector(uint32_t n, const double *state, uint64_t len, const tn_t
     }
   }
   if (s == TN_OK) s = factorize(tr, v.prec, state, len, v.st);
+  if (s == TN_OK) tn::mps_widen(m, cap);
   if (s != TN_OK) {
     tn_mps_free(m);
     return s;

@@ -155,7 +155,24 @@ void emit_sweep(std::vector<Instr> &prog, uint32_t n) {
 // Launch scratch shared by the single-state API calls of one handle.
 struct Launcher {
   DevBuf prog, items, counter, gates, us, outc, probs, ents, pout, ws, gprog, gitems;
-  int sortP = 1, ws_cap = 1, ws_ctas = 1, sms = 1;
+  int sortP = 1, ws_cap = 1, ws_ctas = 0, sms = 1;
+  int clusters = -1;  // resident clusters of kTeamCtas (-1: not asked yet)
+  size_t ws_stride = 0;
+  bool ws_team = false;
+  // workspaces of at least ctas CTAs (the caller has waited for the stream)
+  cudaError_t ensure_ws(int prec, int ctas) {
+    if (ctas <= ws_ctas) return cudaSuccess;
+    ws.release();
+    ws_ctas = 0;
+    const cudaError_t e = alloc_work(prec, ws_cap, ctas, &ws.p, &ws_stride, &ws_team);
+    if (e != cudaSuccess) {
+      ws.p = nullptr;
+      return e;
+    }
+    ws.n = ws_stride * size_t(ctas);
+    ws_ctas = ctas;
+    return cudaSuccess;
+  }
   void release() {
     gprog.release();
     gitems.release();
@@ -180,6 +197,9 @@ struct tn_mps {
   int prec = TN_PREC_F64;
   bool has_trunc = false;
   tn_trunc trunc{};
+  // Upper estimate of the bond dimensions (|0...0> starts at 1, a gate at most
+  // doubles them): picks the launch shape, nothing else depends on it.
+  uint32_t chi_hint = 0x7fffffff;
   cudaStream_t st = nullptr;
   DevBuf gamma, lam, chi, status, dtraj, stats;
   TrajDev h{};
@@ -260,11 +280,12 @@ int mps_alloc(tn_mps *m) {
     cudaDeviceGetAttribute(&m->L.sms, cudaDevAttrMultiProcessorCount, dev);
   }
   m->L.sortP = next_pow2(2 * int(m->cap));
-  CK(m->L.ws.ensure(run_work_bytes(m->prec, m->L.ws_cap)));
+  CK(m->L.ensure_ws(m->prec, 1));
   return TN_OK;
 }
 
 int mps_reset(tn_mps *m) {
+  m->chi_hint = 1;
   CK(m->L.items.ensure(sizeof(int)));
   int zero = 0;
   CK(cudaMemcpyAsync(m->L.items.p, &zero, sizeof(int), cudaMemcpyHostToDevice, m->st));
@@ -279,15 +300,29 @@ int mps_run(tn_mps *m, const std::vector<Instr> &prog, const std::vector<double>
             double *ents, int n_pout, double *pout, const std::vector<Instr> &par = {}) {
   if (prog.empty() && par.empty()) return TN_OK;
   Launcher &L = m->L;
+  for (const std::vector<Instr> *v : {&par, &prog}) {  // disjoint gates double the bonds once, a list once each
+    const bool once = v == &par;
+    for (const Instr &in : *v)
+      if (in.op == OP_GATE) {
+        m->chi_hint = std::min<uint32_t>(m->cap, m->chi_hint >= 0x40000000u ? m->chi_hint : 2 * m->chi_hint);
+        if (once) break;
+      }
+  }
+  // Bonds wider than 32 have more than 64 vectors, which a cluster shares: one
+  // SM of 152 would do them alone otherwise (a chi = 256 gate in double-float:
+  // 930 ms there, 75 ms on eight).  Narrower ones run on one CTA either way.
+  int cluster = 0;
+  if (m->prec != TN_PREC_F64 && L.ws_team && std::min<uint32_t>(m->chi_hint, m->cap) > 32) {
+    if (L.clusters < 0) L.clusters = run_clusters(m->prec, L.sortP, kTeamCtas);
+    if (L.clusters > 0) cluster = kTeamCtas;
+  }
   if (!par.empty()) {
     // independent single-operation items (disjoint gates) spread over SMs
     const int np = int(par.size());
-    const int grid = std::max(1, std::min(np, L.sms));
+    const int grid = std::max(1, std::min(np, cluster ? L.clusters : L.sms));
     if (grid > L.ws_ctas) {
       CK(cudaStreamSynchronize(m->st));
-      L.ws.release();
-      CK(L.ws.ensure(run_work_bytes(m->prec, L.ws_cap) * size_t(grid)));
-      L.ws_ctas = grid;
+      CK(L.ensure_ws(m->prec, grid));
     }
     std::vector<Item> it(np);
     for (int i = 0; i < np; ++i) it[i] = Item{0, i, 1, 0};
@@ -308,7 +343,9 @@ int mps_run(tn_mps *m, const std::vector<Instr> &prog, const std::vector<double>
     la.prog = L.gprog.as<Instr>();
     la.gates = L.gates.as<double>();
     la.ws = L.ws.p;
-    la.ws_stride = run_work_bytes(m->prec, L.ws_cap);
+    la.ws_stride = L.ws_stride;
+    la.ws_team = L.ws_team;
+    la.cluster = cluster;
     la.max_sweeps = kMaxSweeps;
     la.jacobi_scheme = kDefaultScheme;
     CK(launch_run(m->prec, la, grid, L.sortP, L.ws_cap, m->st));
@@ -346,6 +383,8 @@ int mps_run(tn_mps *m, const std::vector<Instr> &prog, const std::vector<double>
   la.pout = L.pout.as<double>();
   la.ws = L.ws.p;
   la.ws_stride = 0;
+  la.ws_team = L.ws_team;
+  la.cluster = cluster;
   la.max_sweeps = kMaxSweeps;
   la.jacobi_scheme = kDefaultScheme;
   CK(launch_run(m->prec, la, 1, L.sortP, L.ws_cap, m->st));
@@ -493,6 +532,7 @@ int tn_mps_clone(const tn_mps *src, tn_mps **out) {
   m->prec = src->prec;
   m->has_trunc = src->has_trunc;
   m->trunc = src->trunc;
+  m->chi_hint = src->chi_hint;
   cudaError_t e = cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     delete m;
@@ -545,6 +585,7 @@ int tn_mps_import(uint32_t n, const uint32_t *chi, const double *gammas, const d
     tn_mps_free(m);
     return TN_ERR_CAPACITY;
   }
+  m->chi_hint = widest;
   const size_t slot = size_t(2) * m->cap * m->cap * elem_bytes(m->prec);
   std::vector<int> ichi(chi, chi + n + 1);
   std::vector<char> tmp;
@@ -864,6 +905,8 @@ int tn_mps_contract(const tn_mps *m, double *out, uint64_t cap) {
 }
 
 }  // extern "C"
+
+void tn::mps_widen(tn_mps *m, uint32_t chi) { m->chi_hint = std::max(m->chi_hint, std::min(chi, m->cap)); }
 
 int tn::mps_view(const tn_mps *m, tn::MpsView *out) {
   if (!m || !out) return TN_ERR_INVALID_ARG;

@@ -90,6 +90,10 @@ struct LaunchArgs {
   double *pout;          // OP_PROBS output, 2 per slot
   void *ws;              // per-CTA workspace
   size_t ws_stride;      // bytes per CTA
+  int ws_team;           // 1: the workspace includes svd_team's part
+  // CTAs that share an item (a cluster; static schedule only, items dealt out
+  // by cluster index, a workspace per cluster); 0 or 1: one
+  int cluster;
   int max_sweeps;
   int jacobi_scheme;      // 0: block pairs, all pairs per step; 1: within-block then cross-block steps
   int theta_simt;         // 1: SIMT theta contraction even where the tensor-core one applies
@@ -108,6 +112,9 @@ struct LaunchArgs {
   unsigned long long queue_wait_ns;  // limit of one such wait (0: kQueueWaitNs)
 };
 
+// Members of a cluster that shares large bond operations (the portable limit).
+constexpr int kTeamCtas = 8;
+
 // Default Jacobi block scheme (see jacobi_svd): all pairs of each block pair,
 // two inner sweeps per step during the first three sweeps.
 constexpr int kDefaultScheme = 3;
@@ -117,8 +124,14 @@ constexpr unsigned long long kQueueWaitNs = 120ull * 1000 * 1000 * 1000;
 
 cudaError_t launch_run(int prec, const LaunchArgs &la, int grid, int sortP, int ws_cap, cudaStream_t st);
 size_t run_smem_bytes(int prec, int sortP);
-size_t run_work_bytes(int prec, int cap);
+// Workspace bytes of a CTA; team: with svd_team's part (large double-float
+// bonds run the slower block Jacobi without it).
+size_t run_work_bytes(int prec, int cap, bool team);
+// Workspaces of ctas CTAs with that part if memory allows, else without.
+cudaError_t alloc_work(int prec, int cap, int ctas, void **ws, size_t *stride, bool *team);
 int run_blocks_per_sm(int prec, int sortP);
+// Clusters of that many executor CTAs that can be resident at once (0: none).
+int run_clusters(int prec, int sortP, int cluster);
 // Observables of one state, outside the executor: op = OP_PROBS (k = site,
 // two values), OP_ENTROPY or OP_RENYI (k = bond, alpha; one value) into out.
 bool observe_fits(int prec, int cap);  // the bond capacity is within its shared memory
@@ -155,6 +168,8 @@ struct MpsView {
 struct tn_mps;
 namespace tn {
 int mps_view(const tn_mps *m, MpsView *out);
+// The handle's bonds may now be as wide as chi (an estimate that picks launch shapes).
+void mps_widen(tn_mps *m, uint32_t chi);
 
 }  // namespace tn
 struct tn_batch;

@@ -267,8 +267,9 @@ __global__ void k_compile_dd(const TrajDev *trajs, const int *list, int nt, cons
 #define TN_DECLARE_RUN(SUFFIX)                                                                              \
   cudaError_t launch_run_##SUFFIX(const LaunchArgs &la, int grid, int sortP, int ws_cap, cudaStream_t st);  \
   size_t run_smem_##SUFFIX(int sortP);                                                                      \
-  size_t run_work_##SUFFIX(int cap);                                                                        \
-  int run_blocks_##SUFFIX(int sortP);
+  size_t run_work_##SUFFIX(int cap, bool team);                                                             \
+  int run_blocks_##SUFFIX(int sortP);                                                                       \
+  int run_clusters_##SUFFIX(int sortP, int cluster);
 TN_DECLARE_RUN(f32)
 TN_DECLARE_RUN(f64)
 TN_DECLARE_RUN(df)
@@ -283,8 +284,24 @@ size_t run_smem_bytes(int prec, int sortP) {
   return prec == 0 ? run_smem_f64(sortP) : (prec == 2 ? run_smem_df(sortP) : run_smem_f32(sortP));
 }
 
-size_t run_work_bytes(int prec, int cap) {
-  return prec == 0 ? run_work_f64(cap) : (prec == 2 ? run_work_df(cap) : run_work_f32(cap));
+size_t run_work_bytes(int prec, int cap, bool team) {
+  return prec == 0 ? run_work_f64(cap, team) : (prec == 2 ? run_work_df(cap, team) : run_work_f32(cap, team));
+}
+
+cudaError_t alloc_work(int prec, int cap, int ctas, void **ws, size_t *stride, bool *team) {
+  for (int full = 1; full >= 0; --full) {
+    *team = full != 0;
+    *stride = run_work_bytes(prec, cap, *team);
+    const cudaError_t e = cudaMalloc(ws, *stride * size_t(ctas));
+    if (e != cudaErrorMemoryAllocation || !full) return e;
+    (void)cudaGetLastError();
+  }
+  return cudaErrorMemoryAllocation;
+}
+
+int run_clusters(int prec, int sortP, int cluster) {
+  if (prec == 0) return run_clusters_f64(sortP, cluster);
+  return prec == 2 ? run_clusters_df(sortP, cluster) : run_clusters_f32(sortP, cluster);
 }
 
 int run_blocks_per_sm(int prec, int sortP) {

@@ -42,6 +42,27 @@ template <>
 struct RedType<double> {
   using type = double;
 };
+// Arithmetic of bond_local: MIXED computes in double-float too, so that its
+// rounding is that of the stored float Gammas.  (All in float it was a third
+// faster, but the rotations' own rounding, sqrt(rotations) 2^-24, made its
+// errors no smaller than before.)  Its vectors need orthogonality to 1e-8 only:
+// what is left enters the recovered side as 1e-8 sigma_1 / sigma_j, of weight
+// sigma_j.
+template <typename TS>
+struct LocalType {
+  using type = dd;
+};
+template <>
+struct LocalType<double> {
+  using type = double;
+};
+__device__ __forceinline__ cpx<dd> widen(cpx<float> v) { return mkc<dd>(dd(v.x), dd(v.y)); }
+__device__ __forceinline__ cpx<dd> widen(cpx<dd> v) { return v; }
+__device__ __forceinline__ cpx<double> widen(cpx<double> v) { return v; }
+template <typename TS, typename T>
+__device__ __forceinline__ cpx<TS> narrow(cpx<T> v) {
+  return mkc<TS>(TS(v.x), TS(v.y));
+}
 __device__ __forceinline__ float lead(float x) { return x; }
 __device__ __forceinline__ float lead(double x) { return float(x); }
 __device__ __forceinline__ float lead(dd x) { return x.hi; }
@@ -152,8 +173,8 @@ __device__ void gemm_exact_from(int M, int N, FK from, int K, FP P, FQ Q, FE E) 
 // b' = b + t |g| and recomputed each sweep.  Stops after a sweep without a
 // pair above `done` (before its rotation).  Returns the sweeps, -1 at the limit.
 template <int NT>
-__device__ int hestenes(cpx<float> *As, int pa, int ell, cpx<float> *Vs, int pv, int c, float *nrm, int *ord,
-                        float floor_, float tol, float done, int max_sweeps) {
+__device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<float> *Vs, int pv, int c, float *nrm, int *ord,
+                                        float floor_, float tol, float done, int max_sweeps) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cp = c + (c & 1), np = cp >> 1, ring = cp - 1;
   int LG = 32;
@@ -213,24 +234,26 @@ __device__ int hestenes(cpx<float> *As, int pa, int ell, cpx<float> *Vs, int pv,
             const float hx = gx * sc, hy = gy * sc, r2 = fmaf(hx, hx, hy * hy);
             far |= int(r2 > done2);
             if (r2 > tol2) {
-              const float rr = rsqrtf(r2);
+              const float rr = rsqrt_near(r2);
               const float z = 0.5f * ((b - a) * sc) * rr;
               const float z1 = fmaf(z, z, 1.f);
               const float tt = fabsf(z) > 1e15f ? __fdividef(0.5f, z)
                                                 : copysignf(__fdividef(1.f, fabsf(z) + z1 * rsqrtf(z1)), z);
-              const float cs = rsqrtf(fmaf(tt, tt, 1.f)), sn = tt * cs;
+              // x' = x - s (y + tau x), y' = y + s (x - tau y), tau = s / (1 + c): one rounding of an element
+              // a rotation, and no scaling by an inexact c
+              const float cs = rsqrt_near(fmaf(tt, tt, 1.f)), sn = tt * cs, tau = __fdividef(sn, 1.f + cs);
               const cpx<float> e = mkc<float>(hx * rr, -hy * rr);
               for (int i = l; i < ell; i += LG) {
                 const cpx<float> x = ap[i], y = cmul(e, aq[i]);
-                ap[i] = mkc<float>(cs * x.x - sn * y.x, cs * x.y - sn * y.y);
-                aq[i] = mkc<float>(sn * x.x + cs * y.x, sn * x.y + cs * y.y);
+                ap[i] = mkc<float>(fmaf(-sn, fmaf(tau, x.x, y.x), x.x), fmaf(-sn, fmaf(tau, x.y, y.y), x.y));
+                aq[i] = mkc<float>(fmaf(sn, fmaf(-tau, y.x, x.x), y.x), fmaf(sn, fmaf(-tau, y.y, x.y), y.y));
               }
               if (Vs) {
                 cpx<float> *vp = Vs + P * pv, *vq = Vs + Q * pv;
                 for (int i = l; i < c; i += LG) {
                   const cpx<float> x = vp[i], y = cmul(e, vq[i]);
-                  vp[i] = mkc<float>(cs * x.x - sn * y.x, cs * x.y - sn * y.y);
-                  vq[i] = mkc<float>(sn * x.x + cs * y.x, sn * x.y + cs * y.y);
+                  vp[i] = mkc<float>(fmaf(-sn, fmaf(tau, x.x, y.x), x.x), fmaf(-sn, fmaf(tau, x.y, y.y), x.y));
+                  vq[i] = mkc<float>(fmaf(sn, fmaf(-tau, y.x, x.x), y.x), fmaf(sn, fmaf(-tau, y.y, x.y), y.y));
                 }
               }
               if (l == 0) {
@@ -253,21 +276,55 @@ __device__ int hestenes(cpx<float> *As, int pa, int ell, cpx<float> *Vs, int pv,
 }
 
 // ------------------------------------------------ 2. unitary to working precision
+// V (I + W) is unitary for V^H V = I + S, S = D + O (D diagonal): V D_g with
+// D_g = (I + D)^(-1/2) has V^H V - I = S1 = D_g O D_g, so
+//   I + W = D_g (I - S1/2 + 3/8 S1^2 - ...).
+// O is small (below 2e-5: the series ends there), D may be larger: the
+// approximate reciprocal square roots of the float rotations shrink every
+// column a little (up to 1e-3 over long sweeps), and a rotation by t in I + K
+// has D = t^2.  dg_minus1: (1 + x)^(-1/2) - 1 in double-float.
+__device__ __forceinline__ dd dg_minus1(dd x) {
+  const dd r = dd(1.f) / sqrt(dd(1.f) + x);
+  // one correction step: r (1 + x) r = 1 to the working precision already; the
+  // small difference from 1 is what is wanted, without cancellation:
+  // r - 1 = -x / (s (1 + s)), s = sqrt(1 + x)
+  const dd s = dd(1.f) / r;
+  return -(x / (s * (dd(1.f) + s)));
+}
+// W[k][y] from S[k][y] (diagonal: x = S[k][k]), the factors dk, dy = D_g - 1 of
+// k and y, and sq = (S1^2)[k][y].
+__device__ __forceinline__ cpx<dd> unit_entry(bool diag, cpx<dd> s, dd dk, dd dy, cpx<float> sq) {
+  const float gk = 1.f + dk.hi;
+  if (diag) return mkc<dd>(dk + dd(0.375f * gk * sq.x), dd(0.f, 0.f));
+  // D_g,k S1 = (1 + dk)^2 O (1 + dy)
+  const dd f = (dd(1.f) + dk) * (dd(1.f) + dk) * (dd(1.f) + dy);
+  const dd ax = f * s.x, ay = f * s.y;
+  return mkc<dd>(dd(-0.5f * ax.hi, -0.5f * ax.lo) + dd(0.375f * gk * sq.x),
+                 dd(-0.5f * ay.hi, -0.5f * ay.lo) + dd(0.375f * gk * sq.y));
+}
+constexpr float kOffMax = 2e-5f, kDiagMax = 0.1f;
+
 // Q (c x c, row-major with pitch pq) <- the unitary factor of V (float,
 // columns Vs[k * pv + r]), V unitary to a few float roundings or I + K.
 // S = V^H V - I is formed from exact float products; float Newton-Schulz
-// steps bring |S| below 1e-5 first where it is larger (I + K with a t near 1);
-// then Q = V (I - S/2 + 3/8 S^2), whose error is of the order |S|^3 < 1e-15.
+// steps bring its off-diagonals below 2e-5 first where they are larger (I + K
+// with a t near 1); then Q = V (I + W) by unit_entry, whose error is of the
+// order |O|^3 < 1e-14.  dg: c double-float values of scratch.
 // The correction V W is accumulated in double-float in every mode (W < 1e-5,
 // so its error is below 1e-16).  Returns false (Q not written) when V is too
 // far from unitary.
 template <typename T, int NT>
-__device__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S, int ps, cpx<T> *Q, int pq, double *red) {
+__device__ __noinline__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S, int ps, cpx<T> *Q, int pq, dd *dg,
+                                       double *red) {
+  __builtin_assume(__isShared(Vs));
+  __builtin_assume(__isShared(S));
+  __builtin_assume(__isShared(Q));
+  __builtin_assume(__isShared(dg));
   constexpr int OPT = NT >= 512 ? 8 : 8;  // outputs per thread: c <= 64 at 512 threads, c <= 32 at 128
   const int tid = threadIdx.x;
   const int ntri = c * (c + 1) / 2;
   for (int it = 0;; ++it) {
-    float smax = 0.f;
+    float smax = 0.f, dmax = 0.f;
     for (int e = tid; e < ntri; e += NT) {
       int p, q;
       tri_entry(e, c, p, q);
@@ -286,12 +343,16 @@ __device__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S, int ps, cpx
       const dd sx = tacc_fin(ax), sy = tacc_fin(ay);
       S[p * ps + q] = mkc<dd>(sx, sy);
       if (p != q) S[q * ps + p] = mkc<dd>(sx, -sy);
-      smax = fmaxf(smax, fmaxf(fabsf(sx.hi), fabsf(sy.hi)));
+      if (p == q)
+        dmax = fmaxf(dmax, fabsf(sx.hi));
+      else
+        smax = fmaxf(smax, fmaxf(fabsf(sx.hi), fabsf(sy.hi)));
       if (!(sx.hi == sx.hi && sy.hi == sy.hi)) smax = __int_as_float(0x7f800000);
     }
     smax = block_max<NT>(smax, red);  // (ends with S visible: its barriers follow the stores)
-    if (smax <= 1e-5f) break;
-    if (!(smax <= 0.5f) || it >= 6) return false;
+    dmax = block_max<NT>(dmax, red);
+    if (smax <= kOffMax && dmax <= kDiagMax) break;
+    if (!(smax <= 0.5f && dmax <= 0.5f) || it >= 6) return false;
     cpx<float> out[OPT];
 #pragma unroll
     for (int u = 0; u < OPT; ++u) {
@@ -315,7 +376,9 @@ __device__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S, int ps, cpx
     }
     __syncthreads();
   }
-  // W = -S/2 + 3/8 S^2 (the square in float), in place of S
+  // W in place of S (the square in float)
+  for (int k = tid; k < c; k += NT) dg[k] = dg_minus1(S[k * ps + k].x);
+  __syncthreads();
   {
     cpx<float> sq[OPT];
 #pragma unroll
@@ -325,10 +388,13 @@ __device__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S, int ps, cpx
         const int y = o / c, x = o - y * c;
         cpx<float> a = czero<float>();
         for (int k = 0; k < c; ++k) {
+          if (k == x || k == y) continue;
           const cpx<dd> s = S[x * ps + k], t = S[k * ps + y];
-          a = cfma(mkc<float>(s.x.hi, s.y.hi), mkc<float>(t.x.hi, t.y.hi), a);
+          const float g = 1.f + dg[k].hi;
+          a = cfma(mkc<float>(s.x.hi * (g * g), s.y.hi * (g * g)), mkc<float>(t.x.hi, t.y.hi), a);
         }
-        sq[u] = a;
+        const float g = (1.f + dg[x].hi) * (1.f + dg[y].hi);
+        sq[u] = mkc<float>(a.x * g, a.y * g);
       }
     }
     __syncthreads();
@@ -337,9 +403,7 @@ __device__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S, int ps, cpx
       const int o = tid + u * NT;
       if (o < c * c) {
         const int y = o / c, x = o - y * c;
-        const cpx<dd> s = S[x * ps + y];
-        S[x * ps + y] = mkc<dd>(dd(-0.5f * s.x.hi, -0.5f * s.x.lo) + dd(0.375f * sq[u].x),
-                                dd(-0.5f * s.y.hi, -0.5f * s.y.lo) + dd(0.375f * sq[u].y));
+        S[x * ps + y] = unit_entry(x == y, S[x * ps + y], dg[x], dg[y], sq[u]);
       }
     }
     __syncthreads();
@@ -487,19 +551,28 @@ struct LocalSvd {
   __host__ __device__ static size_t bytes(int ell, int c) {
     const size_t tail = al(size_t(c) * 8);
     if (sizeof(T) == 4) return first_bytes(ell, c) + tail;
+    // (the factors dg share the norms' and the order's place)
     return first_bytes(ell, c) + al(size_t(c) * odd(c) * 16) + al(size_t(c) * odd(c) * 8) + tail;
   }
   // largest c of the refinement's fixed outputs per thread
   __host__ __device__ static int max_c(int nt) { return sizeof(T) == 4 ? MAXC : (nt >= 512 ? 64 : 32); }
 };
 
+// (svd_tolerance: the block Jacobi's threshold, 4 above the rounding of a Gram
+// entry.)
+template <typename T>
+__device__ __forceinline__ float svd_tolerance(int ell) {
+  return 4.f * sqrtf(float(ell)) * float(Eps<T>::v);
+}
+
 // Orthogonalises the c vectors A[j * ld + i] (length ell; any address space)
-// by unitary column operations.  scratch: LocalSvd<T>::bytes of shared memory,
+// by unitary column operations until |a_p^H a_q| <= tol |a_p| |a_q|.  scratch: LocalSvd<T>::bytes of shared memory,
 // 16-byte aligned.  Returns the number of sweeps and refinement steps, or -1:
 // A is then a unitary transform of the input that has not converged (a
 // degenerate spectrum, or the sweep limit), for the caller's block Jacobi.
 template <typename T, int NT>
-__device__ int svd_local(cpx<T> *A, int ld, int ell, int c, int max_sweeps, unsigned char *scratch, double *red) {
+__device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int max_sweeps, unsigned char *scratch,
+                                         double *red, float tol) {
   using L = LocalSvd<T>;
   const int tid = threadIdx.x;
   const int pa = L::odd(ell), pc = L::odd(c);
@@ -537,8 +610,8 @@ __device__ int svd_local(cpx<T> *A, int ld, int ell, int c, int max_sweeps, unsi
     at += L::al(size_t(c) * pc * 8);
     float *nrm = reinterpret_cast<float *>(at);
     int *ord = reinterpret_cast<int *>(nrm + c);
+    dd *dg = reinterpret_cast<dd *>(nrm);  // (not needed while the sweeps run)
     const float floor_t = float(sweep_floor<T>(ell));
-    const float tol = float(4.0 * sqrt(double(ell)) * double(Eps<T>::v));
     // a correction formed in float is exact to the working precision below this angle
     constexpr float kFloatApply = std::is_same<T, double>::value ? 1e-9f : 1e-7f;
     constexpr int kMaxStages = 3, kMaxSteps = 10;
@@ -558,7 +631,7 @@ __device__ int svd_local(cpx<T> *A, int ld, int ell, int c, int max_sweeps, unsi
                                     1e-4f, min(max_sweeps, 20));
         sweeps += sw < 0 ? min(max_sweeps, 20) : sw;
         ++stages;
-        if (!unitarise<T, NT>(Vs, pc, c, S, pc, Q, pc, red)) return -1;
+        if (!unitarise<T, NT>(Vs, pc, c, S, pc, Q, pc, dg, red)) return -1;
         apply_unitary<T, NT>(A, ld, ell, c, Q, pc, stage, pc);
         bulk = false;
       }
@@ -602,22 +675,34 @@ __device__ int svd_local(cpx<T> *A, int ld, int ell, int c, int max_sweeps, unsi
       if (!(rmax < 2.f)) return -1;  // not a number
       if (rmax <= tol) return sweeps + 1;
       ++sweeps;
-      // the pairs left after this step are of order r times the largest angle
-      const bool last = rmax * kmax * 8.f <= tol;
-      if (kmax <= kFloatApply) {
+      // What is left after this step is of the order of the square: r r' between
+      // vectors of different size (whose angles t are smaller than r), r t
+      // between neighbours.
+      const float far = fmaxf(rmax, kmax);
+      const bool last = rmax * far * 8.f <= tol;
+      if (far <= kFloatApply) {
         apply_small<T, NT>(A, ld, ell, c, Vs, pc, reinterpret_cast<cpx<float> *>(stage), pc);
       } else if (rmax > 1e-3f && kmax > 0.3f && stages < kMaxStages) {
         bulk = true;  // far from converged: vectors that the float stage had left alone
         __syncthreads();
         continue;
       } else {
-        if (!unitarise<T, NT>(Vs, pc, c, S, pc, Q, pc, red)) return -1;
+        if (!unitarise<T, NT>(Vs, pc, c, S, pc, Q, pc, dg, red)) return -1;
         apply_unitary<T, NT>(A, ld, ell, c, Q, pc, stage, pc);
       }
       if (last) return sweeps + 1;
     }
     return -1;
   }
+}
+
+// The same for vectors in global memory (one copy for its several callers).
+template <typename T, int NT>
+__device__ __noinline__ int svd_local_global(cpx<T> *A, int ell, int c, int max_sweeps, unsigned char *scratch,
+                                             double *red) {
+  __builtin_assume(__isShared(scratch));
+  __builtin_assume(__isShared(red));
+  return svd_local<T, NT>(A, ell, ell, c, max_sweeps, scratch, red, svd_tolerance<T>(ell));
 }
 
 // In-place Cholesky S = L L^H of an n x n Hermitian matrix in shared memory
@@ -631,7 +716,7 @@ __device__ bool cholesky_local(cpx<T> *S, int ps, int n, float rel, T *diag0) {
     const T d = S[k * ps + k].x;
     if (!(lead(d) > rel * lead(diag0[k])) || !(lead(d) > 0.f)) return false;  // uniform: every thread read the same
     __syncthreads();
-    if (threadIdx.x < 32 || int(threadIdx.x) < n) {  // whole warps that hold a row below the pivot
+    if (threadIdx.x < 32 || int(threadIdx.x & ~31u) < n - k - 1) {  // whole warps that hold a row below the pivot
       const T l = sqrt(d), il = T(1) / l;
       for (int i = k + 1 + threadIdx.x; i < n; i += NT) S[i * ps + k] = cscale(S[i * ps + k], il);
       if (threadIdx.x == 0) S[k * ps + k] = mkc<T>(l, T(0));
@@ -661,23 +746,25 @@ template <typename T>
 struct LocalBond {
   static constexpr int MAXM = 64;
   size_t theta, vec, svd, lam, vals, total;
+  int c;
   __host__ __device__ static size_t al(size_t x) { return (x + 15) & ~size_t(15); }
   __host__ __device__ static size_t most(size_t a, size_t b) { return a > b ? a : b; }
   __host__ __device__ bool plan(int cL, int cM, int cR, bool lq, size_t room, int nt) {
-    const int m = 2 * cL, nc = 2 * cR, c = m < nc ? m : nc, ell = m < nc ? nc : m;
-    if (ell > MAXM || cM > MAXM || c > LocalSvd<T>::max_c(nt)) return false;
+    const int m = 2 * cL, nc = 2 * cR, mn = m < nc ? m : nc;
+    if (m > MAXM || nc > MAXM || cM > MAXM) return false;
     const size_t e = sizeof(cpx<T>);
-    theta = al(size_t(c) * (ell | 1) * e);
-    vec = theta;
+    // vectors and their length; theta with the same pitch.  (LQ: cM vectors of
+    // length m, theta as columns; the general path takes what LQ declines.)
+    c = lq ? cM : mn;
+    const int ell = lq ? m : (m < nc ? nc : m);
+    if (c > LocalSvd<T>::max_c(nt)) return false;
+    theta = al(size_t(lq ? nc : mn) * (ell | 1) * e);
+    vec = al(size_t(c) * (ell | 1) * e);
     svd = LocalSvd<T>::bytes(ell, c);
-    if (lq) {  // cM vectors of length m, theta as columns; and room for the direct path if it falls back
-      theta = most(theta, al(size_t(nc) * (m | 1) * e));
-      vec = most(vec, al(size_t(cM) * (m | 1) * e));
-      svd = most(svd, LocalSvd<T>::bytes(m, cM));
-      svd = most(svd, al(size_t(cM) * (cM | 1) * e) + al(size_t(cM) * sizeof(T)));
-    }
+    svd = most(svd, al(size_t(cM) * (cM | 1) * e) + al(size_t(cM) * sizeof(T)));    // S and its diagonal
+    svd = most(svd, al(size_t(c) * (lq ? nc : mn) * e));                            // the recovered side
     lam = al(size_t(2) * (cL + cM + cR) * sizeof(T));
-    vals = al(size_t(c) * (3 * sizeof(double) + 3 * sizeof(T) + sizeof(int))) + 128;
+    vals = al(size_t(mn) * (3 * sizeof(double) + 3 * sizeof(T) + sizeof(int))) + 128;
     total = theta + vec + svd + lam + vals;
     return total <= room;
   }
@@ -720,6 +807,7 @@ __device__ __forceinline__ void block_sum2_in(R &a, R &b, double *red) {
 // What bond_local leaves behind.
 struct LocalResult {
   bool done = false;  // the bond is finished; else theta and the vectors are in the global workspace
+  bool declined = false;  // ... or nothing has happened (no LQ factor): the general path starts over
   bool svd_done = false;  // (general path) svd_local has orthogonalised the vectors
   bool lq = false, colmode = false;
   int ell = 0, c = 0, sweeps = 0;

@@ -25,10 +25,17 @@ __global__ void __launch_bounds__(NT, 1) k_run(LaunchArgs la, int sortP, int ws_
   extern __shared__ __align__(256) unsigned char smem[];
   __shared__ Item s_item;
   __shared__ int s_kind;  // 0 done, 1 gate / static item, 2 pushed sweep item, 3 skip
-  __shared__ uint64_t s_bar;
+  __shared__ uint64_t s_bar, s_gbar[2];
   __shared__ uint32_t s_tmem;
   Smem<T, W> sm(smem, sortP);
-  Work<T> wk = make_work<T>(reinterpret_cast<unsigned char *>(la.ws) + size_t(blockIdx.x) * la.ws_stride, ws_cap);
+  Team tm;
+  if (la.cluster > 1) {
+    tm.size = la.cluster;
+    tm.rank = int(blockIdx.x) % la.cluster;  // clusters are consecutive blocks of a one-dimensional grid
+  }
+  const int team_id = int(blockIdx.x) / tm.size;
+  Work<T> wk = make_work<T>(reinterpret_cast<unsigned char *>(la.ws) + size_t(team_id) * la.ws_stride, ws_cap,
+                            la.ws_team != 0);
   const bool dd = la.rem != nullptr;
   // float: one 128 x 256 FP32 accumulator tile (theta and recovery GEMMs);
   // double-float: eight 128 x 64 level accumulators of the tensor-core update
@@ -43,6 +50,8 @@ __global__ void __launch_bounds__(NT, 1) k_run(LaunchArgs la, int sortP, int ws_
     }
     if (threadIdx.x == 0) {
       tc::mbar_init(&s_bar, 1);
+      tc::mbar_init(s_gbar, 1);
+      tc::mbar_init(s_gbar + 1, 1);
       tc::mbar_fence_init();
     }
     tc::fence_before_sync();
@@ -50,10 +59,18 @@ __global__ void __launch_bounds__(NT, 1) k_run(LaunchArgs la, int sortP, int ws_
     tc::fence_after_sync();
     sm.tmem = s_tmem;
     sm.bar = &s_bar;
+    sm.gbar = s_gbar;
     sm.phase = 0;
     sm.tc = la.theta_simt == 0;
   }
-  for (;;) {
+  if (tm.size > 1) {
+    for (int it = team_id; it < la.nitems; it += int(gridDim.x) / tm.size) {
+      const Item item = la.items[it];
+      run_program<T, NT, W>(tm, la, la.prog, item, wk, sm);
+      tm.sync();
+    }
+  }
+  for (; tm.size == 1;) {
     if (threadIdx.x == 0) {
       const int G = la.nitems_dev ? *la.nitems_dev : la.nitems;
       int kind = 0, slot_i = -1;
@@ -106,7 +123,7 @@ __global__ void __launch_bounds__(NT, 1) k_run(LaunchArgs la, int sortP, int ws_
     if (kind == 0) break;
     if (kind == 3) continue;
     if (kind == 2) __threadfence();  // acquire side for every thread of the CTA
-    run_program<T, NT, W>(la, (dd && kind == 1) ? la.gprog : la.prog, item, wk, sm);
+    run_program<T, NT, W>(tm, la, (dd && kind == 1) ? la.gprog : la.prog, item, wk, sm);
     if (dd && kind == 1) {
       __threadfence();  // this thread's writes of the gate's result, visible device-wide
       __syncthreads();
@@ -148,8 +165,45 @@ static cudaError_t launch_run_t(const LaunchArgs &la, int grid, int sortP, int w
   const size_t smem = SmemLayout<T, W>::total(sortP);
   cudaError_t e = ensure_run_smem<T, NT, W>(smem);
   if (e != cudaSuccess) return e;
-  k_run<T, NT, W><<<grid, NT, smem, st>>>(la, sortP, ws_cap);
-  return cudaGetLastError();
+  if (la.cluster <= 1) {
+    k_run<T, NT, W><<<grid, NT, smem, st>>>(la, sortP, ws_cap);
+    return cudaGetLastError();
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(grid) * unsigned(la.cluster));
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(la.cluster);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_run<T, NT, W>, la, sortP, ws_cap);
+}
+
+// Clusters of `cluster` CTAs of k_run<T> that can be resident at once (0: none).
+template <typename T, int NT, int W>
+static int run_clusters_t(int sortP, int cluster) {
+  const size_t smem = SmemLayout<T, W>::total(sortP);
+  if (ensure_run_smem<T, NT, W>(smem) != cudaSuccess) return 0;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(cluster));
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(cluster);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, k_run<T, NT, W>, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return n;
 }
 
 // Blocks of k_run<T> that fit on an SM (at least 1).
@@ -167,7 +221,8 @@ static int run_blocks_t(int sortP) {
     return launch_run_t<T, kThreads, kBlockW>(la, grid, sortP, ws_cap, st);                                \
   }                                                                                                         \
   size_t run_smem_##SUFFIX(int sortP) { return SmemLayout<T, kBlockW>::total(sortP); }                      \
-  size_t run_work_##SUFFIX(int cap) { return work_bytes<T>(cap); }                                          \
-  int run_blocks_##SUFFIX(int sortP) { return run_blocks_t<T, kThreads, kBlockW>(sortP); }
+  size_t run_work_##SUFFIX(int cap, bool team) { return work_bytes<T>(cap) + (team ? team_bytes<T>(cap) : 0); } \
+  int run_blocks_##SUFFIX(int sortP) { return run_blocks_t<T, kThreads, kBlockW>(sortP); }                  \
+  int run_clusters_##SUFFIX(int sortP, int cluster) { return run_clusters_t<T, kThreads, kBlockW>(sortP, cluster); }
 
 }  // namespace tn
