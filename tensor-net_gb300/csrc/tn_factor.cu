@@ -22,6 +22,13 @@
 // norm lies between 1/m and 1) and are left out of the rotations; they end
 // below the EPS cutoff of the rank rule.
 //
+// Sites whose shorter side is at most 64 (every site up to n = 13) run in
+// k_fv_local, one CTA and one launch for all of them in a row: svd_local's
+// float sweeps and float64 refinement on the rows (m <= N) or columns of M, an
+// identity appended to the vectors so that the accumulated unitary gives the
+// other side exactly.  A site that it does not take, or does not separate,
+// goes through the rounds above.
+//
 // This is an initialisation path (validation exports and prepared initial
 // states), sized for n <= 20 (m <= 2048 rows, 2^20 amplitudes); the work per
 // site is O(m^2 N) per sweep, which stays below a second per site there.
@@ -29,6 +36,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "tn_device.cuh"
 #include "tn_internal.h"
 #include "tn_mps.h"
 
@@ -269,6 +277,144 @@ __global__ void k_fv_last(const double2 *q, int udim, int n, tn::TrajDev tr, int
   }
 }
 
+// Sites k0, k0 + 1, ... in one CTA while they fit (see the head of the file).
+// q holds the remainder at k0 (udim rows), qn is a second buffer, vec c (ell +
+// c) values of scratch.  out[0]: the site where it stopped (n - 1: all done),
+// out[1]: its udim (-1: the rank exceeds the capacity), out[2]: 1 when the
+// remainder is in qn.  Bound by float64 arithmetic on one SM (n = 13: 95 ms by
+// rounds of launches, 15 ms here).
+constexpr int kFvLocalC = 64;
+constexpr size_t kFvLocalArena = 212 * 1024;
+
+template <int NT>
+__global__ void __launch_bounds__(NT, 1) k_fv_local(double2 *q, double2 *qn, double2 *vec, uint64_t len, int k0, int udim,
+                                                    int n, tn::TrajDev tr, int prec, int *out) {
+  using C = tn::cpx<double>;
+  extern __shared__ __align__(256) unsigned char fsm[];
+  __shared__ double red[128], sv[kFvLocalC];
+  __shared__ int perm[kFvLocalC];
+  __shared__ double s_snorm, s_norm2;
+  __shared__ int s_rank;
+  C *a = reinterpret_cast<C *>(vec);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int swaps = 0, k = k0;
+  for (; k + 1 < n; ++k) {
+    const int m = 2 * udim;
+    const int nq = int(len >> (k + 1));
+    const bool rows = m <= nq;
+    const int c = rows ? m : nq, ell = rows ? nq : m, ld = ell + c;
+    if (c > kFvLocalC || tn::LocalSvd<double>::bytes(ell, c) > kFvLocalArena) break;
+    for (int idx = tid; idx < m * nq; idx += NT) {
+      const int i = idx / nq, j = idx - i * nq;
+      const double2 z = q[idx];
+      C &d = rows ? a[size_t(i) * ld + j] : a[size_t(j) * ld + i];
+      d.x = z.x;
+      d.y = z.y;
+    }
+    for (int idx = tid; idx < c * c; idx += NT) {
+      C &d = a[size_t(idx / c) * ld + ell + idx % c];
+      d.x = idx % (c + 1) == 0 ? 1.0 : 0.0;
+      d.y = 0.0;
+    }
+    __syncthreads();
+    if (c > 1 && tn::svd_local<double, NT>(a, ld, ell, c, 40, fsm, red, tn::svd_tolerance<double>(ell), c) < 0) break;
+    __syncthreads();
+    for (int j = warp; j < c; j += NT / 32) {
+      double acc = 0.0;
+      for (int i = lane; i < ell; i += 32) acc += tn::cabs2(a[size_t(j) * ld + i]);
+      acc = warp_sum_bcast(acc);
+      if (lane == 0) sv[j] = sqrt(acc);
+    }
+    __syncthreads();
+    for (int j = tid; j < c; j += NT) {
+      int rk = 0;
+      const double x = sv[j];
+      for (int i = 0; i < c; ++i) rk += (sv[i] > x || (sv[i] == x && i < j)) ? 1 : 0;
+      perm[min(rk, c - 1)] = j;
+    }
+    __syncthreads();
+    if (tid == 0) {  // the rank rule of k_fv_finish
+      double tot = 0.0;
+      for (int j = 0; j < c; ++j) tot += sv[perm[j]] * sv[perm[j]];
+      const double snorm = sqrt(tot);
+      const bool has_cut = tr.trunc_mode == TN_TRUNC_CUTOFF || tr.trunc_mode == TN_TRUNC_BOTH;
+      const double noise = 4.0 * sqrt(double(ell)) * 2.220446049250313e-16;
+      const double eps = fmax(has_cut ? fabs(tr.cutoff) : 2.220446049250313e-16, noise);
+      int lead = 0;
+      while (lead < c) {
+        const double x = sv[perm[lead]] / snorm;
+        if (!fv_normal(x) || !(x > eps)) break;
+        ++lead;
+      }
+      int rank = tr.trunc_mode == TN_TRUNC_CONST
+                     ? min(max(tr.chi_max, 1), lead)
+                     : (tr.trunc_mode == TN_TRUNC_BOTH ? max(1, min(tr.chi_max, lead)) : max(lead, 1));
+      double n2 = 0.0;
+      for (int j = 0; j < rank; ++j) {
+        const double x = sv[perm[j]] / snorm;
+        n2 += x * x;
+      }
+      s_snorm = snorm;
+      s_norm2 = sqrt(n2);
+      s_rank = rank <= tr.cap ? rank : -1;
+    }
+    __syncthreads();
+    const int rank = s_rank;
+    if (rank < 1) {
+      udim = -1;
+      break;
+    }
+    const double snorm = s_snorm, norm2 = s_norm2;
+    double *lam = tr.lam + size_t(k + 1) * tr.cap;
+    const double *lam_prev = tr.lam + size_t(k) * tr.cap;
+    for (int j = tid; j < rank; j += NT) lam[j] = (sv[perm[j]] / snorm) / norm2;
+    if (tid == 0) tr.chi[k + 1] = rank;
+    const size_t slot = size_t(2) * tr.cap * tr.cap;
+    for (int idx = tid; idx < m * rank; idx += NT) {
+      const int row = idx / rank, j = idx - row * rank, src = perm[j];
+      double vr, vi;
+      if (rows) {  // U = Q^*, the accumulated unitary
+        const C x = a[size_t(src) * ld + ell + row];
+        vr = x.x;
+        vi = -x.y;
+      } else {
+        const C x = a[size_t(src) * ld + row];
+        vr = x.x / sv[src];
+        vi = x.y / sv[src];
+      }
+      if (k > 0) {
+        const double l = lam_prev[row >> 1];
+        vr /= l;
+        vi /= l;
+      }
+      store_elem(tr.gamma, prec, size_t(k) * slot + idx, vr, vi);
+    }
+    for (int idx = tid; idx < rank * nq; idx += NT) {
+      const int j = idx / nq, col = idx - j * nq, src = perm[j];
+      double2 z;
+      if (rows) {
+        const C x = a[size_t(src) * ld + col];
+        z = make_double2(x.x / snorm, x.y / snorm);
+      } else {
+        const C x = a[size_t(src) * ld + ell + col];
+        z = make_double2(sv[src] * x.x / snorm, -sv[src] * x.y / snorm);
+      }
+      qn[idx] = z;
+    }
+    udim = rank;
+    double2 *t = q;
+    q = qn;
+    qn = t;
+    swaps ^= 1;
+    __syncthreads();
+  }
+  if (tid == 0) {
+    out[0] = k;
+    out[1] = udim;
+    out[2] = swaps;
+  }
+}
+
 struct Scratch {
   void *p = nullptr;
   ~Scratch() {
@@ -305,8 +451,24 @@ int factorize(const tn::TrajDev &tr, int prec, const double *state, uint64_t len
   FV_CK(cudaMemcpyAsync(&norm, dnorm, sizeof(double), cudaMemcpyDeviceToHost, st));
   FV_CK(cudaStreamSynchronize(st));
   if (!(norm > 0.0) || !std::isfinite(norm)) return TN_ERR_INVALID_ARG;
+  // vectors with the appended identity: c (ell + c) <= len + 64^2
+  Scratch sv;
+  FV_CK(cudaMalloc(&sv.p, (len + kFvLocalC * kFvLocalC) * sizeof(double2)));
+  FV_CK(cudaFuncSetAttribute(k_fv_local<tn::kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFvLocalArena)));
   int udim = 1;
   for (int k = 0; k + 1 < n; ++k) {
+    k_fv_local<tn::kThreads><<<1, tn::kThreads, kFvLocalArena, st>>>(qa, qb, static_cast<double2 *>(sv.p), len, k, udim, n,
+                                                                    tr, prec, drank);
+    FV_CK(cudaGetLastError());
+    int done[3] = {0, 0, 0};
+    FV_CK(cudaMemcpyAsync(done, drank, sizeof(done), cudaMemcpyDeviceToHost, st));
+    FV_CK(cudaStreamSynchronize(st));
+    if (done[1] < 1) return TN_ERR_CAPACITY;
+    k = done[0];
+    udim = done[1];
+    if (done[2]) std::swap(qa, qb);
+    if (k + 1 >= n) break;
+    // this site by rounds of disjoint row pairs
     const int m = 2 * udim;
     const uint64_t nq = len >> (k + 1);
     if (m > mmax) return TN_ERR_CAPACITY;

@@ -567,12 +567,14 @@ __device__ __forceinline__ float svd_tolerance(int ell) {
 
 // Orthogonalises the c vectors A[j * ld + i] (length ell; any address space)
 // by unitary column operations until |a_p^H a_q| <= tol |a_p| |a_q|.  scratch: LocalSvd<T>::bytes of shared memory,
-// 16-byte aligned.  Returns the number of sweeps and refinement steps, or -1:
+// 16-byte aligned.  tail: so many further entries of each vector follow the
+// operations without counting as its length (an appended identity becomes the
+// accumulated unitary).  Returns the number of sweeps and refinement steps, or -1:
 // A is then a unitary transform of the input that has not converged (a
 // degenerate spectrum, or the sweep limit), for the caller's block Jacobi.
 template <typename T, int NT>
 __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int max_sweeps, unsigned char *scratch,
-                                         double *red, float tol) {
+                                         double *red, float tol, int tail = 0) {
   using L = LocalSvd<T>;
   const int tid = threadIdx.x;
   const int pa = L::odd(ell), pc = L::odd(c);
@@ -632,7 +634,7 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
         sweeps += sw < 0 ? min(max_sweeps, 20) : sw;
         ++stages;
         if (!unitarise<T, NT>(Vs, pc, c, S, pc, Q, pc, dg, red)) return -1;
-        apply_unitary<T, NT>(A, ld, ell, c, Q, pc, stage, pc);
+        apply_unitary<T, NT>(A, ld, ell + tail, c, Q, pc, stage, pc);
         bulk = false;
       }
       gram_local<T, NT>(A, ld, ell, c, G, pc, stage, pc);
@@ -681,14 +683,14 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
       const float far = fmaxf(rmax, kmax);
       const bool last = rmax * far * 8.f <= tol;
       if (far <= kFloatApply) {
-        apply_small<T, NT>(A, ld, ell, c, Vs, pc, reinterpret_cast<cpx<float> *>(stage), pc);
+        apply_small<T, NT>(A, ld, ell + tail, c, Vs, pc, reinterpret_cast<cpx<float> *>(stage), pc);
       } else if (rmax > 1e-3f && kmax > 0.3f && stages < kMaxStages) {
         bulk = true;  // far from converged: vectors that the float stage had left alone
         __syncthreads();
         continue;
       } else {
         if (!unitarise<T, NT>(Vs, pc, c, S, pc, Q, pc, dg, red)) return -1;
-        apply_unitary<T, NT>(A, ld, ell, c, Q, pc, stage, pc);
+        apply_unitary<T, NT>(A, ld, ell + tail, c, Q, pc, stage, pc);
       }
       if (last) return sweeps + 1;
     }

@@ -96,3 +96,19 @@ def test_measurement_sweep_on_small_bonds(pkg, ref, kind, n, chi, prec):
     a, b = g.measure_postsel_prob(n // 2, p), m.measure_postsel_prob(n // 2, p)
     assert abs(a - b) < TOL[prec]
     _compare(g, m, n, TOL[prec])
+
+
+@pytest.mark.parametrize("kind,n,chi", [("random", 2, 2), ("random", 12, 64), ("random", 13, 64), ("random", 14, 128),
+                                        ("graded", 12, 64), ("low", 12, 5), ("equal", 10, 32)])
+def test_from_vector_sites_on_one_cta(pkg, ref, kind, n, chi):
+    """k_fv_local up to its limit (n = 13) and around it: sites that it leaves to
+    the rounds (the middle of n = 14), rank-deficient and degenerate spectra."""
+    rng = np.random.default_rng(13)
+    psi = {"random": lambda: _random(rng, n), "graded": lambda: _random(rng, n, 6.0),
+           "low": lambda: _low_rank(rng, n, chi), "equal": lambda: _equal(n)}[kind]()
+    g, m = pkg.MPS.from_vector(psi), ref.from_vector(psi)
+    for b in range(n - 1):
+        a, r = g.svals(b), m.svals[b]
+        k = int(np.sum(r > 1e-12))
+        assert a.size >= k and np.max(np.abs(a[:k] - r[:k])) < 1e-12, b
+    assert np.max(np.abs(g.contract() - psi)) < 1e-12
