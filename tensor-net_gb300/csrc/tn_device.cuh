@@ -310,6 +310,16 @@ struct SmemLayout {
   __host__ __device__ static size_t total(int P) { return head_bytes + arena_bytes(P); }
 };
 
+// A pointer into the kernel's dynamic shared memory, written from that memory's
+// own symbol: accesses through it are shared-memory ones.  Functions that are not
+// inlined get generic pointers otherwise, and their inner loops take up to twice
+// as long.
+template <typename X>
+__device__ __forceinline__ X *as_shared(X *p) {
+  extern __shared__ __align__(256) unsigned char smem[];
+  return reinterpret_cast<X *>(smem + (tc::smem_u32(p) - tc::smem_u32(smem)));
+}
+
 template <typename T>
 size_t __host__ __device__ team_bytes(int cap);
 
@@ -329,7 +339,24 @@ struct Smem {
   unsigned char *oz = nullptr;  // double-float executor: tensor-core update staging (1024-byte aligned)
   size_t arena;                 // bytes from r0 on
   unsigned char *base;
-  __device__ Smem(unsigned char *base_, int P) : base(base_) {
+  int sortP;
+  // The same layout from a base that the compiler knows to be shared memory (a
+  // pointer read back from a structure is a generic one), and the way back.
+  __device__ __forceinline__ Smem known() const {
+    Smem s(as_shared(base), sortP);
+    s.take(*this);
+    s.tmem = tmem;
+    s.tc = tc;
+    s.bar = bar;
+    s.gbar = gbar;
+    return s;
+  }
+  __device__ __forceinline__ void take(const Smem &o) {
+    phase = o.phase;
+    gphase = o.gphase;
+    tc_fail = o.tc_fail;
+  }
+  __device__ Smem(unsigned char *base_, int P) : base(base_), sortP(P) {
     using L = SmemLayout<T, W>;
     unsigned char *p = base;
     red = reinterpret_cast<double *>(p);
@@ -443,8 +470,9 @@ __device__ __noinline__ void build_theta(const cpx<T> *__restrict__ gk, const cp
                             const T *__restrict__ lamL, const T *__restrict__ lamM,
                             const T *__restrict__ lamR, int cL, int cM, int cR,
                             const double *__restrict__ gate, cpx<T> *__restrict__ A, cpx<T> *__restrict__ T0,
-                            bool colmode, Smem<T, W> &sm) {
+                            bool colmode, Smem<T, W> &sm_) {
   using L = SmemLayout<T, W>;
+  Smem<T, W> sm = sm_.known();
   constexpr int TILE = L::TILE, TU = L::TU;
   constexpr int PER = (TILE * TILE) / NT;  // (v,w) outputs per thread
   static_assert(PER >= 1 && (TILE * TILE) % NT == 0, "tile/threads");
@@ -1252,26 +1280,26 @@ __device__ void gram_res(int ell, Smem<T, W> &sm) {
   __syncthreads();
 }
 
-// Ab <- Ab J in place (Ab resident, ell <= 4 * NT / 4 rows): thread owns
-// 4 rows x 8 columns, all products formed before the barrier, then stored.
-template <typename T, int NT, int W>
-__device__ void update_res(int ell, const cpx<T> *__restrict__ Jm, Smem<T, W> &sm) {
+// Ab <- Ab J in place (Ab resident): thread owns NR rows x 8 columns, all
+// products formed before the barrier, then stored.  NR = ceil(ell / (NT / 4)):
+// with four rows a thread whatever ell is, 128 rows took as long as 512 (18 us).
+template <typename T, int NT, int W, int NR>
+__device__ __forceinline__ void update_res_rows(int ell, const cpx<T> *__restrict__ Jm, Smem<T, W> &sm) {
   static_assert(W == 32 && NT % 4 == 0, "resident update layout");
   constexpr int TP = SmemLayout<T, W>::AP, RB = NT / 4;
-  static_assert(SmemLayout<T, W>::RES_ROWS <= 4 * RB, "one pass covers every resident row");
   const int qb = threadIdx.x / RB, rb = threadIdx.x % RB;
   const int q0 = qb * 8;
-  cpx<T> acc[4][8];
+  cpx<T> acc[NR][8];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < NR; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[i][j] = czero<T>();
   static_assert(TP % 2 == 0 && sizeof(T) == 4, "16-byte pairs");
   for (int p = 0; p < W; p += 2) {
     // slots p, p + 1 of each of the thread's rows in one 16-byte read
-    float4 a2[4];
+    float4 a2[NR];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < NR; ++i) {
       const int r = rb + i * RB;
       a2[i] = r < ell ? *reinterpret_cast<const float4 *>(sm.Ab + r * TP + p) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -1281,7 +1309,7 @@ __device__ void update_res(int ell, const cpx<T> *__restrict__ Jm, Smem<T, W> &s
 #pragma unroll
       for (int j = 0; j < 8; ++j) jr[j] = Jm[(p + h) * (W + 1) + q0 + j];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < NR; ++i) {
         const cpx<T> a = h ? mkc<T>(a2[i].z, a2[i].w) : mkc<T>(a2[i].x, a2[i].y);
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] = cfma(a, jr[j], acc[i][j]);
@@ -1290,7 +1318,7 @@ __device__ void update_res(int ell, const cpx<T> *__restrict__ Jm, Smem<T, W> &s
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < NR; ++i) {
     const int r = rb + i * RB;
     if (r < ell) {
       float4 *dst = reinterpret_cast<float4 *>(sm.Ab + r * TP + q0);
@@ -1300,6 +1328,19 @@ __device__ void update_res(int ell, const cpx<T> *__restrict__ Jm, Smem<T, W> &s
     }
   }
   __syncthreads();
+}
+
+template <typename T, int NT, int W>
+__device__ void update_res(int ell, const cpx<T> *__restrict__ Jm, Smem<T, W> &sm) {
+  static_assert(SmemLayout<T, W>::RES_ROWS <= NT, "four rows a thread cover every resident row");
+  if (ell <= NT / 4)
+    update_res_rows<T, NT, W, 1>(ell, Jm, sm);
+  else if (ell <= NT / 2)
+    update_res_rows<T, NT, W, 2>(ell, Jm, sm);
+  else if (ell <= 3 * NT / 4)
+    update_res_rows<T, NT, W, 3>(ell, Jm, sm);
+  else
+    update_res_rows<T, NT, W, 4>(ell, Jm, sm);
 }
 
 // Rotation of the Hermitian 2x2 [[a, g], [conj g, b]] that zeroes g
@@ -1528,8 +1569,9 @@ template <typename T, int NT, int W>
 __device__ void bitonic_desc(double *key, int *idx, int P);
 
 template <typename T, int NT, int W>
-__device__ __noinline__ int jacobi_svd(cpx<T> *__restrict__ A, int ell, int c, int max_sweeps, Smem<T, W> &sm,
-                          long long *cyc, double *__restrict__ nrm, int *__restrict__ ord, int scheme) {
+__device__ __forceinline__ int jacobi_svd_body(cpx<T> *__restrict__ A, int ell, int c, int max_sweeps, Smem<T, W> &sm,
+                                               long long *cyc, double *__restrict__ nrm, int *__restrict__ ord,
+                                               int scheme) {
   using L = SmemLayout<T, W>;
   constexpr int B = W / 2;
   const bool resident = (L::RES_ROWS > 0) && ell <= L::RES_ROWS;
@@ -1836,6 +1878,18 @@ __device__ __noinline__ int jacobi_svd(cpx<T> *__restrict__ A, int ell, int c, i
   return -1;
 }
 
+// One copy for its several callers.  The layout is rebuilt from an address
+// known to be in shared memory: through the caller's structure every access
+// would be a generic one, which doubles the time of the inner rotations.
+template <typename T, int NT, int W>
+__device__ __noinline__ int jacobi_svd(cpx<T> *__restrict__ A, int ell, int c, int max_sweeps, Smem<T, W> &sm_,
+                                       long long *cyc, double *__restrict__ nrm, int *__restrict__ ord, int scheme) {
+  Smem<T, W> sm = sm_.known();
+  const int sw = jacobi_svd_body<T, NT, W>(A, ell, c, max_sweeps, sm, cyc, nrm, ord, scheme);
+  sm_.take(sm);
+  return sw;
+}
+
 // =======================================================================
 // Phase 3: singular values, sort, process_svd (mps.rs:236-293), Gamma
 // rebuild (mps.rs:856-877 / 1357-1382), local_renormalize (1206-1209).
@@ -2027,7 +2081,8 @@ template <typename T, int NT, int W>
 __device__ __noinline__ void finalize_bond(const TrajDev &tr, int k, cpx<T> *__restrict__ gk, cpx<T> *__restrict__ gk1,
                               const double *__restrict__ lamL, double *__restrict__ lamM,
                               const double *__restrict__ lamR, int cL, int cR, bool colmode, int ell, int c,
-                              Work<T> &wk, Smem<T, W> &sm) {
+                              Work<T> &wk, Smem<T, W> &sm_) {
+  Smem<T, W> sm = sm_.known();
   const int P = [&] {
     int p = 1;
     while (p < c) p <<= 1;
@@ -2166,6 +2221,7 @@ __device__ __noinline__ void finalize_bond(const TrajDev &tr, int k, cpx<T> *__r
   for (int j = threadIdx.x; j < rank; j += NT) lamM[j] = wk.s2[j];
   if (threadIdx.x == 0) tr.chi[k + 1] = rank;
   __syncthreads();
+  sm_.take(sm);
 }
 
 // ---------------------------------------------------------- accessors
@@ -2229,7 +2285,8 @@ template <typename T, int NT, int W>
 __device__ __noinline__ bool refactor_lq(const cpx<T> *__restrict__ gk, const cpx<T> *__restrict__ gk1,
                             const T *__restrict__ lamL, const T *__restrict__ lamM,
                             const T *__restrict__ lamR, int cL, int cM, int cR, int cap, Work<T> &wk,
-                            Smem<T, W> &sm) {
+                            Smem<T, W> &sm_) {
+  Smem<T, W> sm = sm_.known();
   const int m = 2 * cL, nc = 2 * cR;
   cpx<T> *S = wk.A + size_t(2) * cap * cap;  // chiM x chiM, after M's m x chiM region
   // S = B B^H
@@ -2241,7 +2298,10 @@ __device__ __noinline__ bool refactor_lq(const cpx<T> *__restrict__ gk, const cp
       },
       [&](int x, int y, cpx<T> v) { S[size_t(x) * cM + y] = v; }, sm);
   const double rel = sizeof(T) == 4 ? 0.1 : 1e-3;
-  if (!cholesky_lower<T, NT, W>(S, cM, rel, wk.sig, sm)) return false;
+  if (!cholesky_lower<T, NT, W>(S, cM, rel, wk.sig, sm)) {
+    sm_.take(sm);
+    return false;
+  }
   // M = X diag(Lambda_k) L, stored vector-contiguous: A[j*m + i] = M[i][j]
   cpx<T> *A = wk.A;
   gemm_nt_auto<T, NT, W>(
@@ -2249,6 +2309,7 @@ __device__ __noinline__ bool refactor_lq(const cpx<T> *__restrict__ gk, const cp
       [&](int i, int u) { return cscale(gk[size_t(i) * cM + u], lamL[i >> 1] * lamM[u]); },
       [&](int j, int u) { return u >= j ? S[size_t(u) * cM + j] : czero<T>(); },
       [&](int i, int j, cpx<T> v) { A[size_t(j) * m + i] = v; }, sm);
+  sm_.take(sm);
   return true;
 }
 
@@ -2258,7 +2319,8 @@ __device__ __noinline__ bool refactor_lq(const cpx<T> *__restrict__ gk, const cp
 template <typename TS, int NT, int W>
 __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL, int cM, int cR, const double *gate,
                                                const LocalBond<typename LocalType<TS>::type> &pl, bool try_lq,
-                                               int max_sweeps, Work<TS> &wk, Smem<TS, W> &sm, long long *cyc) {
+                                               int max_sweeps, Work<TS> &wk, Smem<TS, W> &sm_, long long *cyc) {
+  Smem<TS, W> sm = sm_.known();
   using T = typename LocalType<TS>::type;  // of the arithmetic; TS: of the state
   using R = typename RedType<T>::type;
   constexpr bool kExact = std::is_same<T, TS>::value;
@@ -2266,7 +2328,6 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
   const int m = 2 * cL, nc = 2 * cR;
   cpx<TS> *gk = gamma_slot<TS>(tr, k), *gk1 = gamma_slot<TS>(tr, k + 1);
   unsigned char *at = sm.r0;
-  __builtin_assume(__isShared(at));
   cpx<T> *T0 = reinterpret_cast<cpx<T> *>(at);
   at += pl.theta;
   cpx<T> *A = reinterpret_cast<cpx<T> *>(at);
@@ -2673,7 +2734,8 @@ __device__ __forceinline__ bool team_takes(const Team &tm, int cL, int cM, int c
 // as bond_op.  Every member calls it; team-uniform.
 template <typename T, int NT, int W>
 __device__ __noinline__ void bond_team(const Team &tm, const TrajDev &tr, int k, const double *gate, int max_sweeps,
-                                       int scheme, Work<T> &wk, Smem<T, W> &sm) {
+                                       int scheme, Work<T> &wk, Smem<T, W> &sm_) {
+  Smem<T, W> sm = sm_.known();
   using R = typename RedType<T>::type;
   constexpr bool kDD = std::is_same<T, dd>::value;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -2885,18 +2947,9 @@ __device__ __noinline__ void bond_team(const Team &tm, const TrajDev &tr, int k,
   tm.sync();
   const T *sL = wk.scl, *sR = wk.scl + tr.cap, *isig = wk.isig, *isig2 = wk.isig2, *w2 = wk.w2;
   const int *perm = wk.perm;
-  T pk = T(0), pk1 = T(0);
-  auto put0 = [&](int i, int j, cpx<T> u) {
-    const cpx<T> v = cscale(u, sL[i >> 1]);
-    gk[size_t(i) * rank + j] = v;
-    const T l = lL[i >> 1];
-    pk += cabs2(v) * (l * l) * w2[j];
-  };
+  auto put0 = [&](int i, int j, cpx<T> u) { gk[size_t(i) * rank + j] = cscale(u, sL[i >> 1]); };
   auto put1 = [&](int j, int col, cpx<T> u) {
-    const int w = col < cR ? col : col - cR;
-    const cpx<T> v = cscale(u, sR[w]);
-    gk1[size_t(j) * nc + col] = v;
-    pk1 += cabs2(v) * w2[j] * (lR[w] * lR[w]);
+    gk1[size_t(j) * nc + col] = cscale(u, sR[col < cR ? col : col - cR]);
   };
   const cpx<T> *A = wk.A, *T0 = wk.T0;
   if (colmode) {
@@ -2949,21 +3002,32 @@ __device__ __noinline__ void bond_team(const Team &tm, const TrajDev &tr, int k,
         },
         sm, tm.rank, tm.size);
   }
-  // renormalisation: the members' sums in their order
-  R nk = R(pk), nk1 = R(pk1);
-  block_sum2_in<R, NT>(nk, nk1, sm.red);
-  R *part_sum = reinterpret_cast<R *>(wk.sig);
-  if (tid == 0) {
-    part_sum[2 * tm.rank] = nk;
-    part_sum[2 * tm.rank + 1] = nk1;
+  tm.sync();
+  // renormalisation: a sum per row, then the rows in a fixed order, so that the
+  // result has the same bits whatever the team's size
+  R *row0 = reinterpret_cast<R *>(wk.A), *row1 = row0 + m;  // (the vectors have served)
+  for (int i = tm.rank * (NT / 32) + warp; i < m + rank; i += tm.size * (NT / 32)) {
+    T part = T(0);
+    if (i < m) {
+      const T l = lL[i >> 1];
+      for (int j = lane; j < rank; j += 32) part += cabs2(gk[size_t(i) * rank + j]) * (l * l) * w2[j];
+    } else {
+      const cpx<T> *row = gk1 + size_t(i - m) * nc;
+      for (int col = lane; col < nc; col += 32) {
+        const T l = lR[col < cR ? col : col - cR];
+        part += cabs2(row[col]) * w2[i - m] * (l * l);
+      }
+    }
+    R s = R(part);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s = s + shfl_xor(s, o);
+    if (lane == 0) row0[i] = s;
   }
   tm.sync();
-  nk = R(0);
-  nk1 = R(0);
-  for (int i = 0; i < tm.size; ++i) {
-    nk = nk + part_sum[2 * i];
-    nk1 = nk1 + part_sum[2 * i + 1];
-  }
+  R nk = R(0), nk1 = R(0);
+  for (int i = tid; i < m; i += NT) nk = nk + row0[i];
+  for (int i = tid; i < rank; i += NT) nk1 = nk1 + row1[i];
+  block_sum2_in<R, NT>(nk, nk1, sm.red);
   const T ik = T(R(1) / sqrt(nk)), ik1 = T(R(1) / sqrt(nk1));
   for (int o = gid; o < m * rank; o += gthreads) gk[o] = cscale(gk[o], ik);
   for (int o = gid; o < rank * nc; o += gthreads) gk1[o] = cscale(gk1[o], ik1);
@@ -2983,6 +3047,7 @@ __device__ __noinline__ void bond_team(const Team &tm, const TrajDev &tr, int k,
     atomicAdd(tr.stats + STAT_CYC_FINAL, double(clock64() - c2));
     atomicAdd(tr.stats + STAT_BLOCK_STEPS, double(cyc[3]));
   }
+  sm_.take(sm);
   tm.sync();
 }
 

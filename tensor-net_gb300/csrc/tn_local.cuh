@@ -316,10 +316,10 @@ constexpr float kOffMax = 2e-5f, kDiagMax = 0.1f;
 template <typename T, int NT>
 __device__ __noinline__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S, int ps, cpx<T> *Q, int pq, dd *dg,
                                        double *red) {
-  __builtin_assume(__isShared(Vs));
-  __builtin_assume(__isShared(S));
-  __builtin_assume(__isShared(Q));
-  __builtin_assume(__isShared(dg));
+  Vs = as_shared(Vs);
+  S = as_shared(S);
+  Q = as_shared(Q);
+  dg = as_shared(dg);
   constexpr int OPT = NT >= 512 ? 8 : 8;  // outputs per thread: c <= 64 at 512 threads, c <= 32 at 128
   const int tid = threadIdx.x;
   const int ntri = c * (c + 1) / 2;
@@ -702,8 +702,8 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
 template <typename T, int NT>
 __device__ __noinline__ int svd_local_global(cpx<T> *A, int ell, int c, int max_sweeps, unsigned char *scratch,
                                              double *red) {
-  __builtin_assume(__isShared(scratch));
-  __builtin_assume(__isShared(red));
+  scratch = as_shared(scratch);
+  red = as_shared(red);
   return svd_local<T, NT>(A, ell, ell, c, max_sweeps, scratch, red, svd_tolerance<T>(ell));
 }
 

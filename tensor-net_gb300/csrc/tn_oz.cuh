@@ -134,7 +134,8 @@ enum OzOut { kOzPlain, kOzTrans, kOzHerm, kOzHermT };
 // barrier.
 template <int NT, typename S>
 __device__ __noinline__ void oz_gemm(const Team &tm, const OzPlanes &P, const OzPlanes &Q, bool conj, int nlev,
-                                     OzOut out, cpx<dd> *C, int ldc, const cpx<dd> *add, S &sm) {
+                                     OzOut out, cpx<dd> *C, int ldc, const cpx<dd> *add, S &sm_) {
+  S sm = sm_.known();
   const bool tri = out == kOzHerm || out == kOzHermT;
   static_assert(NT == 512, "16 warps: 4 row quarters x 4 column quarters of a tile");
   constexpr uint32_t IDESC = tc::idesc_bf16(kOzM, 2 * kOzN);
@@ -142,8 +143,7 @@ __device__ __noinline__ void oz_gemm(const Team &tm, const OzPlanes &P, const Oz
   const int nch = P.ld / kOzKC;
   const int tm_ = (P.rows + kOzM - 1) / kOzM, tn_ = (Q.rows + kOzN - 1) / kOzN;
   const int ndp = min(P.nd, nlev), ndq = min(Q.nd, nlev);
-  unsigned char *base = sm.r0;
-  __builtin_assume(__isShared(base));
+  unsigned char *base = as_shared(sm.r0);
   int mine = 0;
   for (int t = 0; t < tm_ * tn_; ++t) {
     const int i0 = (t % tm_) * kOzM, y0 = (t / tm_) * kOzN;
@@ -269,6 +269,7 @@ __device__ __noinline__ void oz_gemm(const Team &tm, const OzPlanes &P, const Oz
       }
     }
   }
+  sm_.take(sm);
   __syncthreads();
 }
 

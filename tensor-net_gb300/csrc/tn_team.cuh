@@ -26,15 +26,16 @@ struct TeamWork {
   unsigned int *flag;  // cross-CTA flags and maxima
 };
 constexpr int kTeamFlags = 64;
+constexpr int kTeamItem = 8;  // words after the flags: the work item that the first member took
 
 // Bytes of that workspace for bond capacity cap; zero where svd_team does not run.
 template <typename T>
 size_t __host__ __device__ team_bytes(int cap) {
   if (2 * cap <= 64) return 0;  // bond_local takes every bond
-  if (!std::is_same<T, dd>::value) return sizeof(T) == 4 ? size_t(2) * cap * sizeof(float) + kTeamFlags * 4 + 512 : 0;
+  if (!std::is_same<T, dd>::value) return sizeof(T) == 4 ? size_t(2) * cap * sizeof(float) + 2048 : 0;
   const size_t n4 = size_t(4) * cap * cap, rows = size_t(2) * cap, ld = size_t(4) * cap + 32;
   size_t b = 2 * n4 * sizeof(cpx<float>) + 2 * n4 * sizeof(cpx<dd>) + 2 * (8 * rows * ld * 2) + 2 * rows * sizeof(int) +
-             rows * (2 * sizeof(float) + sizeof(dd)) + kTeamFlags * sizeof(int) + 4096;
+             rows * (2 * sizeof(float) + sizeof(dd)) + (kTeamFlags + kTeamItem) * sizeof(int) + 4096;
   return (b + 255) & ~size_t(255);
 }
 
@@ -48,7 +49,7 @@ __device__ inline TeamWork team_work(void *base, int cap) {
     return q;
   };
   const size_t n4 = size_t(4) * cap * cap, rows = size_t(2) * cap, ld = size_t(4) * cap + 32;
-  w.flag = reinterpret_cast<unsigned int *>(take(kTeamFlags * sizeof(int)));
+  w.flag = reinterpret_cast<unsigned int *>(take((kTeamFlags + kTeamItem) * sizeof(int)));
   w.nrm = reinterpret_cast<float *>(take(rows * sizeof(float)));
   if (std::is_same<T, dd>::value) {
     w.dg = reinterpret_cast<dd *>(take(rows * sizeof(dd)));
@@ -151,7 +152,7 @@ template <int NT, int W, typename S>
 __device__ int float_sweeps(const Team &tm, cpx<float> *A32, int ell, cpx<float> *V32, int c, float floor_, float done,
                             int max_sweeps, TeamWork &tw, int &slot, S &sm, long long *cyc) {
   constexpr int B = W / 2;
-  Smem<float, W> sf(sm.base, 1);
+  Smem<float, W> sf(as_shared(sm.base), 1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nblk = (c + B - 1) / B;
   const float tol = 4.f * sqrtf(float(ell)) * Eps<float>::v;
