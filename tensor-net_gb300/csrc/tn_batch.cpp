@@ -72,6 +72,10 @@ struct tn_batch {
   void *ws = nullptr;
   size_t ws_stride = 0;
   bool ws_team = false;
+  // Upper estimates of the slots' bond dimensions (a layer's disjoint gates at
+  // most double them), for the launch shape only.
+  std::vector<uint32_t> chi_hint;
+  int clusters4 = -1, clusters8 = -1;  // resident clusters (-1: not asked yet)
   // step buffers: one packed device block + one pinned host block
   void *dstep = nullptr, *hstep = nullptr;
   size_t step_bytes = 0;
@@ -185,6 +189,7 @@ int ensure_step(tn_batch *b, uint32_t nt, uint32_t ng, uint32_t nm) {
 }
 
 struct StepPtrs {
+  uint32_t chi_hint = 0;  // widest listed bond (0: unknown)
   const int *list, *order, *goff, *gks, *moff, *mks;
   const int *posts = nullptr;  // per measurement: 0 / 1 post-selected (Meas::Proj), else sampled; null = all sampled
   const double *gates, *us;
@@ -307,8 +312,25 @@ int launch_step(tn_batch *b, uint32_t nt, const StepPtrs &P0, bool timed = true)
     la.dyn_head = b->dcounter + 10;
     la.nsweeps = int(nt + phantom);
     la.queue_wait_ns = b->queue_wait_ns;
+    // A layer lasts as long as its heaviest trajectory's refactor chain. With at
+    // most one trajectory an SM, and bonds wide enough for operations that a
+    // cluster shares (beyond chi = 64), clusters of CTAs shorten that chain by
+    // more than the idle members cost on narrow bonds: 152 trajectories at n =
+    // 16, chi = 128, two layers: 210 -> 108 ms.  Beyond that the SMs have trajectories of their own.
+    // The results have the same bits either way.
+    int grid = gmax;
+    if (b->prec == TN_PREC_DF && b->ws_team && b->grid_limit == 0 && P.chi_hint > 64 && nt <= uint32_t(b->sms)) {
+      const int size = nt <= uint32_t(b->sms) / 8 ? 8 : 4;
+      int &n = size == 8 ? b->clusters8 : b->clusters4;
+      if (n < 0) n = run_clusters(b->prec, b->sortP, size);
+      const int teams = std::min(n, gmax);
+      if (teams > 0) {
+        la.cluster = size;
+        grid = teams;
+      }
+    }
     if (timed) CKB(cudaEventRecord(b->ev[0], b->st));
-    CKB(launch_run(b->prec, la, gmax, b->sortP, b->maxcap, b->st));
+    CKB(launch_run(b->prec, la, grid, b->sortP, b->maxcap, b->st));
     if (timed) {
       CKB(cudaEventRecord(b->ev[1], b->st));
       CKB(cudaEventRecord(b->ev[2], b->st));
@@ -494,6 +516,8 @@ int tn_batch_reset(tn_batch *b, uint32_t t, uint32_t n, const tn_trunc *trunc) {
                       : std::min<uint32_t>(max_rank(n), 256);
   if (want > b->cap[t]) return TN_ERR_CAPACITY;
   d.n = int(n);
+  b->chi_hint.resize(b->ntraj, 1);
+  b->chi_hint[t] = 1;
   if (trunc) {
     d.trunc_mode = trunc->mode;
     d.chi_max = int(std::min<uint32_t>(trunc->chi_max, 0x7fffffff));
@@ -534,6 +558,8 @@ int tn_batch_import(tn_batch *b, uint32_t t, uint32_t n, const uint32_t *chi, co
   CKB(cudaStreamSynchronize(b->st));
   TrajDev &d = b->h[t];
   d.n = int(n);
+  b->chi_hint.resize(b->ntraj, 1);
+  b->chi_hint[t] = *std::max_element(chi, chi + n + 1);
   if (trunc) {
     d.trunc_mode = trunc->mode;
     d.chi_max = int(std::min<uint32_t>(trunc->chi_max, 0x7fffffff));
@@ -660,6 +686,12 @@ int tn_batch_step_post(tn_batch *b, const uint32_t *trajs, uint32_t nt, const ui
   CKB(cudaMemcpyAsync(b->dstep, b->hstep, L.in_bytes, cudaMemcpyHostToDevice, b->st));
   StepPtrs P = ptrs_of(L, reinterpret_cast<char *>(b->dstep));
   P.order = nullptr;  // ranked on the device from the current bond dimensions
+  b->chi_hint.resize(b->ntraj, 1);
+  for (uint32_t i = 0; i < nt; ++i) {
+    uint32_t &hint = b->chi_hint[trajs[i]];
+    if (gate_off[i + 1] > gate_off[i]) hint = std::min<uint32_t>(uint32_t(b->h[trajs[i]].cap), 2 * hint);
+    P.chi_hint = std::max(P.chi_hint, hint);
+  }
   P.posts = posts ? reinterpret_cast<const int *>(reinterpret_cast<char *>(b->dstep) + L.posts) : nullptr;
   const bool step_ev = b->ev_step[0] && b->ev_step[1];  // (not created for the server's engines)
   if (step_ev) CKB(cudaEventRecord(b->ev_step[0], b->st));
@@ -710,6 +742,7 @@ int tn_batch_device_inputs(tn_batch *b, uint32_t max_gates, uint32_t max_meas, v
 int tn_batch_step_device(tn_batch *b, uint32_t nt) {
   if (!b || !b->din || nt > b->ntraj) return TN_ERR_INVALID_ARG;
   if (nt == 0) return TN_OK;
+  b->chi_hint.assign(b->ntraj, 0x3fffffffu);  // gates that the host does not see
   StepLayout L = step_layout(b->ntraj, b->din_gates, b->din_meas);
   auto it = b->graphs.find(nt);
   if (it == b->graphs.end()) {
@@ -740,6 +773,7 @@ int tn_batch_step_ptrs(tn_batch *b, uint32_t nt, const void *d_trajs, const void
   if (!b || nt > b->ntraj || !d_trajs || !d_gate_off || !d_meas_off || !d_entropy)
     return TN_ERR_INVALID_ARG;
   if (nt == 0) return TN_OK;
+  b->chi_hint.assign(b->ntraj, 0x3fffffffu);  // gates that the host does not see
   if (int s = ensure_step(b, b->ntraj, 1, 1)) return s;
   StepPtrs P;
   P.list = static_cast<const int *>(d_trajs);

@@ -91,8 +91,8 @@ struct LaunchArgs {
   void *ws;              // per-CTA workspace
   size_t ws_stride;      // bytes per CTA
   int ws_team;           // 1: the workspace includes svd_team's part
-  // CTAs that share an item (a cluster; static schedule only, items dealt out
-  // by cluster index, a workspace per cluster); 0 or 1: one
+  // CTAs that share an item (a cluster, with one workspace that has svd_team's
+  // part); 0 or 1: one
   int cluster;
   int max_sweeps;
   int jacobi_scheme;      // 0: block pairs, all pairs per step; 1: within-block then cross-block steps

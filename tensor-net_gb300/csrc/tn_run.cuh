@@ -63,15 +63,11 @@ __global__ void __launch_bounds__(NT, 1) k_run(LaunchArgs la, int sortP, int ws_
     sm.phase = 0;
     sm.tc = la.theta_simt == 0;
   }
-  if (tm.size > 1) {
-    for (int it = team_id; it < la.nitems; it += int(gridDim.x) / tm.size) {
-      const Item item = la.items[it];
-      run_program<T, NT, W>(tm, la, la.prog, item, wk, sm);
-      tm.sync();
-    }
-  }
-  for (; tm.size == 1;) {
-    if (threadIdx.x == 0) {
+  // A team's first member takes the items and passes them on through the team's
+  // workspace (a launch with clusters has one).
+  volatile unsigned int *pass = tm.size > 1 ? team_work<T>(wk.team, ws_cap).flag + kTeamFlags : nullptr;
+  for (;;) {
+    if (threadIdx.x == 0 && tm.rank == 0) {
       const int G = la.nitems_dev ? *la.nitems_dev : la.nitems;
       int kind = 0, slot_i = -1;
       if (dd) {
@@ -115,19 +111,37 @@ __global__ void __launch_bounds__(NT, 1) k_run(LaunchArgs la, int sortP, int ws_
         if (kind == 2) s_item = Item{slot->traj, slot->off, slot->len, 0};
       }
       s_kind = kind;
+      if (tm.size > 1) {
+        pass[0] = unsigned(kind);
+        if (kind == 1 || kind == 2) {
+          pass[1] = unsigned(s_item.traj);
+          pass[2] = unsigned(s_item.off);
+          pass[3] = unsigned(s_item.len);
+          pass[4] = unsigned(s_item.aux);
+        }
+      }
     }
-    __syncthreads();
-    const int kind = s_kind;
-    const Item item = s_item;
-    __syncthreads();
+    int kind;
+    Item item;
+    if (tm.size > 1) {
+      tm.sync();
+      kind = int(pass[0]);
+      item = Item{int(pass[1]), int(pass[2]), int(pass[3]), int(pass[4])};
+      tm.sync();
+    } else {
+      __syncthreads();
+      kind = s_kind;
+      item = s_item;
+      __syncthreads();
+    }
     if (kind == 0) break;
     if (kind == 3) continue;
     if (kind == 2) __threadfence();  // acquire side for every thread of the CTA
     run_program<T, NT, W>(tm, la, (dd && kind == 1) ? la.gprog : la.prog, item, wk, sm);
     if (dd && kind == 1) {
       __threadfence();  // this thread's writes of the gate's result, visible device-wide
-      __syncthreads();
-      if (threadIdx.x == 0 && atomicSub(la.rem + item.aux, 1) == 1) {
+      tm.sync();
+      if (threadIdx.x == 0 && tm.rank == 0 && atomicSub(la.rem + item.aux, 1) == 1) {
         __threadfence();
         push_sweep(la.dyn, la.dyn_tail, la.sweeps, item.aux);
       }

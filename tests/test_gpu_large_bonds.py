@@ -54,3 +54,29 @@ def test_gate_and_measurement_on_large_bond(pkg, ref, kind, n, chi, prec):
         w = int(np.sum(r > (1e-4 if prec == "mixed" else 1e-8)))
         assert s.size >= w and np.max(np.abs(s[:w] - r[:w])) < TOL[prec], bd
     assert b.device_status() == 0
+
+
+def test_same_bits_on_teams_of_every_size(pkg):
+    """A double-float layer on clusters of eight (2 trajectories), of four (24)
+    and on single CTAs (160, more than there are SMs): outcomes, probabilities,
+    entropies and Schmidt values with the same bits."""
+    n, chi = 14, 100
+    _, psi = _state("random", n, 128, 22)
+    tr = pkg.Trunc.both(chi, 1e-10)
+    m = pkg.MPS.from_vector(psi, tr, "df")
+    parts = m.export_parts()
+    layers = [pkg.gen_layer(31, 0, t, n, 0.2) for t in range(2)]
+    got = []
+    for count in (2, 24, 160):
+        b = pkg.Batch([n] * count, [tr] * count, "df")
+        for i in (0, count - 1):
+            b.import_state(i, *parts, tr)
+        out = []
+        for la in layers:
+            recs, ent = b.step(list(range(count)), [la] * count)
+            out += [recs[0], recs[-1], ent[0], ent[-1]]
+        out += [b.svals(i, k).tolist() for i in (0, count - 1) for k in range(n - 1)]
+        assert b.device_status() == 0
+        b.close()
+        got.append(out)
+    assert got[0] == got[1] == got[2]
