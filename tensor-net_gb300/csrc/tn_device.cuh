@@ -2347,6 +2347,15 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
   for (int v = tid; v < cL; v += NT) lL[v] = T(lamL[v]);
   for (int u = tid; u < cM; u += NT) lM[u] = T(lamM[u]);
   for (int w = tid; w < cR; w += NT) lR[w] = T(lamR[w]);
+  // the gate and the rank rule's threshold in the arithmetic used here: float64
+  // conversions and comparisons are slow enough to be done once, by idle warps
+  T *op = reinterpret_cast<T *>(sm.red + 64);  // 32 real values
+  if (gate && tid >= NT - 64 && tid < NT - 32) op[tid - (NT - 64)] = T(gate[tid - (NT - 64)]);
+  R *eps = reinterpret_cast<R *>(sm.red) + 60;
+  if (tid == NT - 1) {
+    const bool cut = tr.trunc_mode == 2 || tr.trunc_mode == 3;
+    *eps = R(fmax(cut ? fabs(tr.cutoff) : 2.220446049250313e-16, rank_floor<TS>(pl.ell)));
+  }
   __syncthreads();
   // theta, one (v, w) with its four (s1, s2) a thread; dst2 gets the copy that the sweeps work on
   auto theta = [&](bool colmode, cpx<T> *dst2) {
@@ -2373,25 +2382,21 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
       cpx<T> th[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) th[q] = cscale(cscale(acc_fin<T>(acc[q]), lL[v]), lR[w]);
-      if (gate) {
-        cpx<T> t2[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          cpx<T> s = czero<T>();
-#pragma unroll
-          for (int b = 0; b < 4; ++b)
-            s = cfma(mkc<T>(T(gate[8 * a + 2 * b]), T(gate[8 * a + 2 * b + 1])), th[b], s);
-          t2[a] = s;
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a) th[a] = t2[a];
-      }
-#pragma unroll
+#pragma unroll 1
       for (int a = 0; a < 4; ++a) {
+        cpx<T> r;
+        if (gate) {
+          typename CAcc<T>::type s = acc_zero<T>();
+#pragma unroll
+          for (int b = 0; b < 4; ++b) acc_fma<T>(s, mkc<T>(op[8 * a + 2 * b], op[8 * a + 2 * b + 1]), th[b]);
+          r = acc_fin<T>(s);
+        } else {
+          r = a < 2 ? (a ? th[1] : th[0]) : (a == 2 ? th[2] : th[3]);
+        }
         const int i = 2 * v + (a >> 1), j = (a & 1) * cR + w;
         const int at2 = colmode ? j * ld + i : i * ld + j;
-        T0[at2] = th[a];
-        if (dst2) dst2[at2] = th[a];
+        T0[at2] = r;
+        if (dst2) dst2[at2] = r;
       }
     }
     __syncthreads();
@@ -2484,12 +2489,11 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) tot = tot + shfl_xor(tot, o);
     const int mode = tr.trunc_mode;
-    const double eps = fmax((mode == 2 || mode == 3) ? fabs(tr.cutoff) : 2.220446049250313e-16, rank_floor<TS>(ell));
-    const double least = eps * eps * double(tot);
+    const R least = *eps * *eps * tot;
     int bad = c;
     for (int j = lane; j < c; j += 32) {
-      const double x = double(ssq[j]);
-      if (!(isfinite(x) && x > least && x > 0.0)) bad = min(bad, j);
+      const R x = ssq[j];
+      if (!(isfinite(x) && x > least && x > R(0))) bad = min(bad, j);
     }
     const int nlead = __reduce_min_sync(0xffffffffu, bad);
     int rank = mode == 1 ? max(1, min(max(tr.chi_max, 1), nlead))
@@ -2502,25 +2506,30 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
     for (int j = lane; j < rank; j += 32) kept = kept + ssq[j];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) kept = kept + shfl_xor(kept, o);
-    const double dk = double(kept);
-    for (int j = lane; j < rank; j += 32) s2[j] = sqrt(double(ssq[j]) / dk);
     if (lane == 0) {
-      // norm of the kept values relative to all of them
-      reinterpret_cast<R *>(sm.red)[127] = sqrt(kept / tot);
+      reinterpret_cast<R *>(sm.red)[126] = kept;
+      reinterpret_cast<R *>(sm.red)[127] = tot;
       sm.ired[0] = rank;
     }
   }
   __syncthreads();
   const int rank = sm.ired[0];
-  const R n2 = reinterpret_cast<R *>(sm.red)[127];
+  // the stored Lambda in float64 (a warp or two of its own), the factors of the
+  // values (first warps) and of both outer bonds (last warps)
+  const R kept = reinterpret_cast<R *>(sm.red)[126];
   for (int j = tid; j < rank; j += NT) {
-    const R x = sqrt(ssq[j]), y = R(s2[j]), ix = R(1) / x;
-    isig[j] = T(ix);
-    isig2[j] = T(ix * ix);
-    w2[j] = T(y * y);
+    const R x = ssq[j], y = x / kept, ix2 = R(1) / x;
+    isig[j] = T(sqrt(ix2));
+    isig2[j] = T(ix2);
+    w2[j] = T(y);
   }
-  for (int v = tid; v < cL; v += NT) sL[v] = T(R(1) / R(lamL[v]));
-  for (int w = tid; w < cR; w += NT) sR[w] = T(n2 / R(lamR[w]));
+  if (tid >= 256)
+    for (int j = tid - 256; j < rank; j += NT - 256) s2[j] = sqrt(double(ssq[j]) / double(kept));
+  for (int v = NT - 1 - tid; v < cL; v += NT) sL[v] = T(R(1) / R(lL[v]));
+  if (int(threadIdx.x) >= 128 && int(threadIdx.x) < 128 + ((cR + 31) & ~31)) {
+    const R n2 = sqrt(kept / reinterpret_cast<R *>(sm.red)[127]);  // norm of the kept values relative to all
+    for (int w = tid - 128; w < cR; w += NT) sR[w] = T(n2 / R(lR[w]));
+  }
   __syncthreads();
   // Gamma_k and Gamma_{k+1}: one side from the vectors, the other recovered
   // from theta into the scratch; first the sums of local_renormalize, then
@@ -3096,7 +3105,8 @@ __device__ void measure_site(const TrajDev &tr, int k, double u, int post, int *
       atomicAdd(tr.stats + STAT_BYTES, double(sizeof(cpx<T>)) * 2.0 * 2.0 * tr.chi[k] * tr.chi[k + 1]);
     }
     if (out_outcome) *out_outcome = outcome;
-    if (out_prob) *out_prob = prob;
+    // (a certain outcome's float sum can come out one unit above 1)
+    if (out_prob) *out_prob = sizeof(T) == 4 && prob > 1.0 && prob < 1.0 + 1e-6 ? 1.0 : prob;
     const double ptol = (sizeof(T) == 8) ? 1e-9 : 1e-4;
     if (!(fabs(sum - 1.0) <= ptol)) atomicOr(tr.status, ST_PROB_SUM);
   }

@@ -178,7 +178,7 @@ __device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<flo
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cp = c + (c & 1), np = cp >> 1, ring = cp - 1;
   int LG = 32;
-  while (LG > 4 && np * LG > NT) LG >>= 1;
+  while (LG > 4 && (np * LG > NT || LG >= 2 * ell)) LG >>= 1;  // (short vectors need no more lanes)
   const int l = tid & (LG - 1), grp = tid / LG, ngrp = NT / LG;
   const int active = min(NT, ((np * LG + 31) >> 5) << 5);  // threads that own a pair (whole warps)
   const float tol2 = tol * tol, done2 = done * done;
@@ -192,16 +192,17 @@ __device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<flo
     }
     __syncthreads();
     float fro = 0.f;
-    for (int j = tid; j < c; j += NT) {
-      const float x = nrm[j];
+    {
+      const float x = tid < c ? nrm[tid] : 0.f;  // (c <= NT)
       int rk = 0;
+#pragma unroll 4
       for (int i = 0; i < c; ++i) {
         const float y = nrm[i];
-        rk += (y > x || (y == x && i < j)) ? 1 : 0;
+        fro += y;
+        rk += (y > x || (y == x && i < tid)) ? 1 : 0;
       }
-      ord[min(rk, c - 1)] = j;
+      if (tid < c) ord[min(rk, c - 1)] = tid;
     }
-    for (int i = 0; i < c; ++i) fro += nrm[i];
     const float tiny2 = fmaxf(fro * floor_ * floor_, 1e-37f);
     __syncthreads();
     int far = 0;
@@ -229,37 +230,35 @@ __device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<flo
           const float a = nrm[P], b = nrm[Q];
           __syncwarp();
           if (valid && a > tiny2 && b > tiny2) {
-            // scaled by the norms: g / (|a_p| |a_q|) stays in range for vectors of any size
-            const float ra = rsqrtf(a), rb = rsqrtf(b), sc = ra * rb;
-            const float hx = gx * sc, hy = gy * sc, r2 = fmaf(hx, hx, hy * hy);
-            far |= int(r2 > done2);
-            if (r2 > tol2) {
-              const float rr = rsqrt_near(r2);
-              const float z = 0.5f * ((b - a) * sc) * rr;
-              const float z1 = fmaf(z, z, 1.f);
-              const float tt = fabsf(z) > 1e15f ? __fdividef(0.5f, z)
-                                                : copysignf(__fdividef(1.f, fabsf(z) + z1 * rsqrtf(z1)), z);
-              // x' = x - s (y + tau x), y' = y + s (x - tau y), tau = s / (1 + c): one rounding of an element
-              // a rotation, and no scaling by an inexact c
-              const float cs = rsqrt_near(fmaf(tt, tt, 1.f)), sn = tt * cs, tau = __fdividef(sn, 1.f + cs);
-              const cpx<float> e = mkc<float>(hx * rr, -hy * rr);
+            // The rotation from the half difference d and h = sqrt(d^2 + |g|^2): cos^2 = (1 + |d| / h) / 2 and
+            // s e = conj(g) / (2 h c); scaled by a + b, so that vectors of any size stay in range.  Two square
+            // roots in a row instead of four special functions.
+            const float sc = __fdividef(1.f, a + b);
+            const float hx = gx * sc, hy = gy * sc, as = a * sc, bs = b * sc;
+            const float g2 = fmaf(hx, hx, hy * hy), ab = as * bs;
+            far |= int(g2 > done2 * ab);
+            if (g2 > tol2 * ab) {
+              const float d = 0.5f * (bs - as), h2 = fmaf(d, d, g2), rh = rsqrt_near(h2);
+              const float c2 = fmaf(0.5f * fabsf(d), rh, 0.5f), rc = rsqrt_near(c2), cs = c2 * rc;
+              const float w = copysignf(0.5f * rh * rc, d);
+              const cpx<float> se = mkc<float>(hx * w, -hy * w);
               for (int i = l; i < ell; i += LG) {
-                const cpx<float> x = ap[i], y = cmul(e, aq[i]);
-                ap[i] = mkc<float>(fmaf(-sn, fmaf(tau, x.x, y.x), x.x), fmaf(-sn, fmaf(tau, x.y, y.y), x.y));
-                aq[i] = mkc<float>(fmaf(sn, fmaf(-tau, y.x, x.x), y.x), fmaf(sn, fmaf(-tau, y.y, x.y), y.y));
+                const cpx<float> x = ap[i], y = aq[i];
+                ap[i] = mkc<float>(cs * x.x - (se.x * y.x - se.y * y.y), cs * x.y - (se.x * y.y + se.y * y.x));
+                aq[i] = mkc<float>(cs * y.x + (se.x * x.x + se.y * x.y), cs * y.y + (se.x * x.y - se.y * x.x));
               }
               if (Vs) {
                 cpx<float> *vp = Vs + P * pv, *vq = Vs + Q * pv;
                 for (int i = l; i < c; i += LG) {
-                  const cpx<float> x = vp[i], y = cmul(e, vq[i]);
-                  vp[i] = mkc<float>(fmaf(-sn, fmaf(tau, x.x, y.x), x.x), fmaf(-sn, fmaf(tau, x.y, y.y), x.y));
-                  vq[i] = mkc<float>(fmaf(sn, fmaf(-tau, y.x, x.x), y.x), fmaf(sn, fmaf(-tau, y.y, x.y), y.y));
+                  const cpx<float> x = vp[i], y = vq[i];
+                  vp[i] = mkc<float>(cs * x.x - (se.x * y.x - se.y * y.y), cs * x.y - (se.x * y.y + se.y * y.x));
+                  vq[i] = mkc<float>(cs * y.x + (se.x * x.x + se.y * x.y), cs * y.y + (se.x * x.y - se.y * x.x));
                 }
               }
-              if (l == 0) {
-                const float d = tt * (r2 * rr) * (a * ra) * (b * rb);
-                nrm[P] = a - d;
-                nrm[Q] = b + d;
+              if (l == 0) {  // t |g| = |g|^2 / (|d| + h), signed as d
+                const float u = copysignf(__fdividef(g2, fabsf(d) + h2 * rh), d) * (a + b);
+                nrm[P] = a - u;
+                nrm[Q] = b + u;
               }
             }
           }
@@ -284,11 +283,8 @@ __device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<flo
 // column a little (up to 1e-3 over long sweeps), and a rotation by t in I + K
 // has D = t^2.  dg_minus1: (1 + x)^(-1/2) - 1 in double-float.
 __device__ __forceinline__ dd dg_minus1(dd x) {
-  const dd r = dd(1.f) / sqrt(dd(1.f) + x);
-  // one correction step: r (1 + x) r = 1 to the working precision already; the
-  // small difference from 1 is what is wanted, without cancellation:
-  // r - 1 = -x / (s (1 + s)), s = sqrt(1 + x)
-  const dd s = dd(1.f) / r;
+  // without cancellation: 1 / s - 1 = -x / (s (1 + s)), s = sqrt(1 + x)
+  const dd s = sqrt(dd(1.f) + x);
   return -(x / (s * (dd(1.f) + s)));
 }
 // W[k][y] from S[k][y] (diagonal: x = S[k][k]), the factors dk, dy = D_g - 1 of
@@ -641,8 +637,12 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
       float fro = 0.f;
       for (int j = 0; j < c; ++j) fro += lead(G[j * pc + j].x);
       const float tiny2 = fmaxf(fro * floor_t * floor_t, 1e-37f);
-      // K of every pair above the threshold, r = |g| / (|a_p| |a_q|) and |t|
-      float rmax = 0.f, kmax = 0.f;
+      // K of every pair above the threshold, r = |g| / (|a_p| |a_q|) and |t|.
+      // Pairs below it, down to rounding, go along where their t is small: what
+      // they leave would enter the recovered side as r sigma_p / sigma_q, and
+      // with them a trajectory's error against float64 is 2-10 times smaller.
+      float rmax = 0.f, kmax = 0.f, small = 0.f;
+      const float least = tol < 1e-10f ? 0.03125f * tol : tol;
       for (int e = tid; e < c * (c + 1) / 2; e += NT) {
         int p, q;
         tri_entry(e, c, p, q);
@@ -658,15 +658,19 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
           const float sc = rsqrtf(a) * rsqrtf(b);
           const float hx = lead(g.x) * sc, hy = lead(g.y) * sc, r2 = fmaf(hx, hx, hy * hy), r = sqrtf(r2);
           rmax = fmaxf(rmax, r);
-          if (r > tol) {
+          if (r > least) {
             const float rr = 1.f / r;
             const float z = 0.5f * (lead(bt_ - at_) * sc) * rr;
             const float z1 = fmaf(z, z, 1.f);
             const float t = fabsf(z) > 1e15f ? 0.5f / z : copysignf(1.f / (fabsf(z) + sqrtf(z1)), z);
-            kmax = fmaxf(kmax, fabsf(t));
-            const float ex = hx * rr, ey = -hy * rr;
-            vqp = mkc<float>(-t * ex, -t * ey);
-            vpq = mkc<float>(t * ex, -t * ey);
+            const bool over = r > tol, take = over || fabsf(t) <= kFloatApply;
+            if (over) kmax = fmaxf(kmax, fabsf(t));
+            if (take) {
+              small = 1.f;
+              const float ex = hx * rr, ey = -hy * rr;
+              vqp = mkc<float>(-t * ex, -t * ey);
+              vpq = mkc<float>(t * ex, -t * ey);
+            }
           }
         }
         Vs[p * pc + q] = vqp;  // column p, row q
@@ -674,8 +678,12 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
       }
       rmax = block_max<NT>(rmax, red);
       kmax = block_max<NT>(kmax, red);
+      small = block_max<NT>(small, red);
       if (!(rmax < 2.f)) return -1;  // not a number
-      if (rmax <= tol) return sweeps + 1;
+      if (rmax <= tol) {
+        if (small > 0.f) apply_small<T, NT>(A, ld, ell + tail, c, Vs, pc, reinterpret_cast<cpx<float> *>(stage), pc);
+        return sweeps + 1;
+      }
       ++sweeps;
       // What is left after this step is of the order of the square: r r' between
       // vectors of different size (whose angles t are smaller than r), r t
@@ -748,7 +756,7 @@ template <typename T>
 struct LocalBond {
   static constexpr int MAXM = 64;
   size_t theta, vec, svd, lam, vals, total;
-  int c;
+  int c, ell;
   __host__ __device__ static size_t al(size_t x) { return (x + 15) & ~size_t(15); }
   __host__ __device__ static size_t most(size_t a, size_t b) { return a > b ? a : b; }
   __host__ __device__ bool plan(int cL, int cM, int cR, bool lq, size_t room, int nt) {
@@ -758,7 +766,7 @@ struct LocalBond {
     // vectors and their length; theta with the same pitch.  (LQ: cM vectors of
     // length m, theta as columns; the general path takes what LQ declines.)
     c = lq ? cM : mn;
-    const int ell = lq ? m : (m < nc ? nc : m);
+    ell = lq ? m : (m < nc ? nc : m);
     if (c > LocalSvd<T>::max_c(nt)) return false;
     theta = al(size_t(lq ? nc : mn) * (ell | 1) * e);
     vec = al(size_t(c) * (ell | 1) * e);
