@@ -2344,31 +2344,35 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
   const double *lamL = lam_slot(tr, k), *lamR = lam_slot(tr, k + 2);
   double *lamM = lam_slot(tr, k + 1);
   LocalResult res;
+#pragma unroll 1
   for (int v = tid; v < cL; v += NT) lL[v] = T(lamL[v]);
+#pragma unroll 1
   for (int u = tid; u < cM; u += NT) lM[u] = T(lamM[u]);
+#pragma unroll 1
   for (int w = tid; w < cR; w += NT) lR[w] = T(lamR[w]);
   // the gate and the rank rule's threshold in the arithmetic used here: float64
   // conversions and comparisons are slow enough to be done once, by idle warps
   T *op = reinterpret_cast<T *>(sm.red + 64);  // 32 real values
   if (gate && tid >= NT - 64 && tid < NT - 32) op[tid - (NT - 64)] = T(gate[tid - (NT - 64)]);
+  __syncthreads();
   R *eps = reinterpret_cast<R *>(sm.red) + 60;
-  if (tid == NT - 1) {
+  if (tid == NT - 1) {  // (read after many barriers)
     const bool cut = tr.trunc_mode == 2 || tr.trunc_mode == 3;
     *eps = R(fmax(cut ? fabs(tr.cutoff) : 2.220446049250313e-16, rank_floor<TS>(pl.ell)));
   }
-  __syncthreads();
   // theta, one (v, w) with its four (s1, s2) a thread; dst2 gets the copy that the sweeps work on
   auto theta = [&](bool colmode, cpx<T> *dst2) {
     const int ld = (colmode ? m : nc) | 1;
+#pragma unroll 1
     for (int o = tid; o < cL * cR; o += NT) {
       const int v = o / cR, w = o - v * cR;
       typename CAcc<T>::type acc[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[q] = acc_zero<T>();
       const cpx<TS> *x = gk + size_t(2 * v) * cM, *y = gk1 + w;
-#pragma unroll 2
+#pragma unroll 1
       for (int u = 0; u < cM; ++u) {
-        if ((u & 3) == 0) {
+        if ((u & 1) == 0) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) acc_renorm(acc[q]);
         }
@@ -2409,13 +2413,15 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
     cpx<T> *S = reinterpret_cast<cpx<T> *>(scratch);
     const int ps = cM | 1;
     T *diag0 = reinterpret_cast<T *>(scratch + LocalBond<T>::al(size_t(cM) * ps * sizeof(cpx<T>)));
+#pragma unroll 1
     for (int e = tid; e < cM * (cM + 1) / 2; e += NT) {
       int p, q;
       tri_entry(e, cM, p, q);
       typename CAcc<T>::type acc = acc_zero<T>();
       const cpx<TS> *bp = gk1 + size_t(p) * nc, *bq = gk1 + size_t(q) * nc;
-#pragma unroll 2
+#pragma unroll 1
       for (int col = 0; col < nc; ++col) {
+        if ((col & 1) == 0) acc_renorm(acc);
         const T l = lR[col < cR ? col : col - cR];
         acc_jfma<T>(acc, cscale(widen(bp[col]), l), cscale(widen(bq[col]), l));
       }
@@ -2453,10 +2459,15 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
   if (sw < 0) {  // go on in the global workspace
     __syncthreads();
     const int nv = colmode ? nc : m;
+#pragma unroll 1
     for (int idx = tid; idx < c * ell; idx += NT) wk.A[idx] = narrow<TS>(A[(idx / ell) * ld + idx % ell]);
+#pragma unroll 1
     for (int idx = tid; idx < nv * ell; idx += NT) wk.T0[idx] = narrow<TS>(T0[(idx / ell) * ld + idx % ell]);
+#pragma unroll 1
     for (int v = tid; v < cL; v += NT) wk.lam3[v] = TS(lL[v]);
+#pragma unroll 1
     for (int u = tid; u < cM; u += NT) wk.lam3[tr.cap + u] = TS(lM[u]);
+#pragma unroll 1
     for (int w = tid; w < cR; w += NT) wk.lam3[2 * tr.cap + w] = TS(lR[w]);
     __syncthreads();
     return res;
@@ -2465,15 +2476,18 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
   // order, rank rule s_j / ||s|| > eps, kept values.  float64 square roots and
   // divisions only where a stored Lambda needs one, in one warp: repeated by
   // every warp, or chained, they would cost more than the products.
+#pragma unroll 1
   for (int j = warp; j < c; j += NT / 32) {
     T part = T(0);
+#pragma unroll 1
     for (int i = lane; i < ell; i += 32) part += cabs2(A[j * ld + i]);
     R s = R(part);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s = s + shfl_xor(s, o);
+#pragma unroll 1
+    for (int o = warp_half(ell); o > 0; o >>= 1) s = s + shfl_xor(s, o);
     if (lane == 0) sq[j] = s;
   }
   __syncthreads();
+#pragma unroll 1
   for (int j = tid; j < c; j += NT) {
     const R x = sq[j];
     int rk = 0;
@@ -2485,12 +2499,14 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
   __syncthreads();
   if (warp == 0) {
     R tot = R(0);
+#pragma unroll 1
     for (int j = lane; j < c; j += 32) tot = tot + ssq[j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tot = tot + shfl_xor(tot, o);
+#pragma unroll 1
+    for (int o = warp_half(c); o > 0; o >>= 1) tot = tot + shfl_xor(tot, o);
     const int mode = tr.trunc_mode;
     const R least = *eps * *eps * tot;
     int bad = c;
+#pragma unroll 1
     for (int j = lane; j < c; j += 32) {
       const R x = ssq[j];
       if (!(isfinite(x) && x > least && x > R(0))) bad = min(bad, j);
@@ -2503,9 +2519,10 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
       rank = tr.cap;
     }
     R kept = R(0);
+#pragma unroll 1
     for (int j = lane; j < rank; j += 32) kept = kept + ssq[j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) kept = kept + shfl_xor(kept, o);
+#pragma unroll 1
+    for (int o = warp_half(c); o > 0; o >>= 1) kept = kept + shfl_xor(kept, o);
     if (lane == 0) {
       reinterpret_cast<R *>(sm.red)[126] = kept;
       reinterpret_cast<R *>(sm.red)[127] = tot;
@@ -2517,6 +2534,7 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
   // the stored Lambda in float64 (a warp or two of its own), the factors of the
   // values (first warps) and of both outer bonds (last warps)
   const R kept = reinterpret_cast<R *>(sm.red)[126];
+#pragma unroll 1
   for (int j = tid; j < rank; j += NT) {
     const R x = ssq[j], y = x / kept, ix2 = R(1) / x;
     isig[j] = T(sqrt(ix2));
@@ -2524,73 +2542,71 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
     w2[j] = T(y);
   }
   if (tid >= 256)
+#pragma unroll 1
     for (int j = tid - 256; j < rank; j += NT - 256) s2[j] = sqrt(double(ssq[j]) / double(kept));
+#pragma unroll 1
   for (int v = NT - 1 - tid; v < cL; v += NT) sL[v] = T(R(1) / R(lL[v]));
   if (int(threadIdx.x) >= 128 && int(threadIdx.x) < 128 + ((cR + 31) & ~31)) {
     const R n2 = sqrt(kept / reinterpret_cast<R *>(sm.red)[127]);  // norm of the kept values relative to all
+#pragma unroll 1
     for (int w = tid - 128; w < cR; w += NT) sR[w] = T(n2 / R(lR[w]));
   }
   __syncthreads();
-  // Gamma_k and Gamma_{k+1}: one side from the vectors, the other recovered
-  // from theta into the scratch; first the sums of local_renormalize, then
-  // both written once, scaled.
+  // Gamma_k and Gamma_{k+1}: one side straight from the vectors ("d": entry t of
+  // vector j), the other recovered from theta into the scratch ("r": row y of
+  // theta times conj(vector j)); first the sums of local_renormalize, then both
+  // written once, scaled.  One copy of the code for both orientations: these
+  // operations wait for instructions more than for arithmetic.
   cpx<T> *rec = reinterpret_cast<cpx<T> *>(scratch);
-  T pk = T(0), pk1 = T(0);
-  auto side0 = [&](int i, int j, cpx<T> u) { return cscale(u, sL[i >> 1]); };
-  auto side1 = [&](int col, cpx<T> u) { return cscale(u, sR[col < cR ? col : col - cR]); };
-  auto add0 = [&](int i, int j, cpx<T> v) {
-    const T l = lL[i >> 1];
-    pk += cabs2(v) * (l * l) * w2[j];
+  const int nv = colmode ? nc : m, din = colmode ? rank : ell, rin = colmode ? nc : rank;
+  auto left = [&](int i) { return i >> 1; };
+  auto right = [&](int i) { return i < cR ? i : i - cR; };
+  const T *const dsc = colmode ? sL : sR, *const rsc = colmode ? sR : sL;
+  const T *const dlm = colmode ? lL : lR, *const rlm = colmode ? lR : lL;
+  auto dindex = [&](int t) { return colmode ? left(t) : right(t); };
+  auto rindex = [&](int y) { return colmode ? right(y) : left(y); };
+  // o-th entry of the direct side in its order in memory, times f
+  auto direct = [&](int o, int &t, int &j, T f) {
+    const int h = o / din, l = o - h * din;
+    t = colmode ? h : l;
+    j = colmode ? l : h;
+    return cscale(A[perm[j] * ld + t], (isig[j] * dsc[dindex(t)]) * f);
   };
-  auto add1 = [&](int j, int col, cpx<T> v) {
-    const T l = lR[col < cR ? col : col - cR];
-    pk1 += cabs2(v) * w2[j] * (l * l);
-  };
-  auto direct0 = [&](int i, int j) { return side0(i, j, cscale(A[perm[j] * ld + i], isig[j])); };
-  auto direct1 = [&](int j, int col) { return side1(col, cscale(A[perm[j] * ld + col], isig[j])); };
-  if (colmode) {
-    for (int o = tid; o < m * rank; o += NT) add0(o / rank, o % rank, direct0(o / rank, o % rank));
-    gemm_exact<T, NT>(
-        rank, nc, m,
-        [&](int j, int i) {
-          const cpx<T> a = A[perm[j] * ld + i];
-          return mkc<T>(a.x, -a.y);
-        },
-        [&](int col, int i) { return T0[col * ld + i]; },
-        [&](int j, int col, cpx<T> v) {
-          v = side1(col, cscale(v, isig2[j]));
-          rec[j * nc + col] = v;
-          add1(j, col, v);
-        });
-  } else {
-    for (int o = tid; o < rank * nc; o += NT) add1(o / nc, o % nc, direct1(o / nc, o % nc));
-    gemm_exact<T, NT>(
-        m, rank, nc, [&](int i, int col) { return T0[i * ld + col]; },
-        [&](int j, int col) {
-          const cpx<T> a = A[perm[j] * ld + col];
-          return mkc<T>(a.x, -a.y);
-        },
-        [&](int i, int j, cpx<T> v) {
-          v = side0(i, j, cscale(v, isig2[j]));
-          rec[i * rank + j] = v;
-          add0(i, j, v);
-        });
+  T pd = T(0), pr = T(0);
+#pragma unroll 1
+  for (int o = tid; o < ell * rank; o += NT) {
+    int t, j;
+    const cpx<T> v = direct(o, t, j, T(1.f));
+    const T l = dlm[dindex(t)];
+    pd += cabs2(v) * (l * l) * w2[j];
   }
-  R nk = R(pk), nk1 = R(pk1);
-  block_sum2_in<R, NT>(nk, nk1, sm.red);
-  if (tid < 32) {
-    const R a = R(1) / sqrt(nk), b = R(1) / sqrt(nk1);
-    __syncwarp();
-    T *f = reinterpret_cast<T *>(sm.red + 100);
-    if (tid == 0) {
-      f[0] = T(a);
-      f[1] = T(b);
+#pragma unroll 1
+  for (int o = tid; o < nv * rank; o += NT) {
+    const int h = o / rin, l_ = o - h * rin, y = colmode ? l_ : h, j = colmode ? h : l_;
+    const cpx<T> *th = T0 + y * ld, *a = A + perm[j] * ld;
+    typename CAcc<T>::type acc = acc_zero<T>();
+#pragma unroll 2
+    for (int t = 0; t < ell; ++t) {
+      if ((t & 1) == 0) acc_renorm(acc);
+      acc_jfma<T>(acc, a[t], th[t]);
     }
+    const int q = rindex(y);
+    const cpx<T> v = cscale(acc_fin<T>(acc), isig2[j] * rsc[q]);
+    rec[o] = v;
+    const T l = rlm[q];
+    pr += cabs2(v) * w2[j] * (l * l);
   }
-  __syncthreads();
-  const T ik = reinterpret_cast<T *>(sm.red + 100)[0], ik1 = reinterpret_cast<T *>(sm.red + 100)[1];
-  for (int o = tid; o < m * rank; o += NT) gk[o] = narrow<TS>(cscale(colmode ? direct0(o / rank, o % rank) : rec[o], ik));
-  for (int o = tid; o < rank * nc; o += NT) gk1[o] = narrow<TS>(cscale(colmode ? rec[o] : direct1(o / nc, o % nc), ik1));
+  norms_in<R, T, NT>(R(pd), R(pr), max(ell, nv) * rank, sm.red, reinterpret_cast<T *>(sm.red + 100));
+  const T fd = reinterpret_cast<T *>(sm.red + 100)[0], fr = reinterpret_cast<T *>(sm.red + 100)[1];
+  cpx<TS> *const gd = colmode ? gk : gk1, *const gr = colmode ? gk1 : gk;
+#pragma unroll 1
+  for (int o = tid; o < ell * rank; o += NT) {
+    int t, j;
+    gd[o] = narrow<TS>(direct(o, t, j, fd));
+  }
+#pragma unroll 1
+  for (int o = tid; o < nv * rank; o += NT) gr[o] = narrow<TS>(cscale(rec[o], fr));
+#pragma unroll 1
   for (int j = tid; j < rank; j += NT) lamM[j] = s2[j];
   if (tid == 0) tr.chi[k + 1] = rank;
   __syncthreads();
@@ -2599,19 +2615,31 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
   return res;
 }
 
-// Work counters of one bond operation (one thread; whole numbers below 2^53,
-// in integer arithmetic to spare the thread a chain of float64 operations).
-template <typename T>
-__device__ void bond_stats(const TrajDev &tr, int cL, int cM, int cR, bool gate, bool lq, int sweeps) {
-  const long long m = 2 * cL, nc = 2 * cR, a = m > nc ? m : nc, b = m > nc ? nc : m;
-  if (lq) atomicAdd(tr.stats + STAT_LQ_OPS, 1.0);
-  atomicAdd(tr.stats + STAT_FLOP_THETA, double(8 * m * cM * nc + (gate ? 128ll * cL * cR : 0ll)));
-  atomicAdd(tr.stats + STAT_FLOP_SVD, double(4 * (4 * a * a * b + 8 * a * b * b + 9 * b * b * b)));
-  atomicAdd(tr.stats + STAT_BOND_OPS, 1.0);
-  atomicAdd(tr.stats + STAT_SWEEPS, double(sweeps));
+// Counters of one bond operation, by the last warp, one counter a lane: one
+// conversion and one atomic, beside whatever the other warps go on with (a
+// single thread's chain of them held every small operation up by 7000 cycles).
+// Whole numbers below 2^53.  cyc: theta, Gram, rotations, update, final; steps.
+template <typename T, int NT>
+__device__ void bond_stats(const TrajDev &tr, int cL, int cM, int cR, bool gate, bool lq, int sweeps,
+                           long long theta, long long rot, long long fin, const long long *cyc) {
+  const int lane = int(threadIdx.x) - (NT - 32);
+  if (lane < 0 || !tr.stats) return;
+  const long long m = 2 * cL, nc = 2 * cR, a = m > nc ? m : nc, b = m > nc ? nc : m, eb = sizeof(cpx<T>);
+  long long v = 0;
+  if (lane == STAT_FLOP_THETA) v = 8 * m * cM * nc + (gate ? 128ll * cL * cR : 0ll);
+  if (lane == STAT_FLOP_SVD) v = 4 * (4 * a * a * b + 8 * a * b * b + 9 * b * b * b);
+  if (lane == STAT_BOND_OPS) v = 1;
+  if (lane == STAT_SWEEPS) v = sweeps;
   // read the Gamma pair + Lambdas, write the new Gamma pair
-  const long long eb = sizeof(cpx<T>);
-  atomicAdd(tr.stats + STAT_BYTES, double(eb * 4 * (1ll * cL * cM + 1ll * cM * cR) + 8ll * (cL + cM + cR)));
+  if (lane == STAT_BYTES) v = eb * 4 * (1ll * cL * cM + 1ll * cM * cR) + 8ll * (cL + cM + cR);
+  if (lane == STAT_LQ_OPS) v = lq;
+  if (lane == STAT_CYC_THETA) v = theta;
+  if (lane == STAT_CYC_ROT) v = rot;
+  if (lane == STAT_CYC_FINAL) v = fin;
+  if (lane == STAT_CYC_GRAM) v = cyc[0];
+  if (lane == STAT_CYC_UPDATE) v = cyc[2];
+  if (lane == STAT_BLOCK_STEPS) v = cyc[3];
+  if (v) atomicAdd(tr.stats + lane, double(v));
 }
 
 // One bond operation on (k, k+1): gate != nullptr -> apply_unitary2, else local_refactor.
@@ -2702,24 +2730,15 @@ __device__ void bond_op(const TrajDev &tr, int k, int cL, int cM, int cR, const 
         atomicAdd(tr.stats + (lq ? STAT_NONCONV_LQ : STAT_NONCONV_DIRECT), double(c));
       }
     }
-    if (tr.stats) bond_stats<T>(tr, cL, cM, cR, gate != nullptr, lq, sw < 0 ? max_sweeps : sw);
   }
   if (!loc.done) finalize_bond<T, NT, W>(tr, k, gk, gk1, lamL, lamM, lamR, cL, cR, colmode, ell, c, wk, sm);
   if (sm.tc_fail) {  // a tensor-core wait gave up: the op's result is not trustworthy
     if (threadIdx.x == 0) atomicOr(tr.status, ST_BAD_INSTR);
     sm.tc_fail = false;
   }
-  if (threadIdx.x == 0 && tr.stats) {
-    // in shared memory the whole SVD counts as rotations
-    atomicAdd(tr.stats + STAT_CYC_THETA, double(local ? lcyc[0] : c1 - c0));
-    atomicAdd(tr.stats + STAT_CYC_ROT, double(cyc[1] + lcyc[1]));
-    atomicAdd(tr.stats + STAT_CYC_FINAL, double(loc.done ? lcyc[2] : clock64() - c2));
-    if (!loc.done) {
-      atomicAdd(tr.stats + STAT_CYC_GRAM, double(cyc[0]));
-      atomicAdd(tr.stats + STAT_CYC_UPDATE, double(cyc[2]));
-      atomicAdd(tr.stats + STAT_BLOCK_STEPS, double(cyc[3]));
-    }
-  }
+  // in shared memory the whole SVD counts as rotations
+  bond_stats<T, NT>(tr, cL, cM, cR, gate != nullptr, lq, sw < 0 ? max_sweeps : sw, local ? lcyc[0] : c1 - c0,
+                    cyc[1] + lcyc[1], loc.done ? lcyc[2] : clock64() - c2, cyc);
 }
 
 // Whether bond_team takes the bond, in the modes that have a float bulk and
@@ -2896,7 +2915,6 @@ __device__ __noinline__ void bond_team(const Team &tm, const TrajDev &tr, int k,
         atomicAdd(tr.stats + (lq ? STAT_NONCONV_LQ : STAT_NONCONV_DIRECT), double(c));
       }
     }
-    if (tr.stats) bond_stats<T>(tr, cL, cM, cR, gate != nullptr, lq, sw < 0 ? max_sweeps : sw);
   }
   // process_svd and the Gamma rebuild (finalize_bond); every member sorts for itself
   for (int j = tm.rank * (NT / 32) + warp; j < c; j += tm.size * (NT / 32)) {
@@ -3048,14 +3066,8 @@ __device__ __noinline__ void bond_team(const Team &tm, const TrajDev &tr, int k,
     if (tid == 0) atomicOr(tr.status, ST_BAD_INSTR);
     sm.tc_fail = false;
   }
-  if (tid == 0 && tm.rank == 0 && tr.stats) {
-    atomicAdd(tr.stats + STAT_CYC_THETA, double(c1 - c0));
-    atomicAdd(tr.stats + STAT_CYC_GRAM, double(cyc[0]));
-    atomicAdd(tr.stats + STAT_CYC_ROT, double(cyc[1]));
-    atomicAdd(tr.stats + STAT_CYC_UPDATE, double(cyc[2]));
-    atomicAdd(tr.stats + STAT_CYC_FINAL, double(clock64() - c2));
-    atomicAdd(tr.stats + STAT_BLOCK_STEPS, double(cyc[3]));
-  }
+  if (tm.rank == 0)
+    bond_stats<T, NT>(tr, cL, cM, cR, gate != nullptr, lq, sw < 0 ? max_sweeps : sw, c1 - c0, cyc[1], clock64() - c2, cyc);
   sm_.take(sm);
   tm.sync();
 }

@@ -121,6 +121,10 @@ __device__ __forceinline__ float block_max(float v, double *red) {
   return __uint_as_float(m);
 }
 
+// Half of the smallest power of two that is at least n, within a warp: the
+// first distance of a butterfly sum whose lanes from n on hold zeros.
+__device__ __forceinline__ int warp_half(int n) { return n > 16 ? 16 : n > 1 ? 1 << (31 - __clz(n - 1)) : 0; }
+
 // Upper-triangle entry e -> (p, q), p <= q < c, row by row.
 __device__ __forceinline__ void tri_entry(int e, int c, int &p, int &q) {
   const float b = float(2 * c + 1);
@@ -133,31 +137,18 @@ __device__ __forceinline__ void tri_entry(int e, int c, int &p, int &q) {
   q = r + (e - start(r));
 }
 
-// C[x][y] = sum_k P(x, k) Q(y, k), one output a thread, exactly M N K terms.
-// Faster than the 64 x 64 tiles of gemm_nt while the outputs are at most a
-// few per thread: a 16 x 16 x 16 double-float product is one pass of 16 terms
-// here and a whole padded tile there.
-template <typename T, int NT, class FP, class FQ, class FE>
-__device__ void gemm_exact(int M, int N, int K, FP P, FQ Q, FE E) {
-  for (int o = threadIdx.x; o < M * N; o += NT) {
-    const int x = o / N, y = o - x * N;
-    typename CAcc<T>::type acc = acc_zero<T>();
-#pragma unroll 4
-    for (int k = 0; k < K; ++k) {
-      if ((k & 3) == 0) acc_renorm(acc);
-      acc_fma<T>(acc, P(x, k), Q(y, k));
-    }
-    E(x, y, acc_fin<T>(acc));
-  }
-}
-
-// The same with the terms k < from(x, y) of an output left out (a triangular factor).
+// C[x][y] = sum_k P(x, k) Q(y, k) over from(x, y) <= k < K (a triangular
+// factor), one output a thread, exactly as many terms as there are.  Faster
+// than the 64 x 64 tiles of gemm_nt while the outputs are at most a few per
+// thread: a 16 x 16 x 16 double-float product is one pass of 16 terms here and
+// a whole padded tile there.
 template <typename T, int NT, class FK, class FP, class FQ, class FE>
 __device__ void gemm_exact_from(int M, int N, FK from, int K, FP P, FQ Q, FE E) {
+#pragma unroll 1
   for (int o = threadIdx.x; o < M * N; o += NT) {
     const int x = o / N, y = o - x * N;
     typename CAcc<T>::type acc = acc_zero<T>();
-#pragma unroll 2
+#pragma unroll 1
     for (int k = from(x, y); k < K; ++k) acc_fma<T>(acc, P(x, k), Q(y, k));
     E(x, y, acc_fin<T>(acc));
   }
@@ -183,11 +174,13 @@ __device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<flo
   const int active = min(NT, ((np * LG + 31) >> 5) << 5);  // threads that own a pair (whole warps)
   const float tol2 = tol * tol, done2 = done * done;
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+#pragma unroll 1
     for (int j = warp; j < c; j += NT / 32) {
       float s = 0.f;
+#pragma unroll 1
       for (int i = lane; i < ell; i += 32) s += cabs2(As[j * pa + i]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+#pragma unroll 1
+      for (int o = warp_half(ell); o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       if (lane == 0) nrm[j] = s;
     }
     __syncthreads();
@@ -316,11 +309,12 @@ __device__ __noinline__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S
   S = as_shared(S);
   Q = as_shared(Q);
   dg = as_shared(dg);
-  constexpr int OPT = NT >= 512 ? 8 : 8;  // outputs per thread: c <= 64 at 512 threads, c <= 32 at 128
+  cpx<float> *const tmp = reinterpret_cast<cpx<float> *>(Q);  // c x c floats, until Q is written
   const int tid = threadIdx.x;
   const int ntri = c * (c + 1) / 2;
   for (int it = 0;; ++it) {
     float smax = 0.f, dmax = 0.f;
+#pragma unroll 1
     for (int e = tid; e < ntri; e += NT) {
       int p, q;
       tri_entry(e, c, p, q);
@@ -328,7 +322,7 @@ __device__ __noinline__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S
       tacc ax, ay;
       ax.mid = ax.lo = ay.hi = ay.mid = ay.lo = 0.f;
       ax.hi = p == q ? -1.f : 0.f;
-#pragma unroll 2
+#pragma unroll 1
       for (int k = 0; k < c; ++k) {
         const cpx<float> x = vp[k], y = vq[k];
         tacc_add_prod(ax, x.x, y.x);
@@ -349,66 +343,53 @@ __device__ __noinline__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S
     dmax = block_max<NT>(dmax, red);
     if (smax <= kOffMax && dmax <= kDiagMax) break;
     if (!(smax <= 0.5f && dmax <= 0.5f) || it >= 6) return false;
-    cpx<float> out[OPT];
-#pragma unroll
-    for (int u = 0; u < OPT; ++u) {
-      const int o = tid + u * NT;
-      if (o < c * c) {
-        const int y = o / c, r = o - y * c;
-        cpx<float> a = czero<float>();
-        for (int k = 0; k < c; ++k) {
-          const cpx<dd> s = S[k * ps + y];
-          a = cfma(Vs[k * pv + r], mkc<float>(s.x.hi, s.y.hi), a);
-        }
-        const cpx<float> v = Vs[y * pv + r];
-        out[u] = mkc<float>(fmaf(-0.5f, a.x, v.x), fmaf(-0.5f, a.y, v.y));
+#pragma unroll 1
+    for (int o = tid; o < c * c; o += NT) {
+      const int y = o / c, r = o - y * c;
+      cpx<float> a = czero<float>();
+#pragma unroll 1
+      for (int k = 0; k < c; ++k) {
+        const cpx<dd> s = S[k * ps + y];
+        a = cfma(Vs[k * pv + r], mkc<float>(s.x.hi, s.y.hi), a);
       }
+      const cpx<float> v = Vs[y * pv + r];
+      tmp[o] = mkc<float>(fmaf(-0.5f, a.x, v.x), fmaf(-0.5f, a.y, v.y));
     }
     __syncthreads();
-#pragma unroll
-    for (int u = 0; u < OPT; ++u) {
-      const int o = tid + u * NT;
-      if (o < c * c) Vs[(o / c) * pv + o % c] = out[u];
-    }
+#pragma unroll 1
+    for (int o = tid; o < c * c; o += NT) Vs[(o / c) * pv + o % c] = tmp[o];
     __syncthreads();
   }
   // W in place of S (the square in float)
   for (int k = tid; k < c; k += NT) dg[k] = dg_minus1(S[k * ps + k].x);
   __syncthreads();
-  {
-    cpx<float> sq[OPT];
-#pragma unroll
-    for (int u = 0; u < OPT; ++u) {
-      const int o = tid + u * NT;
-      if (o < c * c) {
-        const int y = o / c, x = o - y * c;
-        cpx<float> a = czero<float>();
-        for (int k = 0; k < c; ++k) {
-          if (k == x || k == y) continue;
-          const cpx<dd> s = S[x * ps + k], t = S[k * ps + y];
-          const float g = 1.f + dg[k].hi;
-          a = cfma(mkc<float>(s.x.hi * (g * g), s.y.hi * (g * g)), mkc<float>(t.x.hi, t.y.hi), a);
-        }
-        const float g = (1.f + dg[x].hi) * (1.f + dg[y].hi);
-        sq[u] = mkc<float>(a.x * g, a.y * g);
-      }
+#pragma unroll 1
+  for (int o = tid; o < c * c; o += NT) {
+    const int y = o / c, x = o - y * c;
+    cpx<float> a = czero<float>();
+#pragma unroll 1
+    for (int k = 0; k < c; ++k) {
+      if (k == x || k == y) continue;
+      const cpx<dd> s = S[x * ps + k], t = S[k * ps + y];
+      const float g = 1.f + dg[k].hi;
+      a = cfma(mkc<float>(s.x.hi * (g * g), s.y.hi * (g * g)), mkc<float>(t.x.hi, t.y.hi), a);
     }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < OPT; ++u) {
-      const int o = tid + u * NT;
-      if (o < c * c) {
-        const int y = o / c, x = o - y * c;
-        S[x * ps + y] = unit_entry(x == y, S[x * ps + y], dg[x], dg[y], sq[u]);
-      }
-    }
-    __syncthreads();
+    const float g = (1.f + dg[x].hi) * (1.f + dg[y].hi);
+    tmp[o] = mkc<float>(a.x * g, a.y * g);
   }
+  __syncthreads();
+#pragma unroll 1
+  for (int o = tid; o < c * c; o += NT) {
+    const int y = o / c, x = o - y * c;
+    S[x * ps + y] = unit_entry(x == y, S[x * ps + y], dg[x], dg[y], tmp[o]);
+  }
+  __syncthreads();
+#pragma unroll 1
   for (int o = tid; o < c * c; o += NT) {
     const int y = o / c, r = o - y * c;
     dacc ax, ay;
     ax.hi = ax.lo = ay.hi = ay.lo = 0.f;
-#pragma unroll 2
+#pragma unroll 1
     for (int k = 0; k < c; ++k) {
       const cpx<float> v = Vs[k * pv + r];
       const cpx<dd> w = S[k * ps + y];
@@ -427,6 +408,7 @@ __device__ __noinline__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S
 // 32 rows [i0, i0 + 32) of the vectors A[j * ld + i] as stage[r * pt + j].
 template <typename T, int NT>
 __device__ __forceinline__ void stage_rows(const cpx<T> *A, int ld, int ell, int c, int i0, cpx<T> *stage, int pt) {
+#pragma unroll 1
   for (int idx = threadIdx.x; idx < 32 * c; idx += NT) {
     const int r = idx & 31, p = idx >> 5;
     stage[r * pt + p] = i0 + r < ell ? A[size_t(p) * ld + i0 + r] : czero<T>();
@@ -440,13 +422,14 @@ __device__ void apply_unitary(cpx<T> *A, int ld, int ell, int c, const cpx<T> *Q
     stage_rows<T, NT>(A, ld, ell, c, i0, stage, pt);
     __syncthreads();
     const int rows = min(32, ell - i0);
+#pragma unroll 1
     for (int o = threadIdx.x; o < 32 * c; o += NT) {
       const int r = o & 31, y = o >> 5;
       if (r < rows) {
         typename CAcc<T>::type acc = acc_zero<T>();
-#pragma unroll 4
+#pragma unroll 2
         for (int p = 0; p < c; ++p) {
-          if ((p & 3) == 0) acc_renorm(acc);
+          if ((p & 1) == 0) acc_renorm(acc);
           acc_fma<T>(acc, stage[r * pt + p], Q[p * pq + y]);
         }
         A[size_t(y) * ld + i0 + r] = acc_fin<T>(acc);
@@ -463,6 +446,7 @@ template <typename T, int NT>
 __device__ void apply_small(cpx<T> *A, int ld, int ell, int c, const cpx<float> *Ks, int pk, cpx<float> *stage,
                             int pt) {
   for (int i0 = 0; i0 < ell; i0 += 32) {
+#pragma unroll 1
     for (int idx = threadIdx.x; idx < 32 * c; idx += NT) {
       const int r = idx & 31, p = idx >> 5;
       cpx<float> v = czero<float>();
@@ -474,10 +458,12 @@ __device__ void apply_small(cpx<T> *A, int ld, int ell, int c, const cpx<float> 
     }
     __syncthreads();
     const int rows = min(32, ell - i0);
+#pragma unroll 1
     for (int o = threadIdx.x; o < 32 * c; o += NT) {
       const int r = o & 31, y = o >> 5;
       if (r < rows) {
         cpx<float> a = czero<float>();
+#pragma unroll 2
         for (int p = 0; p < c; ++p)
           if (p != y) a = cfma(stage[r * pt + p], Ks[y * pk + p], a);
         cpx<T> &x = A[size_t(y) * ld + i0 + r];
@@ -492,40 +478,33 @@ __device__ void apply_small(cpx<T> *A, int ld, int ell, int c, const cpx<float> 
 // G = A^H A (upper triangle G[p * pg + q], p <= q) in the working precision.
 template <typename T, int NT>
 __device__ void gram_local(const cpx<T> *A, int ld, int ell, int c, cpx<T> *G, int pg, cpx<T> *stage, int pt) {
-  constexpr int PER = 5;  // c (c + 1) / 2 entries: c <= 64 at 512 threads, c <= 32 at 128
+  // (one entry a thread up to c = 31 at 512 threads; beyond, the rows are staged
+  // again for every further group of entries: cheaper than the code of several
+  // sums a thread, which all sizes would fetch)
   const int ntri = c * (c + 1) / 2;
-  typename CAcc<T>::type acc[PER];
-#pragma unroll
-  for (int u = 0; u < PER; ++u) acc[u] = acc_zero<T>();
-  for (int i0 = 0; i0 < ell; i0 += 32) {
-    stage_rows<T, NT>(A, ld, ell, c, i0, stage, pt);
-    __syncthreads();
-    const int rows = min(32, ell - i0);
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-      const int e = threadIdx.x + u * NT;
-      if (e < ntri) {
-        int p, q;
-        tri_entry(e, c, p, q);
-        typename CAcc<T>::type a = acc[u];
-#pragma unroll 4
-        for (int r = 0; r < rows; ++r) {
-          if ((r & 3) == 0) acc_renorm(a);
-          acc_jfma<T>(a, stage[r * pt + p], stage[r * pt + q]);
-        }
-        acc[u] = a;
+#pragma unroll 1
+  for (int e0 = 0; e0 < ntri; e0 += NT) {
+    const int e = e0 + threadIdx.x;
+    int p = 0, q = 0;
+    if (e < ntri) tri_entry(e, c, p, q);
+    typename CAcc<T>::type acc = acc_zero<T>();
+#pragma unroll 1
+    for (int i0 = 0; i0 < ell; i0 += 32) {
+      if (e0 == 0 || ell > 32) {
+        stage_rows<T, NT>(A, ld, ell, c, i0, stage, pt);
+        __syncthreads();
       }
+      const int rows = min(32, ell - i0);
+      if (e < ntri) {
+#pragma unroll 2
+        for (int r = 0; r < rows; ++r) {
+          if ((r & 1) == 0) acc_renorm(acc);
+          acc_jfma<T>(acc, stage[r * pt + p], stage[r * pt + q]);
+        }
+      }
+      if (ell > 32) __syncthreads();
     }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int u = 0; u < PER; ++u) {
-    const int e = threadIdx.x + u * NT;
-    if (e < ntri) {
-      int p, q;
-      tri_entry(e, c, p, q);
-      G[p * pg + q] = acc_fin<T>(acc[u]);
-    }
+    if (e < ntri) G[p * pg + q] = acc_fin<T>(acc);
   }
   __syncthreads();
 }
@@ -579,6 +558,7 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
   at += L::first_bytes(ell, c);
   const float tolf = 4.f * sqrtf(float(ell)) * Eps<float>::v;
   auto load = [&]() {
+#pragma unroll 1
     for (int idx = tid; idx < c * ell; idx += NT) {
       const int j = idx / ell, i = idx - j * ell;
       const cpx<T> x = A[size_t(j) * ld + i];
@@ -614,10 +594,14 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
     constexpr float kFloatApply = std::is_same<T, double>::value ? 1e-9f : 1e-7f;
     constexpr int kMaxStages = 3, kMaxSteps = 10;
     int sweeps = 0, stages = 0;
-    bool bulk = true;  // a float stage is due
-    for (int step = 0; step < kMaxSteps; ++step) {
+    // what is due: a float stage, a product with the unitary factor of V (or
+    // of I + K), a small correction; one copy of each in the loop
+    bool bulk = true, small_step = false, last = false;
+#pragma unroll 1
+    for (int step = 0;; ++step) {
       if (bulk) {
         load();
+#pragma unroll 1
         for (int idx = tid; idx < c * c; idx += NT) {
           const int y = idx / c, r = idx - y * c;
           Vs[y * pc + r] = mkc<float>(y == r ? 1.f : 0.f, 0.f);
@@ -629,10 +613,16 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
                                     1e-4f, min(max_sweeps, 20));
         sweeps += sw < 0 ? min(max_sweeps, 20) : sw;
         ++stages;
-        if (!unitarise<T, NT>(Vs, pc, c, S, pc, Q, pc, dg, red)) return -1;
-        apply_unitary<T, NT>(A, ld, ell + tail, c, Q, pc, stage, pc);
         bulk = false;
       }
+      if (small_step) {
+        apply_small<T, NT>(A, ld, ell + tail, c, Vs, pc, reinterpret_cast<cpx<float> *>(stage), pc);
+      } else {
+        if (!unitarise<T, NT>(Vs, pc, c, S, pc, Q, pc, dg, red)) return -1;
+        apply_unitary<T, NT>(A, ld, ell + tail, c, Q, pc, stage, pc);
+      }
+      if (last) return sweeps + 1;
+      if (step == kMaxSteps) return -1;
       gram_local<T, NT>(A, ld, ell, c, G, pc, stage, pc);
       float fro = 0.f;
       for (int j = 0; j < c; ++j) fro += lead(G[j * pc + j].x);
@@ -643,6 +633,7 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
       // with them a trajectory's error against float64 is 2-10 times smaller.
       float rmax = 0.f, kmax = 0.f, small = 0.f;
       const float least = tol < 1e-10f ? 0.03125f * tol : tol;
+#pragma unroll 1
       for (int e = tid; e < c * (c + 1) / 2; e += NT) {
         int p, q;
         tri_entry(e, c, p, q);
@@ -681,28 +672,21 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
       small = block_max<NT>(small, red);
       if (!(rmax < 2.f)) return -1;  // not a number
       if (rmax <= tol) {
-        if (small > 0.f) apply_small<T, NT>(A, ld, ell + tail, c, Vs, pc, reinterpret_cast<cpx<float> *>(stage), pc);
-        return sweeps + 1;
+        if (!(small > 0.f)) return sweeps + 1;
+        small_step = last = true;
+        continue;
       }
       ++sweeps;
       // What is left after this step is of the order of the square: r r' between
       // vectors of different size (whose angles t are smaller than r), r t
       // between neighbours.
       const float far = fmaxf(rmax, kmax);
-      const bool last = rmax * far * 8.f <= tol;
-      if (far <= kFloatApply) {
-        apply_small<T, NT>(A, ld, ell + tail, c, Vs, pc, reinterpret_cast<cpx<float> *>(stage), pc);
-      } else if (rmax > 1e-3f && kmax > 0.3f && stages < kMaxStages) {
-        bulk = true;  // far from converged: vectors that the float stage had left alone
-        __syncthreads();
-        continue;
-      } else {
-        if (!unitarise<T, NT>(Vs, pc, c, S, pc, Q, pc, dg, red)) return -1;
-        apply_unitary<T, NT>(A, ld, ell + tail, c, Q, pc, stage, pc);
-      }
-      if (last) return sweeps + 1;
+      small_step = far <= kFloatApply;
+      // far from converged: vectors that the float stage had left alone
+      bulk = !small_step && rmax > 1e-3f && kmax > 0.3f && stages < kMaxStages;
+      last = !bulk && rmax * far * 8.f <= tol;
+      if (bulk) __syncthreads();
     }
-    return -1;
   }
 }
 
@@ -720,6 +704,7 @@ __device__ __noinline__ int svd_local_global(cpx<T> *A, int ell, int c, int max_
 // when a pivot falls below `rel` times its original diagonal.
 template <typename T, int NT>
 __device__ bool cholesky_local(cpx<T> *S, int ps, int n, float rel, T *diag0) {
+#pragma unroll 1
   for (int i = threadIdx.x; i < n; i += NT) diag0[i] = S[i * ps + i].x;
   __syncthreads();
   for (int k = 0; k < n; ++k) {
@@ -728,11 +713,13 @@ __device__ bool cholesky_local(cpx<T> *S, int ps, int n, float rel, T *diag0) {
     __syncthreads();
     if (threadIdx.x < 32 || int(threadIdx.x & ~31u) < n - k - 1) {  // whole warps that hold a row below the pivot
       const T l = sqrt(d), il = T(1) / l;
+#pragma unroll 1
       for (int i = k + 1 + threadIdx.x; i < n; i += NT) S[i * ps + k] = cscale(S[i * ps + k], il);
       if (threadIdx.x == 0) S[k * ps + k] = mkc<T>(l, T(0));
     }
     __syncthreads();
     const int rem = n - k - 1;
+#pragma unroll 1
     for (int idx = threadIdx.x; idx < rem * rem; idx += NT) {
       const int i = k + 1 + idx / rem, j = k + 1 + idx % rem;
       if (j > i) continue;
@@ -755,26 +742,26 @@ __device__ bool cholesky_local(cpx<T> *S, int ps, int n, float rel, T *diag0) {
 template <typename T>
 struct LocalBond {
   static constexpr int MAXM = 64;
-  size_t theta, vec, svd, lam, vals, total;
+  unsigned theta, vec, svd, lam, vals, total;  // (below 2^20: at most 64 x 64)
   int c, ell;
-  __host__ __device__ static size_t al(size_t x) { return (x + 15) & ~size_t(15); }
-  __host__ __device__ static size_t most(size_t a, size_t b) { return a > b ? a : b; }
+  __host__ __device__ static unsigned al(unsigned x) { return (x + 15) & ~15u; }
+  __host__ __device__ static unsigned most(unsigned a, unsigned b) { return a > b ? a : b; }
   __host__ __device__ bool plan(int cL, int cM, int cR, bool lq, size_t room, int nt) {
     const int m = 2 * cL, nc = 2 * cR, mn = m < nc ? m : nc;
     if (m > MAXM || nc > MAXM || cM > MAXM) return false;
-    const size_t e = sizeof(cpx<T>);
+    const unsigned e = sizeof(cpx<T>);
     // vectors and their length; theta with the same pitch.  (LQ: cM vectors of
     // length m, theta as columns; the general path takes what LQ declines.)
     c = lq ? cM : mn;
     ell = lq ? m : (m < nc ? nc : m);
     if (c > LocalSvd<T>::max_c(nt)) return false;
-    theta = al(size_t(lq ? nc : mn) * (ell | 1) * e);
-    vec = al(size_t(c) * (ell | 1) * e);
-    svd = LocalSvd<T>::bytes(ell, c);
-    svd = most(svd, al(size_t(cM) * (cM | 1) * e) + al(size_t(cM) * sizeof(T)));    // S and its diagonal
-    svd = most(svd, al(size_t(c) * (lq ? nc : mn) * e));                            // the recovered side
-    lam = al(size_t(2) * (cL + cM + cR) * sizeof(T));
-    vals = al(size_t(mn) * (3 * sizeof(double) + 3 * sizeof(T) + sizeof(int))) + 128;
+    theta = al((lq ? nc : mn) * (ell | 1) * e);
+    vec = al(c * (ell | 1) * e);
+    svd = unsigned(LocalSvd<T>::bytes(ell, c));
+    svd = most(svd, al(cM * (cM | 1) * e) + al(cM * unsigned(sizeof(T))));  // S and its diagonal
+    svd = most(svd, al(c * (lq ? nc : mn) * e));                            // the recovered side
+    lam = al(2 * (cL + cM + cR) * unsigned(sizeof(T)));
+    vals = al(mn * unsigned(3 * sizeof(double) + 3 * sizeof(T) + sizeof(int))) + 128;
     total = theta + vec + svd + lam + vals;
     return total <= room;
   }
@@ -812,6 +799,41 @@ __device__ __forceinline__ void block_sum2_in(R &a, R &b, double *red) {
   __syncthreads();
   a = r[2 * (NT / 32)];
   b = r[2 * (NT / 32) + 1];
+}
+// f[0], f[1] = 1 / sqrt of the block's sums of a and b (in order: the same bits
+// for the same block).  terms: threads from this one on hold zeros; up to a
+// warp's worth need no second stage.
+template <typename R, typename T, int NT>
+__device__ __forceinline__ void norms_in(R a, R b, int terms, double *red, T *f) {
+  R *r = reinterpret_cast<R *>(red);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll 1
+  for (int o = warp_half(terms); o > 0; o >>= 1) {
+    a = a + shfl_xor(a, o);
+    b = b + shfl_xor(b, o);
+  }
+  if (terms > 32) {
+    __syncthreads();
+    if (lane == 0) {
+      r[warp] = a;
+      r[NT / 32 + warp] = b;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      a = lane < NT / 32 ? r[lane] : R(0);
+      b = lane < NT / 32 ? r[NT / 32 + lane] : R(0);
+#pragma unroll 1
+      for (int o = NT / 64; o > 0; o >>= 1) {
+        a = a + shfl_xor(a, o);
+        b = b + shfl_xor(b, o);
+      }
+    }
+  }
+  if (warp == 0) {
+    const R x = R(1) / sqrt(lane & 1 ? b : a);
+    if (lane < 2) f[lane] = T(x);
+  }
+  __syncthreads();
 }
 
 // What bond_local leaves behind.
