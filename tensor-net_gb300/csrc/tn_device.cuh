@@ -1,8 +1,8 @@
 // tn_device.cuh -- device side of the Gamma-Lambda MPS trajectory engine (sm_103a).
 //
-// One CTA owns one trajectory for the whole of a launch and executes that
-// trajectory's instruction list (gates, refactors, measurements, entropy reads)
-// in order.  Trajectory state stays in HBM between launches:
+// A CTA (or a cluster of them, for few trajectories with wide bonds) takes work
+// items and executes their instruction lists (gates, refactors, measurements,
+// entropy reads) in order.  Trajectory state stays in HBM between launches:
 //   gamma : n slots of 2*cap*cap complex<T>; site k holds Gamma_k as a dense
 //           row-major (chi_{k-1}, 2, chi_k) array at the slot start (the
 //           reference layout, tensor-net/lib/mps.rs:344-349);

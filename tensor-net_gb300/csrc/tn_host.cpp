@@ -310,7 +310,7 @@ int mps_run(tn_mps *m, const std::vector<Instr> &prog, const std::vector<double>
   }
   // Bonds wider than 32 have more than 64 vectors, which a cluster shares: one
   // SM of 152 would do them alone otherwise (a chi = 256 gate in double-float:
-  // 930 ms there, 75 ms on eight).  Narrower ones run on one CTA either way.
+  // 920 ms there, 65 ms on eight).  Narrower ones run on one CTA either way.
   int cluster = 0;
   if (m->prec != TN_PREC_F64 && L.ws_team && std::min<uint32_t>(m->chi_hint, m->cap) > 32) {
     if (L.clusters < 0) L.clusters = run_clusters(m->prec, L.sortP, kTeamCtas);

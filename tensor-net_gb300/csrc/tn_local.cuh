@@ -14,8 +14,8 @@
 //     to its rounding, so the float angles cost no accuracy;
 //  3. refinement: the Gram matrix of A in the working precision gives every
 //     remaining rotation at once, tan(theta) = t for each pair as in a Jacobi
-//     rotation; I + K with K_qp = -t e, K_pq = t conj(e) is made unitary by the
-//     same step and applied.  The off-diagonals fall quadratically; two steps
+//     rotation; I + K with K_qp = -t e, K_pq = t conj(e) is made unitary (by a
+//     short series while t is small, unitary_step; else as in 2) and applied.  The off-diagonals fall quadratically; two steps
 //     usually reach the working precision's threshold.
 //
 // The sweeps of 1 are the many, cheap ones; the working precision pays for two
