@@ -24,6 +24,7 @@
 
 #include "tn_dd.cuh"
 #include "tn_internal.h"
+#include "tn_order.h"
 #include "tn_tc.cuh"
 
 namespace tn {
@@ -925,10 +926,10 @@ __device__ __forceinline__ float scale2f(float x, int e) {
   return __fmul_rn(x, pow2f(e));
 }
 // Exponent e with |v| < 2^e for every |v| <= m (m the largest magnitude of a
-// row or column; 0 when m == 0).
+// row or column; 0 when m == 0 or not finite).
 __device__ __forceinline__ int oz_exponent(float m) {
   int e = 0;
-  if (m > 0.f) frexpf(m, &e);
+  if (m > 0.f && isfinite(m)) frexpf(m, &e);
   return e;
 }
 // ND signed BITS-bit digits of the double-float x = hi + lo relative to 2^E
@@ -1656,7 +1657,7 @@ __device__ __forceinline__ int jacobi_svd_body(cpx<T> *__restrict__ A, int ell, 
       double *key = reinterpret_cast<double *>(sm.r0);
       int *kidx = reinterpret_cast<int *>(key + P);
       for (int j = threadIdx.x; j < P; j += NT) {
-        key[j] = j < c ? nrm[j] : -1.0;
+        key[j] = j < c ? order_key(nrm[j]) : kOrderPad;
         kidx[j] = j;
       }
       __syncthreads();
@@ -1896,7 +1897,8 @@ __device__ __noinline__ int jacobi_svd(cpx<T> *__restrict__ A, int ell, int c, i
 // =======================================================================
 template <typename T, int NT, int W>
 __device__ void bitonic_desc(double *key, int *idx, int P) {
-  // order: key descending, index ascending on ties
+  // order: key descending, index ascending on ties.  Keys are order_key's, padding kOrderPad: without NaN the
+  // places before the padding hold a permutation of the listed indices.
   for (int k = 2; k <= P; k <<= 1) {
     for (int j = k >> 1; j > 0; j >>= 1) {
       for (int t = threadIdx.x; t < P; t += NT) {
@@ -2102,7 +2104,7 @@ __device__ __noinline__ void finalize_bond(const TrajDev &tr, int k, cpx<T> *__r
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) {
-      key[j] = (j < c) ? sqrt(acc) : -1.0;
+      key[j] = (j < c) ? order_key(sqrt(acc)) : kOrderPad;
       pidx[j] = j;
     }
   }
@@ -2110,7 +2112,7 @@ __device__ __noinline__ void finalize_bond(const TrajDev &tr, int k, cpx<T> *__r
   bitonic_desc<T, NT, W>(key, pidx, P);
   // norm of all singular values, normalise
   double part = 0.0;
-  for (int j = threadIdx.x; j < c; j += NT) part += key[j] * key[j];
+  for (int j = threadIdx.x; j < c; j += NT) part += order_square(key[j]);
   const double norm1 = sqrt(block_sum<NT>(part, sm.red));
   // rank rule on s/||s||
   int mode = tr.trunc_mode;
@@ -2489,11 +2491,8 @@ __device__ __noinline__ LocalResult bond_local(const TrajDev &tr, int k, int cL,
   __syncthreads();
 #pragma unroll 1
   for (int j = tid; j < c; j += NT) {
-    const R x = sq[j];
-    int rk = 0;
-    for (int i = 0; i < c; ++i) rk += (sq[i] > x || (sq[i] == x && i < j)) ? 1 : 0;
-    rk = min(rk, c - 1);
-    ssq[rk] = x;
+    const int rk = order_rank(sq, c, j);
+    ssq[rk] = sq[j];
     perm[rk] = j;
   }
   __syncthreads();
@@ -2932,13 +2931,13 @@ __device__ __noinline__ void bond_team(const Team &tm, const TrajDev &tr, int k,
   double *key = reinterpret_cast<double *>(sm.r0);
   int *pidx = reinterpret_cast<int *>(key + P);
   for (int j = tid; j < P; j += NT) {
-    key[j] = j < c ? sqrt(wk.sig[j]) : -1.0;
+    key[j] = j < c ? order_key(sqrt(wk.sig[j])) : kOrderPad;
     pidx[j] = j;
   }
   __syncthreads();
   bitonic_desc<T, NT, W>(key, pidx, P);
   double part = 0.0;
-  for (int j = tid; j < c; j += NT) part += key[j] * key[j];
+  for (int j = tid; j < c; j += NT) part += order_square(key[j]);
   const double norm1 = sqrt(block_sum<NT>(part, sm.red));
   const int mode = tr.trunc_mode;
   const double eps = fmax((mode == 2 || mode == 3) ? fabs(tr.cutoff) : 2.220446049250313e-16, rank_floor<T>(ell));

@@ -326,12 +326,7 @@ __global__ void __launch_bounds__(NT, 1) k_fv_local(double2 *q, double2 *qn, dou
       if (lane == 0) sv[j] = sqrt(acc);
     }
     __syncthreads();
-    for (int j = tid; j < c; j += NT) {
-      int rk = 0;
-      const double x = sv[j];
-      for (int i = 0; i < c; ++i) rk += (sv[i] > x || (sv[i] == x && i < j)) ? 1 : 0;
-      perm[min(rk, c - 1)] = j;
-    }
+    for (int j = tid; j < c; j += NT) perm[tn::order_rank(sv, c, j)] = j;
     __syncthreads();
     if (tid == 0) {  // the rank rule of k_fv_finish
       double tot = 0.0;

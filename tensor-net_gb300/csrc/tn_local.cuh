@@ -170,7 +170,10 @@ __device__ void gemm_exact_from(int M, int N, FK from, int K, FP P, FQ Q, FE E) 
 // (de Rijk); a pair belongs to LG lanes, which form the inner product and
 // apply the rotation to their elements.  Norms are carried by a' = a - t |g|,
 // b' = b + t |g| and recomputed each sweep.  Stops after a sweep without a
-// pair above `done` (before its rotation).  Returns the sweeps, -1 at the limit.
+// pair above `done` (before its rotation).  Returns the sweeps, -1 at the
+// limit, -2 before a sweep whose sum of squared norms is not below kNormMax
+// (a NaN or an infinity among them; the vectors are as the sweep found them).
+constexpr float kNormMax = 1e30f;
 template <int NT>
 __device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<float> *Vs, int pv, int c, float *nrm, int *ord,
                                         float floor_, float tol, float done, int max_sweeps) {
@@ -195,14 +198,15 @@ __device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<flo
     float fro = 0.f;
     {
       const float x = tid < c ? nrm[tid] : 0.f;  // (c <= NT)
-      int rk = 0;
+      int rk = 0;  // as order_rank: below, every value is finite
 #pragma unroll 4
       for (int i = 0; i < c; ++i) {
         const float y = nrm[i];
         fro += y;
         rk += (y > x || (y == x && i < tid)) ? 1 : 0;
       }
-      if (tid < c) ord[min(rk, c - 1)] = tid;
+      if (!(fro < kNormMax)) return -2;  // uniform: every thread adds the same values in the same order
+      if (tid < c) ord[rk] = tid;
     }
     const float tiny2 = fmaxf(fro * floor_ * floor_, 1e-37f);
     __syncthreads();
@@ -601,7 +605,8 @@ __device__ __forceinline__ float svd_tolerance(int ell) {
 // operations without counting as its length (an appended identity becomes the
 // accumulated unitary).  Returns the number of sweeps and refinement steps, or -1:
 // A is then a unitary transform of the input that has not converged (a
-// degenerate spectrum, or the sweep limit), for the caller's block Jacobi.
+// degenerate spectrum, or the sweep limit) or the input itself (norms that the
+// float stage cannot hold, NaN), for the caller's block Jacobi.
 template <typename T, int NT>
 __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int max_sweeps, unsigned char *scratch,
                                          double *red, float tol, int tail = 0) {
@@ -627,6 +632,7 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
     __syncthreads();
     const int sw = hestenes<NT>(As, pa, ell, nullptr, 0, c, nrm, ord, float(sweep_floor<float>(ell)), tolf,
                                 fmaxf(tolf, kFloatDone), max_sweeps);
+    if (sw == -2) return -1;
     for (int idx = tid; idx < c * ell; idx += NT) {
       const int j = idx / ell, i = idx - j * ell;
       A[size_t(j) * ld + i] = As[j * pa + i];
@@ -666,6 +672,7 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
         // holds them to its own precision the next one resolves them too
         const int sw = hestenes<NT>(As, pa, ell, Vs, pc, c, nrm, ord, stages == 0 ? Eps<float>::v : floor_t, tolf,
                                     1e-4f, min(max_sweeps, 20));
+        if (sw == -2) return -1;
         sweeps += sw < 0 ? min(max_sweeps, 20) : sw;
         ++stages;
         bulk = false;
@@ -684,6 +691,7 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
       gram_local<T, NT>(A, ld, ell, c, G, pc, stage, pc);
       float fro = 0.f;
       for (int j = 0; j < c; ++j) fro += lead(G[j * pc + j].x);
+      if (!(fro < kNormMax)) return -1;
       const float tiny2 = fmaxf(fro * floor_t * floor_t, 1e-37f);
       // K of every pair above the threshold, r = |g| / (|a_p| |a_q|) and |t|.
       // Pairs below it, down to rounding, go along where their t is small: what

@@ -174,8 +174,8 @@ __device__ int float_sweeps(const Team &tm, cpx<float> *A32, int ell, cpx<float>
     int *kidx = reinterpret_cast<int *>(key + P);
     float part = 0.f;
     for (int j = threadIdx.x; j < P; j += NT) {
-      const float x = j < c ? tw.nrm[j] : -1.f;
-      key[j] = double(x);
+      const float x = j < c ? tw.nrm[j] : 0.f;
+      key[j] = j < c ? double(order_key(x)) : kOrderPad;
       kidx[j] = j;
       if (j < c) part += x;
     }
