@@ -18,6 +18,7 @@
 
 #include "tn_internal.h"
 #include "tn_mps.h"
+#include "tn_workspace.h"
 
 using namespace tn;
 
@@ -69,9 +70,7 @@ struct tn_batch {
   TrajDev *dtraj = nullptr;
   int *dstatus = nullptr;
   double *dstats = nullptr;
-  void *ws = nullptr;
-  size_t ws_stride = 0;
-  bool ws_team = false;
+  Workspace<DeviceMem> ws;
   // Upper estimates of the slots' bond dimensions (a layer's disjoint gates at
   // most double them), for the launch shape only.
   std::vector<uint32_t> chi_hint;
@@ -144,6 +143,15 @@ StepLayout step_layout(uint32_t nt, uint32_t ng, uint32_t nm) {
   L.ents = take(sizeof(double) * std::max<uint32_t>(nt, 1));
   L.total = p;
   return L;
+}
+
+// The batch's workspaces, one per CTA of its largest launch.
+int init_workspace(tn_batch *b) {
+  b->ws.stride = run_work_bytes(b->prec, b->maxcap);
+  b->ws.team_stride = run_team_bytes(b->prec, b->maxcap);
+  const int e = b->ws.ensure(b->grid_max);
+  if (!e) b->ws.ensure_teams(b->grid_max, b->grid_max);
+  return e;
 }
 
 int ensure_step(tn_batch *b, uint32_t nt, uint32_t ng, uint32_t nm) {
@@ -267,6 +275,11 @@ int tune_before(tn_batch *b) {
   return stats_flops(b, &T.flops0);
 }
 
+// Parts for `want` CTAs or clusters, or none, so that every CTA computes alike.
+void *step_parts(tn_batch *b, int want) { return b->ws.teams >= want ? b->ws.team : nullptr; }
+
+int step_ctas(const tn_batch *b) { return b->grid_limit > 0 ? std::min(b->grid_limit, b->grid_max) : b->grid_max; }
+
 int launch_step(tn_batch *b, uint32_t nt, const StepPtrs &P0, bool timed = true) {
   StepPtrs P = P0;
   if (!P.order) {  // most expensive trajectories first, by their current bond dimensions
@@ -281,14 +294,14 @@ int launch_step(tn_batch *b, uint32_t nt, const StepPtrs &P0, bool timed = true)
   la.probs = P.probs;
   la.ents = P.ents;
   la.pout = P.probs;
-  la.ws = b->ws;
-  la.ws_stride = b->ws_stride;
-  la.ws_team = b->ws_team;
+  la.ws = b->ws.base;
+  la.ws_stride = b->ws.stride;
+  la.team_stride = b->ws.team_stride;
   la.max_sweeps = b->max_sweeps;
   la.jacobi_scheme = b->scheme;
   la.theta_simt = b->theta_simt;
   la.qerr = b->dcounter + 9;
-  const int gmax = b->grid_limit > 0 ? std::min(b->grid_limit, b->grid_max) : b->grid_max;
+  const int gmax = step_ctas(b);
   if (b->schedule == 1) {
     // One launch: gate items (most expensive trajectories first), then each
     // trajectory's sweep program as soon as its last gate item has finished.
@@ -319,16 +332,17 @@ int launch_step(tn_batch *b, uint32_t nt, const StepPtrs &P0, bool timed = true)
     // 16, chi = 128, two layers: 210 -> 105 ms.  Beyond that the SMs have trajectories of their own.
     // The results have the same bits either way.
     int grid = gmax;
-    if (b->prec == TN_PREC_DF && b->ws_team && b->grid_limit == 0 && P.chi_hint > 64 && nt <= uint32_t(b->sms)) {
+    if (b->prec == TN_PREC_DF && b->grid_limit == 0 && P.chi_hint > 64 && nt <= uint32_t(b->sms)) {
       const int size = nt <= uint32_t(b->sms) / 8 ? 8 : 4;
       int &n = size == 8 ? b->clusters8 : b->clusters4;
       if (n < 0) n = run_clusters(b->prec, b->sortP, size);
       const int teams = std::min(n, gmax);
-      if (teams > 0) {
+      if (teams > 0 && (la.team = step_parts(b, teams))) {
         la.cluster = size;
         grid = teams;
       }
     }
+    if (!la.cluster) la.team = step_parts(b, gmax);
     if (timed) CKB(cudaEventRecord(b->ev[0], b->st));
     CKB(launch_run(b->prec, la, grid, b->sortP, b->maxcap, b->st));
     if (timed) {
@@ -340,6 +354,7 @@ int launch_step(tn_batch *b, uint32_t nt, const StepPtrs &P0, bool timed = true)
     }
     return TN_OK;
   }
+  la.team = step_parts(b, gmax);
   CKB(launch_compile(b->dtraj, P.list, int(nt), P.order, P.goff, P.gks, P.moff, P.mks, P.posts, b->pcap, b->dprog,
                      b->ditems, b->dgprog, b->dgitems, b->gcap, b->dcounter + 3, b->st));
   CKB(cudaMemsetAsync(b->dcounter, 0, 3 * sizeof(int), b->st));
@@ -468,7 +483,7 @@ int tn_batch_create(uint32_t ntraj, const uint32_t *ns, const tn_trunc *truncs, 
   b->bps = run_blocks_per_sm(precision, b->sortP);
   b->grid_max = std::max(1, b->sms * b->bps);
   b->grid_max = std::min<int>(b->grid_max, int(std::max<uint32_t>(ntraj, b->sum_n / 2)));
-  e = alloc_work(precision, b->maxcap, b->grid_max, &b->ws, &b->ws_stride, &b->ws_team);
+  e = cudaError_t(init_workspace(b));
   if (e != cudaSuccess) return bail(fail(e, "cudaMalloc(workspace)"));
   b->pcap = 4 * b->maxn + 8;
   // reset all slots to |0...0>
@@ -493,7 +508,7 @@ int tn_batch_free(tn_batch *b) {
   if (b->dprog) cudaFree(b->dprog);
   if (b->dstep) cudaFree(b->dstep);
   if (b->hstep) cudaFreeHost(b->hstep);
-  if (b->ws) cudaFree(b->ws);
+  b->ws.release();
   if (b->dtraj) cudaFree(b->dtraj);
   if (b->arena) cudaFree(b->arena);
   for (auto &ev : b->ev)
@@ -1001,7 +1016,7 @@ tn_batch *batch_engine_create(uint32_t slots, int prec, int ws_cap, int max_n, i
   b->bps = run_blocks_per_sm(prec, b->sortP);
   b->grid_max = std::max(1, b->sms * b->bps);
   if (grid_limit > 0) b->grid_max = std::min(b->grid_max, grid_limit);
-  e = alloc_work(prec, b->maxcap, b->grid_max, &b->ws, &b->ws_stride, &b->ws_team);
+  e = cudaError_t(init_workspace(b));
   if (e != cudaSuccess) return bail(fail(e, "cudaMalloc(workspace)"));
   b->pcap = 4 * max_n + 8;
   e = cudaStreamSynchronize(b->st);

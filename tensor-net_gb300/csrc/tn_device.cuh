@@ -321,9 +321,6 @@ __device__ __forceinline__ X *as_shared(X *p) {
   return reinterpret_cast<X *>(smem + (tc::smem_u32(p) - tc::smem_u32(smem)));
 }
 
-template <typename T>
-size_t __host__ __device__ team_bytes(int cap);
-
 template <typename T, int W>
 struct Smem {
   unsigned char *r0;
@@ -405,9 +402,8 @@ __host__ __device__ inline size_t work_bytes(int cap) {
 }
 
 template <typename T>
-__device__ inline Work<T> make_work(void *base, int cap, bool team) {
+__device__ inline Work<T> make_work(void *base, int cap) {
   Work<T> w;
-  w.team = team && team_bytes<T>(cap) ? reinterpret_cast<unsigned char *>(base) + work_bytes<T>(cap) : nullptr;
   unsigned char *p = reinterpret_cast<unsigned char *>(base);
   size_t n4 = size_t(4) * cap * cap;
   w.A = reinterpret_cast<cpx<T> *>(p);

@@ -15,6 +15,7 @@
 
 #include "tn_internal.h"
 #include "tn_mps.h"
+#include "tn_workspace.h"
 
 using namespace tn;
 
@@ -154,25 +155,10 @@ void emit_sweep(std::vector<Instr> &prog, uint32_t n) {
 
 // Launch scratch shared by the single-state API calls of one handle.
 struct Launcher {
-  DevBuf prog, items, counter, gates, us, outc, probs, ents, pout, ws, gprog, gitems;
-  int sortP = 1, ws_cap = 1, ws_ctas = 0, sms = 1;
+  DevBuf prog, items, counter, gates, us, outc, probs, ents, pout, gprog, gitems;
+  Workspace<DeviceMem> ws;
+  int sortP = 1, ws_cap = 1, sms = 1;
   int clusters = -1;  // resident clusters of kTeamCtas (-1: not asked yet)
-  size_t ws_stride = 0;
-  bool ws_team = false;
-  // workspaces of at least ctas CTAs (the caller has waited for the stream)
-  cudaError_t ensure_ws(int prec, int ctas) {
-    if (ctas <= ws_ctas) return cudaSuccess;
-    ws.release();
-    ws_ctas = 0;
-    const cudaError_t e = alloc_work(prec, ws_cap, ctas, &ws.p, &ws_stride, &ws_team);
-    if (e != cudaSuccess) {
-      ws.p = nullptr;
-      return e;
-    }
-    ws.n = ws_stride * size_t(ctas);
-    ws_ctas = ctas;
-    return cudaSuccess;
-  }
   void release() {
     gprog.release();
     gitems.release();
@@ -280,7 +266,9 @@ int mps_alloc(tn_mps *m) {
     cudaDeviceGetAttribute(&m->L.sms, cudaDevAttrMultiProcessorCount, dev);
   }
   m->L.sortP = next_pow2(2 * int(m->cap));
-  CK(m->L.ensure_ws(m->prec, 1));
+  m->L.ws.stride = run_work_bytes(m->prec, m->L.ws_cap);
+  m->L.ws.team_stride = run_team_bytes(m->prec, m->L.ws_cap);
+  CK(cudaError_t(m->L.ws.ensure(1)));
   return TN_OK;
 }
 
@@ -308,22 +296,27 @@ int mps_run(tn_mps *m, const std::vector<Instr> &prog, const std::vector<double>
         if (once) break;
       }
   }
-  // Bonds wider than 32 have more than 64 vectors, which a cluster shares: one
-  // SM of 152 would do them alone otherwise (a chi = 256 gate in double-float:
-  // 920 ms there, 65 ms on eight).  Narrower ones run on one CTA either way.
-  int cluster = 0;
-  if (m->prec != TN_PREC_F64 && L.ws_team && std::min<uint32_t>(m->chi_hint, m->cap) > 32) {
+  // Independent single-operation items (disjoint gates) spread over SMs.  Bonds
+  // wider than 32 have more than 64 vectors, which a cluster shares where the
+  // mode has the shared path: one SM of 152 would do them alone otherwise.
+  // Narrower ones run on one CTA either way.
+  const int np = std::max(1, int(par.size()));
+  int teams = 0;
+  if (L.ws.team_stride && std::min<uint32_t>(m->chi_hint, m->cap) > 32) {
     if (L.clusters < 0) L.clusters = run_clusters(m->prec, L.sortP, kTeamCtas);
-    if (L.clusters > 0) cluster = kTeamCtas;
+    const int want = std::min(np, L.clusters > 0 ? L.clusters : L.sms);
+    if (want > L.ws.teams) CK(cudaStreamSynchronize(m->st));
+    teams = L.ws.ensure_teams(want);
   }
+  const LaunchShape shape = launch_shape(np, L.sms, L.clusters, teams);
+  if (shape.grid > L.ws.ctas) {
+    CK(cudaStreamSynchronize(m->st));
+    CK(cudaError_t(L.ws.ensure(shape.grid)));
+  }
+  const int cluster = shape.clusters ? kTeamCtas : 0;
+  void *const team = shape.parts ? L.ws.team : nullptr;
   if (!par.empty()) {
-    // independent single-operation items (disjoint gates) spread over SMs
-    const int np = int(par.size());
-    const int grid = std::max(1, std::min(np, cluster ? L.clusters : L.sms));
-    if (grid > L.ws_ctas) {
-      CK(cudaStreamSynchronize(m->st));
-      CK(L.ensure_ws(m->prec, grid));
-    }
+    const int grid = shape.grid;
     std::vector<Item> it(np);
     for (int i = 0; i < np; ++i) it[i] = Item{0, i, 1, 0};
     CK(L.gprog.ensure(np * sizeof(Instr)));
@@ -342,9 +335,10 @@ int mps_run(tn_mps *m, const std::vector<Instr> &prog, const std::vector<double>
     la.trajs = m->dtraj.as<TrajDev>();
     la.prog = L.gprog.as<Instr>();
     la.gates = L.gates.as<double>();
-    la.ws = L.ws.p;
-    la.ws_stride = L.ws_stride;
-    la.ws_team = L.ws_team;
+    la.ws = L.ws.base;
+    la.ws_stride = L.ws.stride;
+    la.team = team;
+    la.team_stride = L.ws.team_stride;
     la.cluster = cluster;
     la.max_sweeps = kMaxSweeps;
     la.jacobi_scheme = kDefaultScheme;
@@ -381,9 +375,9 @@ int mps_run(tn_mps *m, const std::vector<Instr> &prog, const std::vector<double>
   la.probs = L.probs.as<double>();
   la.ents = L.ents.as<double>();
   la.pout = L.pout.as<double>();
-  la.ws = L.ws.p;
+  la.ws = L.ws.base;
   la.ws_stride = 0;
-  la.ws_team = L.ws_team;
+  la.team = team;
   la.cluster = cluster;
   la.max_sweeps = kMaxSweeps;
   la.jacobi_scheme = kDefaultScheme;

@@ -90,9 +90,9 @@ struct LaunchArgs {
   double *pout;          // OP_PROBS output, 2 per slot
   void *ws;              // per-CTA workspace
   size_t ws_stride;      // bytes per CTA
-  int ws_team;           // 1: the workspace includes svd_team's part
-  // CTAs that share an item (a cluster, with one workspace that has svd_team's
-  // part); 0 or 1: one
+  void *team;            // bond_team's part of each CTA or cluster, or null
+  size_t team_stride;    // bytes per part
+  // CTAs that share an item (a cluster, with one workspace and one part); 0 or 1: one
   int cluster;
   int max_sweeps;
   int jacobi_scheme;      // 0: block pairs, all pairs per step; 1: within-block then cross-block steps
@@ -124,11 +124,17 @@ constexpr unsigned long long kQueueWaitNs = 120ull * 1000 * 1000 * 1000;
 
 cudaError_t launch_run(int prec, const LaunchArgs &la, int grid, int sortP, int ws_cap, cudaStream_t st);
 size_t run_smem_bytes(int prec, int sortP);
-// Workspace bytes of a CTA; team: with svd_team's part (large double-float
-// bonds run the slower block Jacobi without it).
-size_t run_work_bytes(int prec, int cap, bool team);
-// Workspaces of ctas CTAs with that part if memory allows, else without.
-cudaError_t alloc_work(int prec, int cap, int ctas, void **ws, size_t *stride, bool *team);
+// Workspace bytes of a CTA, and of a CTA's or cluster's part for bond_team
+// (large double-float bonds run the slower block Jacobi without it; 0: none).
+size_t run_work_bytes(int prec, int cap);
+size_t run_team_bytes(int prec, int cap);
+// Device memory for Workspace.  An allocation may fall into another thread's
+// stream capture, which it does not concern.
+struct DeviceMem {
+  int alloc(void **p, size_t bytes);
+  void free(void *p);
+  size_t available();
+};
 int run_blocks_per_sm(int prec, int sortP);
 // Clusters of that many executor CTAs that can be resident at once (0: none).
 int run_clusters(int prec, int sortP, int cluster);

@@ -267,7 +267,8 @@ __global__ void k_compile_dd(const TrajDev *trajs, const int *list, int nt, cons
 #define TN_DECLARE_RUN(SUFFIX)                                                                              \
   cudaError_t launch_run_##SUFFIX(const LaunchArgs &la, int grid, int sortP, int ws_cap, cudaStream_t st);  \
   size_t run_smem_##SUFFIX(int sortP);                                                                      \
-  size_t run_work_##SUFFIX(int cap, bool team);                                                             \
+  size_t run_work_##SUFFIX(int cap);                                                                        \
+  size_t run_team_##SUFFIX(int cap);                                                                        \
   int run_blocks_##SUFFIX(int sortP);                                                                       \
   int run_clusters_##SUFFIX(int sortP, int cluster);
 TN_DECLARE_RUN(f32)
@@ -275,6 +276,7 @@ TN_DECLARE_RUN(f64)
 TN_DECLARE_RUN(df)
 
 cudaError_t launch_run(int prec, const LaunchArgs &la, int grid, int sortP, int ws_cap, cudaStream_t st) {
+  if (la.cluster > 1 && !la.team) return cudaErrorInvalidValue;  // its members meet in the part
   if (prec == 0) return launch_run_f64(la, grid, sortP, ws_cap, st);
   if (prec == 2) return launch_run_df(la, grid, sortP, ws_cap, st);
   return launch_run_f32(la, grid, sortP, ws_cap, st);
@@ -284,19 +286,35 @@ size_t run_smem_bytes(int prec, int sortP) {
   return prec == 0 ? run_smem_f64(sortP) : (prec == 2 ? run_smem_df(sortP) : run_smem_f32(sortP));
 }
 
-size_t run_work_bytes(int prec, int cap, bool team) {
-  return prec == 0 ? run_work_f64(cap, team) : (prec == 2 ? run_work_df(cap, team) : run_work_f32(cap, team));
+size_t run_work_bytes(int prec, int cap) {
+  return prec == 0 ? run_work_f64(cap) : (prec == 2 ? run_work_df(cap) : run_work_f32(cap));
 }
 
-cudaError_t alloc_work(int prec, int cap, int ctas, void **ws, size_t *stride, bool *team) {
-  for (int full = 1; full >= 0; --full) {
-    *team = full != 0;
-    *stride = run_work_bytes(prec, cap, *team);
-    const cudaError_t e = cudaMalloc(ws, *stride * size_t(ctas));
-    if (e != cudaErrorMemoryAllocation || !full) return e;
+size_t run_team_bytes(int prec, int cap) {
+  return prec == 0 ? run_team_f64(cap) : (prec == 2 ? run_team_df(cap) : run_team_f32(cap));
+}
+
+int DeviceMem::alloc(void **p, size_t bytes) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const cudaError_t e = cudaMalloc(p, bytes);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) {
+    *p = nullptr;
     (void)cudaGetLastError();
   }
-  return cudaErrorMemoryAllocation;
+  return int(e);
+}
+
+void DeviceMem::free(void *p) { (void)cudaFree(p); }
+
+size_t DeviceMem::available() {
+  size_t avail = 0, total = 0;
+  if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return avail;
 }
 
 int run_clusters(int prec, int sortP, int cluster) {

@@ -103,7 +103,7 @@ extern "C" int tn_mps_apply_unitary2_noalloc(tn_mps *m, uint32_t k, const double
   if (rows != 4 || cols != 4) return TN_ERR_OPERATOR_SHAPE;
   for (int i = 0; i < 32; ++i)
     if (!std::isfinite(op[i])) return TN_ERR_INVALID_ARG;
-  const size_t need = tn::run_work_bytes(v.prec, v.cap, false);
+  const size_t need = tn::run_work_bytes(v.prec, v.cap);
   if (need > kScratchBytes) {
     tn::set_last_error("tn_mps_apply_unitary2_noalloc: the handle's bond capacity needs more scratch than the "
                        "4.5 MiB fixed array (chi <= 270 in mixed precision, chi <= 191 in float64 or double-float)",

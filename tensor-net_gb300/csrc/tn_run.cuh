@@ -34,8 +34,8 @@ __global__ void __launch_bounds__(NT, 1) k_run(LaunchArgs la, int sortP, int ws_
     tm.rank = int(blockIdx.x) % la.cluster;  // clusters are consecutive blocks of a one-dimensional grid
   }
   const int team_id = int(blockIdx.x) / tm.size;
-  Work<T> wk = make_work<T>(reinterpret_cast<unsigned char *>(la.ws) + size_t(team_id) * la.ws_stride, ws_cap,
-                            la.ws_team != 0);
+  Work<T> wk = make_work<T>(reinterpret_cast<unsigned char *>(la.ws) + size_t(team_id) * la.ws_stride, ws_cap);
+  if (la.team) wk.team = reinterpret_cast<unsigned char *>(la.team) + size_t(team_id) * la.team_stride;
   const bool dd = la.rem != nullptr;
   // float: one 128 x 256 FP32 accumulator tile (theta and recovery GEMMs);
   // double-float: eight 128 x 64 level accumulators of the tensor-core update
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(NT, 1) k_run(LaunchArgs la, int sortP, int ws_
     sm.tc = la.theta_simt == 0;
   }
   // A team's first member takes the items and passes them on through the team's
-  // workspace (a launch with clusters has one).
+  // part (launch_run refuses clusters without one).
   volatile unsigned int *pass = tm.size > 1 ? team_work<T>(wk.team, ws_cap).flag + kTeamFlags : nullptr;
   for (;;) {
     if (threadIdx.x == 0 && tm.rank == 0) {
@@ -235,7 +235,8 @@ static int run_blocks_t(int sortP) {
     return launch_run_t<T, kThreads, kBlockW>(la, grid, sortP, ws_cap, st);                                \
   }                                                                                                         \
   size_t run_smem_##SUFFIX(int sortP) { return SmemLayout<T, kBlockW>::total(sortP); }                      \
-  size_t run_work_##SUFFIX(int cap, bool team) { return work_bytes<T>(cap) + (team ? team_bytes<T>(cap) : 0); } \
+  size_t run_work_##SUFFIX(int cap) { return work_bytes<T>(cap); }                                          \
+  size_t run_team_##SUFFIX(int cap) { return team_bytes<T>(cap); }                                          \
   int run_blocks_##SUFFIX(int sortP) { return run_blocks_t<T, kThreads, kBlockW>(sortP); }                  \
   int run_clusters_##SUFFIX(int sortP, int cluster) { return run_clusters_t<T, kThreads, kBlockW>(sortP, cluster); }
 
