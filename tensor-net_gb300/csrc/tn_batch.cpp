@@ -72,7 +72,7 @@ struct tn_batch {
   double *dstats = nullptr;
   Workspace<DeviceMem> ws;
   // Upper estimates of the slots' bond dimensions (a layer's disjoint gates at
-  // most double them), for the launch shape only.
+  // most double them), for the launch shape and the parts only.
   std::vector<uint32_t> chi_hint;
   int clusters4 = -1, clusters8 = -1;  // resident clusters (-1: not asked yet)
   // step buffers: one packed device block + one pinned host block
@@ -149,9 +149,8 @@ StepLayout step_layout(uint32_t nt, uint32_t ng, uint32_t nm) {
 int init_workspace(tn_batch *b) {
   b->ws.stride = run_work_bytes(b->prec, b->maxcap);
   b->ws.team_stride = run_team_bytes(b->prec, b->maxcap);
-  const int e = b->ws.ensure(b->grid_max);
-  if (!e) b->ws.ensure_teams(b->grid_max, b->grid_max);
-  return e;
+  b->ws.keep_parts = true;  // graphs of earlier launches point to them
+  return b->ws.ensure(b->grid_max);
 }
 
 int ensure_step(tn_batch *b, uint32_t nt, uint32_t ng, uint32_t nm) {
@@ -275,8 +274,17 @@ int tune_before(tn_batch *b) {
   return stats_flops(b, &T.flops0);
 }
 
-// Parts for `want` CTAs or clusters, or none, so that every CTA computes alike.
-void *step_parts(tn_batch *b, int want) { return b->ws.teams >= want ? b->ws.team : nullptr; }
+// Parts for `want` CTAs or clusters of a launch whose widest bond is chi_hint
+// (0: not known), when it can have an operation for bond_team: on a single CTA
+// that is double-float beyond chi = 32.  All of them or none, so that every CTA
+// computes alike.  None is taken while the batch's stream is captured.
+void *step_parts(tn_batch *b, int want, uint32_t chi_hint) {
+  if (b->prec != TN_PREC_DF || (chi_hint != 0 && chi_hint <= 32)) return nullptr;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (b->ws.teams < want && cudaStreamIsCapturing(b->st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone)
+    b->ws.ensure_teams(want, want);
+  return b->ws.teams >= want ? b->ws.team : nullptr;
+}
 
 int step_ctas(const tn_batch *b) { return b->grid_limit > 0 ? std::min(b->grid_limit, b->grid_max) : b->grid_max; }
 
@@ -337,12 +345,12 @@ int launch_step(tn_batch *b, uint32_t nt, const StepPtrs &P0, bool timed = true)
       int &n = size == 8 ? b->clusters8 : b->clusters4;
       if (n < 0) n = run_clusters(b->prec, b->sortP, size);
       const int teams = std::min(n, gmax);
-      if (teams > 0 && (la.team = step_parts(b, teams))) {
+      if (teams > 0 && (la.team = step_parts(b, teams, P.chi_hint))) {
         la.cluster = size;
         grid = teams;
       }
     }
-    if (!la.cluster) la.team = step_parts(b, gmax);
+    if (!la.cluster) la.team = step_parts(b, gmax, P.chi_hint);
     if (timed) CKB(cudaEventRecord(b->ev[0], b->st));
     CKB(launch_run(b->prec, la, grid, b->sortP, b->maxcap, b->st));
     if (timed) {
@@ -354,7 +362,7 @@ int launch_step(tn_batch *b, uint32_t nt, const StepPtrs &P0, bool timed = true)
     }
     return TN_OK;
   }
-  la.team = step_parts(b, gmax);
+  la.team = step_parts(b, gmax, P.chi_hint);
   CKB(launch_compile(b->dtraj, P.list, int(nt), P.order, P.goff, P.gks, P.moff, P.mks, P.posts, b->pcap, b->dprog,
                      b->ditems, b->dgprog, b->dgitems, b->gcap, b->dcounter + 3, b->st));
   CKB(cudaMemsetAsync(b->dcounter, 0, 3 * sizeof(int), b->st));
@@ -763,6 +771,7 @@ int tn_batch_step_device(tn_batch *b, uint32_t nt) {
   if (it == b->graphs.end()) {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
+    step_parts(b, step_ctas(b), 0);  // (the capture itself allocates nothing)
     CKB(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
     StepPtrs P = ptrs_of(L, reinterpret_cast<char *>(b->din));
     P.order = nullptr;  // ranked on the device inside the graph
@@ -1040,6 +1049,8 @@ int batch_bind(tn_batch *b, uint32_t t, const TrajDev &d) {
   b->n_alloc[t] = uint32_t(d.n);
   b->cap[t] = uint32_t(d.cap);
   b->maxn = std::max(b->maxn, d.n);
+  b->chi_hint.resize(b->ntraj, 1);
+  b->chi_hint[t] = 1;
   CKB(cudaMemcpyAsync(b->dtraj + t, &h, sizeof(TrajDev), cudaMemcpyHostToDevice, b->st));
   int *dl = b->dcounter + 4 + (t & 3);  // small staging words, distinct per pending bind
   int tt = int(t);
