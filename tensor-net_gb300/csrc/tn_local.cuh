@@ -171,12 +171,13 @@ __device__ void gemm_exact_from(int M, int N, FK from, int K, FP P, FQ Q, FE E) 
 // apply the rotation to their elements.  Norms are carried by a' = a - t |g|,
 // b' = b + t |g| and recomputed each sweep.  Stops after a sweep without a
 // pair above `done` (before its rotation).  Returns the sweeps, -1 at the
-// limit, -2 before a sweep whose sum of squared norms is not below kNormMax
-// (a NaN or an infinity among them; the vectors are as the sweep found them).
-constexpr float kNormMax = 1e30f;
+// limit, -2 before a sweep whose sum of squared norms is below `least` or not
+// below kNormMax (a NaN or an infinity among them; the vectors are as the sweep
+// found them).
+constexpr float kNormMax = 1e30f, kNormTiny = 1e-37f;
 template <int NT>
 __device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<float> *Vs, int pv, int c, float *nrm, int *ord,
-                                        float floor_, float tol, float done, int max_sweeps) {
+                                        float floor_, float least, float tol, float done, int max_sweeps) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cp = c + (c & 1), np = cp >> 1, ring = cp - 1;
   int LG = 32;
@@ -205,10 +206,10 @@ __device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<flo
         fro += y;
         rk += (y > x || (y == x && i < tid)) ? 1 : 0;
       }
-      if (!(fro < kNormMax)) return -2;  // uniform: every thread adds the same values in the same order
+      if (!(fro >= least && fro < kNormMax)) return -2;  // uniform: every thread adds the same values in the same order
       if (tid < c) ord[rk] = tid;
     }
-    const float tiny2 = fmaxf(fro * floor_ * floor_, 1e-37f);
+    const float tiny2 = fmaxf(fro * floor_ * floor_, kNormTiny);
     __syncthreads();
     int far = 0;
     if (tid < active) {
@@ -606,10 +607,11 @@ __device__ __forceinline__ float svd_tolerance(int ell) {
 // accumulated unitary).  Returns the number of sweeps and refinement steps, or -1:
 // A is then a unitary transform of the input that has not converged (a
 // degenerate spectrum, or the sweep limit) or the input itself (norms that the
-// float stage cannot hold, NaN), for the caller's block Jacobi.
+// float stage cannot hold, NaN), for the caller's block Jacobi.  svd_local_steps
+// returns -2 for such norms.
 template <typename T, int NT>
-__device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int max_sweeps, unsigned char *scratch,
-                                         double *red, float tol, int tail = 0) {
+__device__ __forceinline__ int svd_local_steps(cpx<T> *A, int ld, int ell, int c, int max_sweeps, unsigned char *scratch,
+                                               double *red, float tol, int tail) {
   using L = LocalSvd<T>;
   const int tid = threadIdx.x;
   const int pa = L::odd(ell), pc = L::odd(c);
@@ -630,9 +632,9 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
     int *ord = reinterpret_cast<int *>(nrm + c);
     load();
     __syncthreads();
-    const int sw = hestenes<NT>(As, pa, ell, nullptr, 0, c, nrm, ord, float(sweep_floor<float>(ell)), tolf,
+    const int sw = hestenes<NT>(As, pa, ell, nullptr, 0, c, nrm, ord, float(sweep_floor<float>(ell)), 0.f, tolf,
                                 fmaxf(tolf, kFloatDone), max_sweeps);
-    if (sw == -2) return -1;
+    if (sw == -2) return -2;
     for (int idx = tid; idx < c * ell; idx += NT) {
       const int j = idx / ell, i = idx - j * ell;
       A[size_t(j) * ld + i] = As[j * pa + i];
@@ -651,6 +653,16 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
     int *ord = reinterpret_cast<int *>(nrm + c);
     dd *dg = reinterpret_cast<dd *>(nrm);  // (not needed while the sweeps run)
     const float floor_t = float(sweep_floor<T>(ell));
+    // float64: the float stage takes no vectors whose noise level is out of its
+    // range.  The Gram matrix is scaled before its entries are compared in float:
+    // tol times the smallest kept value squared is 4e-44 at norm 1.
+    const float least2 = std::is_same<T, double>::value ? kNormTiny / (floor_t * floor_t) : 0.f;
+    auto gram = [](T x) {
+      if constexpr (std::is_same<T, double>::value)
+        return lead(x * 0x1p66);
+      else
+        return lead(x);
+    };
     // a correction formed in float is exact to the working precision below this angle
     constexpr float kFloatApply = std::is_same<T, double>::value ? 1e-9f : 1e-7f;
     constexpr int kMaxStages = 3, kMaxSteps = 10;
@@ -670,9 +682,9 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
         __syncthreads();
         // the first stage leaves vectors at the float noise level alone; once A
         // holds them to its own precision the next one resolves them too
-        const int sw = hestenes<NT>(As, pa, ell, Vs, pc, c, nrm, ord, stages == 0 ? Eps<float>::v : floor_t, tolf,
-                                    1e-4f, min(max_sweeps, 20));
-        if (sw == -2) return -1;
+        const int sw = hestenes<NT>(As, pa, ell, Vs, pc, c, nrm, ord, stages == 0 ? Eps<float>::v : floor_t, least2,
+                                    tolf, 1e-4f, min(max_sweeps, 20));
+        if (sw == -2) return stages == 0 ? -2 : -1;
         sweeps += sw < 0 ? min(max_sweeps, 20) : sw;
         ++stages;
         bulk = false;
@@ -690,9 +702,9 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
       if (step == kMaxSteps) return -1;
       gram_local<T, NT>(A, ld, ell, c, G, pc, stage, pc);
       float fro = 0.f;
-      for (int j = 0; j < c; ++j) fro += lead(G[j * pc + j].x);
+      for (int j = 0; j < c; ++j) fro += gram(G[j * pc + j].x);
       if (!(fro < kNormMax)) return -1;
-      const float tiny2 = fmaxf(fro * floor_t * floor_t, 1e-37f);
+      const float tiny2 = fmaxf(fro * floor_t * floor_t, kNormTiny);
       // K of every pair above the threshold, r = |g| / (|a_p| |a_q|) and |t|.
       // Pairs below it, down to rounding, go along where their t is small: what
       // they leave would enter the recovered side as r sigma_p / sigma_q, and
@@ -709,15 +721,15 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
         }
         cpx<float> vpq = czero<float>(), vqp = czero<float>();
         const T at_ = G[p * pc + p].x, bt_ = G[q * pc + q].x;
-        const float a = lead(at_), b = lead(bt_);
+        const float a = gram(at_), b = gram(bt_);
         if (a > tiny2 && b > tiny2) {
           const cpx<T> g = G[p * pc + q];
           const float sc = rsqrtf(a) * rsqrtf(b);
-          const float hx = lead(g.x) * sc, hy = lead(g.y) * sc, r2 = fmaf(hx, hx, hy * hy), r = sqrtf(r2);
+          const float hx = gram(g.x) * sc, hy = gram(g.y) * sc, r2 = fmaf(hx, hx, hy * hy), r = sqrtf(r2);
           rmax = fmaxf(rmax, r);
           if (r > least) {
             const float rr = 1.f / r;
-            const float z = 0.5f * (lead(bt_ - at_) * sc) * rr;
+            const float z = 0.5f * (gram(bt_ - at_) * sc) * rr;
             const float z1 = fmaf(z, z, 1.f);
             const float t = fabsf(z) > 1e15f ? 0.5f / z : copysignf(1.f / (fabsf(z) + sqrtf(z1)), z);
             const bool over = r > tol, take = over || fabsf(t) <= kFloatApply;
@@ -757,6 +769,44 @@ __device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int 
         __syncthreads();
       }
     }
+  }
+}
+
+// A scaled by 2^e (its ell entries, not the tail).
+template <int NT>
+__device__ __noinline__ void scale_vectors(cpx<double> *A, int ld, int ell, int c, int e) {
+  for (int idx = threadIdx.x; idx < c * ell; idx += NT) {
+    cpx<double> &x = A[size_t(idx / ell) * ld + idx % ell];
+    x = mkc<double>(scalbn(x.x, e), scalbn(x.y, e));
+  }
+  __syncthreads();
+}
+
+// In float64, vectors out of the float stage's range (a gate or a state far from
+// norm 1) are brought to norm 1 by a power of two for the time of the SVD.
+template <typename T, int NT>
+__device__ __forceinline__ int svd_local(cpx<T> *A, int ld, int ell, int c, int max_sweeps, unsigned char *scratch,
+                                         double *red, float tol, int tail = 0) {
+  if constexpr (!std::is_same<T, double>::value) {
+    return max(-1, svd_local_steps<T, NT>(A, ld, ell, c, max_sweeps, scratch, red, tol, tail));
+  } else {
+    int e = 0, r;
+#pragma unroll 1
+    for (;;) {
+      r = svd_local_steps<T, NT>(A, ld, ell, c, max_sweeps, scratch, red, tol, tail);
+      if (r != -2 || e != 0) break;
+      int top = 0;  // largest exponent field
+      for (int idx = threadIdx.x; idx < c * ell; idx += NT) {
+        const cpx<T> x = A[size_t(idx / ell) * ld + idx % ell];
+        top = max(top, max(__double2hiint(fabs(x.x)), __double2hiint(fabs(x.y))) >> 20);
+      }
+      top = int(block_max<NT>(float(top), red));
+      if (top == 0 || top == 2047 || top == 1023) break;  // zeros; not finite
+      e = 1023 - top;
+      scale_vectors<NT>(A, ld, ell, c, e);
+    }
+    if (e != 0) scale_vectors<NT>(A, ld, ell, c, -e);
+    return max(-1, r);
   }
 }
 
