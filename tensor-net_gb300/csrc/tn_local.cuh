@@ -129,6 +129,40 @@ __device__ __forceinline__ float block_max(float v, double *red) {
   return __uint_as_float(m);
 }
 
+// Sums of two values over the CTA in the arithmetic R (uniform result).
+template <typename R, int NT>
+__device__ __forceinline__ void block_sum2_in(R &a, R &b, double *red) {
+  R *r = reinterpret_cast<R *>(red);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a = a + shfl_xor(a, o);
+    b = b + shfl_xor(b, o);
+  }
+  __syncthreads();
+  if (lane == 0) {
+    r[warp] = a;
+    r[NT / 32 + warp] = b;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    a = lane < NT / 32 ? r[lane] : R(0);
+    b = lane < NT / 32 ? r[NT / 32 + lane] : R(0);
+#pragma unroll
+    for (int o = NT / 64; o > 0; o >>= 1) {
+      a = a + shfl_xor(a, o);
+      b = b + shfl_xor(b, o);
+    }
+    if (lane == 0) {
+      r[2 * (NT / 32)] = a;
+      r[2 * (NT / 32) + 1] = b;
+    }
+  }
+  __syncthreads();
+  a = r[2 * (NT / 32)];
+  b = r[2 * (NT / 32) + 1];
+}
+
 // Half of the smallest power of two that is at least n, within a warp: the
 // first distance of a butterfly sum whose lanes from n on hold zeros.
 __device__ __forceinline__ int warp_half(int n) { return n > 16 ? 16 : n > 1 ? 1 << (31 - __clz(n - 1)) : 0; }
@@ -283,36 +317,40 @@ __device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<flo
 // ------------------------------------------------ 2. unitary to working precision
 // V (I + W) is unitary for V^H V = I + S, S = D + O (D diagonal): V D_g with
 // D_g = (I + D)^(-1/2) has V^H V - I = S1 = D_g O D_g, so
-//   I + W = D_g (I - S1/2 + 3/8 S1^2 - ...).
-// O is small (below 2e-5: the series ends there), D may be larger: the
-// approximate reciprocal square roots of the float rotations shrink every
-// column a little (up to 1e-3 over long sweeps), and a rotation by t in I + K
-// has D = t^2.  dg_minus1: (1 + x)^(-1/2) - 1 in double-float.
+//   I + W = D_g (I - S1/2 + 3/8 S1^2 - 5/16 S1^3 + 35/128 S1^4 - ...).
+// O is small, D may be larger: the approximate reciprocal square roots of the
+// float rotations shrink every column a little (up to 1e-3 over long sweeps),
+// and a rotation by t in I + K has D = t^2.  What a truncated series leaves is
+// a power of S1's spectral norm, so its limits are on norms (Frobenius here,
+// row sums in team_correction): entries alone say little, 64 x 64 of them at
+// 2e-5 have norm 6e-4.  dg_minus1: (1 + x)^(-1/2) - 1 in double-float.
 __device__ __forceinline__ dd dg_minus1(dd x) {
   // without cancellation: 1 / s - 1 = -x / (s (1 + s)), s = sqrt(1 + x)
   const dd s = sqrt(dd(1.f) + x);
   return -(x / (s * (dd(1.f) + s)));
 }
 // W[k][y] from S[k][y] (diagonal: x = S[k][k]), the factors dk, dy = D_g - 1 of
-// k and y, and sq = (S1^2)[k][y].
-__device__ __forceinline__ cpx<dd> unit_entry(bool diag, cpx<dd> s, dd dk, dd dy, cpx<float> sq) {
+// k and y, and hi = (3/8 S1^2 - ...)[k][y].
+__device__ __forceinline__ cpx<dd> unit_entry(bool diag, cpx<dd> s, dd dk, dd dy, cpx<float> hi) {
   const float gk = 1.f + dk.hi;
-  if (diag) return mkc<dd>(dk + dd(0.375f * gk * sq.x), dd(0.f, 0.f));
+  if (diag) return mkc<dd>(dk + dd(gk * hi.x), dd(0.f, 0.f));
   // D_g,k S1 = (1 + dk)^2 O (1 + dy)
   const dd f = (dd(1.f) + dk) * (dd(1.f) + dk) * (dd(1.f) + dy);
   const dd ax = f * s.x, ay = f * s.y;
-  return mkc<dd>(dd(-0.5f * ax.hi, -0.5f * ax.lo) + dd(0.375f * gk * sq.x),
-                 dd(-0.5f * ay.hi, -0.5f * ay.lo) + dd(0.375f * gk * sq.y));
+  return mkc<dd>(dd(-0.5f * ax.hi, -0.5f * ax.lo) + dd(gk * hi.x), dd(-0.5f * ay.hi, -0.5f * ay.lo) + dd(gk * hi.y));
 }
-constexpr float kOffMax = 2e-5f, kDiagMax = 0.1f;
+// Frobenius norms of O and D: the third-order term is left out below kOffSquare
+// (it is 2e-17 there), the fourth below kOffMax (4e-16 at the most; S1^2 in float
+// errs by no more).
+constexpr float kOffSquare = 3e-6f, kOffMax = 2e-4f, kDiagMax = 0.3f;
 
 // Q (c x c, row-major with pitch pq) <- the unitary factor of V (float,
 // columns Vs[k * pv + r]), V unitary to a few float roundings or I + K.
 // S = V^H V - I is formed from exact float products; float Newton-Schulz
-// steps bring its off-diagonals below 2e-5 first where they are larger (I + K
-// with a t near 1); then Q = V (I + W) by unit_entry, whose error is of the
-// order |O|^3 < 1e-14.  dg: c double-float values of scratch.
-// The correction V W is accumulated in double-float in every mode (W < 1e-5,
+// steps bring its off-diagonals below kOffMax first where they are larger (I + K
+// with a t near 1); then Q = V (I + W) by unit_entry.  dg: c double-float values
+// of scratch.
+// The correction V W is accumulated in double-float in every mode (W < 2e-4,
 // so its error is below 1e-16).  Returns false (Q not written) when V is too
 // far from unitary.
 template <typename T, int NT>
@@ -322,11 +360,12 @@ __device__ __noinline__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S
   S = as_shared(S);
   Q = as_shared(Q);
   dg = as_shared(dg);
-  cpx<float> *const tmp = reinterpret_cast<cpx<float> *>(Q);  // c x c floats, until Q is written
+  cpx<float> *const tmp = reinterpret_cast<cpx<float> *>(Q);  // twice c x c floats, until Q is written
+  float off = 0.f;
   const int tid = threadIdx.x;
   const int ntri = c * (c + 1) / 2;
   for (int it = 0;; ++it) {
-    float smax = 0.f, dmax = 0.f;
+    float o2 = 0.f, d2 = 0.f;
 #pragma unroll 1
     for (int e = tid; e < ntri; e += NT) {
       int p, q;
@@ -347,15 +386,14 @@ __device__ __noinline__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S
       S[p * ps + q] = mkc<dd>(sx, sy);
       if (p != q) S[q * ps + p] = mkc<dd>(sx, -sy);
       if (p == q)
-        dmax = fmaxf(dmax, fabsf(sx.hi));
+        d2 = fmaf(sx.hi, sx.hi, d2);
       else
-        smax = fmaxf(smax, fmaxf(fabsf(sx.hi), fabsf(sy.hi)));
-      if (!(sx.hi == sx.hi && sy.hi == sy.hi)) smax = __int_as_float(0x7f800000);
+        o2 = fmaf(2.f * sx.hi, sx.hi, fmaf(2.f * sy.hi, sy.hi, o2));
     }
-    smax = block_max<NT>(smax, red);  // (ends with S visible: its barriers follow the stores)
-    dmax = block_max<NT>(dmax, red);
-    if (smax <= kOffMax && dmax <= kDiagMax) break;
-    if (!(smax <= 0.5f && dmax <= 0.5f) || it >= 6) return false;
+    block_sum2_in<float, NT>(o2, d2, red);  // (ends with S visible: its barriers follow the stores)
+    off = sqrtf(o2);
+    if (off <= kOffMax && d2 <= kDiagMax * kDiagMax) break;
+    if (!(o2 <= 1.f && d2 <= 1.f) || it >= 6) return false;
 #pragma unroll 1
     for (int o = tid; o < c * c; o += NT) {
       const int y = o / c, r = o - y * c;
@@ -373,7 +411,7 @@ __device__ __noinline__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S
     for (int o = tid; o < c * c; o += NT) Vs[(o / c) * pv + o % c] = tmp[o];
     __syncthreads();
   }
-  // W in place of S (the square in float)
+  // W in place of S (the square and the cube in float)
   for (int k = tid; k < c; k += NT) dg[k] = dg_minus1(S[k * ps + k].x);
   __syncthreads();
 #pragma unroll 1
@@ -391,10 +429,31 @@ __device__ __noinline__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S
     tmp[o] = mkc<float>(a.x * g, a.y * g);
   }
   __syncthreads();
+  cpx<float> *const hi = off > kOffSquare ? tmp + c * c : tmp;
+  const float w2 = off > kOffSquare ? 1.f : 0.375f;
+  if (off > kOffSquare) {
+#pragma unroll 1
+    for (int o = tid; o < c * c; o += NT) {
+      const int y = o / c, x = o - y * c;
+      cpx<float> a = czero<float>();
+#pragma unroll 1
+      for (int k = 0; k < c; ++k) {
+        if (k == x) continue;
+        const cpx<dd> s = S[x * ps + k];
+        const float g = 1.f + dg[k].hi;
+        a = cfma(mkc<float>(s.x.hi * g, s.y.hi * g), tmp[y * c + k], a);
+      }
+      const float g = 0.3125f * (1.f + dg[x].hi);
+      const cpx<float> q = tmp[o];
+      hi[o] = mkc<float>(fmaf(0.375f, q.x, -g * a.x), fmaf(0.375f, q.y, -g * a.y));
+    }
+    __syncthreads();
+  }
 #pragma unroll 1
   for (int o = tid; o < c * c; o += NT) {
     const int y = o / c, x = o - y * c;
-    S[x * ps + y] = unit_entry(x == y, S[x * ps + y], dg[x], dg[y], tmp[o]);
+    const cpx<float> h = hi[o];
+    S[x * ps + y] = unit_entry(x == y, S[x * ps + y], dg[x], dg[y], mkc<float>(w2 * h.x, w2 * h.y));
   }
   __syncthreads();
 #pragma unroll 1
@@ -419,12 +478,12 @@ __device__ __noinline__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S
 }
 
 // Q <- the unitary factor of I + K for a refinement step: K anti-Hermitian,
-// float, K[x][y] = Vs[y * pv + x] off the diagonal, entries at most kStepMax.
-// (I + K)(I - K^2)^(-1/2) = I + K + K^2 / 2 + K^3 / 2 + 3/8 K^4 + O(K^5): K is
-// exact, K^2 is summed in double-float, and what follows is below 1e-10, so
-// floats do.  Two passes instead of unitarise's five and its maxima: a third of
+// float, K[x][y] = Vs[y * pv + x] off the diagonal, of Frobenius norm at most
+// kStepMax.  (I + K)(I - K^2)^(-1/2) = I + K + K^2 / 2 + K^3 / 2 + 3/8 K^4 +
+// 3/8 K^5 ...: K is exact, K^2 is summed in double-float, what follows is below
+// 5e-10, so floats do, and what is left out is below 4e-16.  Two passes instead of unitarise's five and its maxima: a third of
 // its time.  Y: c x c of scratch for K^2.
-constexpr float kStepMax = 3e-4f;
+constexpr float kStepMax = 1e-3f;
 template <typename T, int NT>
 __device__ __noinline__ void unitary_step(const cpx<float> *Vs, int pv, int c, cpx<dd> *Y, int py, cpx<T> *Q, int pq) {
   Vs = as_shared(Vs);
@@ -664,7 +723,8 @@ __device__ __forceinline__ int svd_local_steps(cpx<T> *A, int ld, int ell, int c
         return lead(x);
     };
     // a correction formed in float is exact to the working precision below this angle
-    constexpr float kFloatApply = std::is_same<T, double>::value ? 1e-9f : 1e-7f;
+    // and its square, which that leaves out, is below the working precision
+    constexpr float kFloatApply = std::is_same<T, double>::value ? 1e-9f : 3e-8f;
     constexpr int kMaxStages = 3, kMaxSteps = 10;
     int sweeps = 0, stages = 0;
     // what is due: a float stage, a product with the unitary factor of V (or
@@ -706,11 +766,13 @@ __device__ __forceinline__ int svd_local_steps(cpx<T> *A, int ld, int ell, int c
       if (!(fro < kNormMax)) return -1;
       const float tiny2 = fmaxf(fro * floor_t * floor_t, kNormTiny);
       // K of every pair above the threshold, r = |g| / (|a_p| |a_q|) and |t|.
-      // Pairs below it, down to rounding, go along where their t is small: what
-      // they leave would enter the recovered side as r sigma_p / sigma_q, and
-      // with them a trajectory's error against float64 is 2-10 times smaller.
-      float rmax = 0.f, kmax = 0.f, small = 0.f;
-      const float least = tol < 1e-10f ? 0.03125f * tol : tol;
+      // Pairs below it, down to rounding, go along where their t is small (so
+      // that all of them together stay below kFloatApply): what they leave would
+      // enter the recovered side as r sigma_p / sigma_q, and with them a
+      // trajectory's error against float64 is 2-10 times smaller.  k2: the
+      // squared Frobenius norm of K.
+      float rmax = 0.f, kmax = 0.f, k2 = 0.f, none = 0.f;
+      const float least = tol < 1e-10f ? 0.03125f * tol : tol, along = kFloatApply / float(c);
 #pragma unroll 1
       for (int e = tid; e < c * (c + 1) / 2; e += NT) {
         int p, q;
@@ -732,10 +794,10 @@ __device__ __forceinline__ int svd_local_steps(cpx<T> *A, int ld, int ell, int c
             const float z = 0.5f * (gram(bt_ - at_) * sc) * rr;
             const float z1 = fmaf(z, z, 1.f);
             const float t = fabsf(z) > 1e15f ? 0.5f / z : copysignf(1.f / (fabsf(z) + sqrtf(z1)), z);
-            const bool over = r > tol, take = over || fabsf(t) <= kFloatApply;
+            const bool over = r > tol, take = over || fabsf(t) <= along;
             if (over) kmax = fmaxf(kmax, fabsf(t));
             if (take) {
-              small = 1.f;
+              k2 = fmaf(2.f * t, t, k2);
               const float ex = hx * rr, ey = -hy * rr;
               vqp = mkc<float>(-t * ex, -t * ey);
               vpq = mkc<float>(t * ex, -t * ey);
@@ -747,10 +809,10 @@ __device__ __forceinline__ int svd_local_steps(cpx<T> *A, int ld, int ell, int c
       }
       rmax = block_max<NT>(rmax, red);
       kmax = block_max<NT>(kmax, red);
-      small = block_max<NT>(small, red);
+      block_sum2_in<float, NT>(k2, none, red);
       if (!(rmax < 2.f)) return -1;  // not a number
       if (rmax <= tol) {
-        if (!(small > 0.f)) return sweeps + 1;
+        if (!(k2 > 0.f)) return sweeps + 1;
         small_step = last = true;
         continue;
       }
@@ -759,8 +821,8 @@ __device__ __forceinline__ int svd_local_steps(cpx<T> *A, int ld, int ell, int c
       // vectors of different size (whose angles t are smaller than r), r t
       // between neighbours.
       const float far = fmaxf(rmax, kmax);
-      small_step = far <= kFloatApply;
-      near = kmax <= kStepMax;
+      small_step = far <= kFloatApply && k2 <= kFloatApply * kFloatApply;
+      near = k2 <= kStepMax * kStepMax;
       // far from converged: vectors that the float stage had left alone
       bulk = !small_step && rmax > 1e-3f && kmax > 0.3f && stages < kMaxStages;
       last = !bulk && rmax * far * 8.f <= tol;
@@ -887,39 +949,6 @@ struct LocalBond {
   }
 };
 
-// Sums of two values over the CTA in the arithmetic R (uniform result).
-template <typename R, int NT>
-__device__ __forceinline__ void block_sum2_in(R &a, R &b, double *red) {
-  R *r = reinterpret_cast<R *>(red);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a = a + shfl_xor(a, o);
-    b = b + shfl_xor(b, o);
-  }
-  __syncthreads();
-  if (lane == 0) {
-    r[warp] = a;
-    r[NT / 32 + warp] = b;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    a = lane < NT / 32 ? r[lane] : R(0);
-    b = lane < NT / 32 ? r[NT / 32 + lane] : R(0);
-#pragma unroll
-    for (int o = NT / 64; o > 0; o >>= 1) {
-      a = a + shfl_xor(a, o);
-      b = b + shfl_xor(b, o);
-    }
-    if (lane == 0) {
-      r[2 * (NT / 32)] = a;
-      r[2 * (NT / 32) + 1] = b;
-    }
-  }
-  __syncthreads();
-  a = r[2 * (NT / 32)];
-  b = r[2 * (NT / 32) + 1];
-}
 // f[0], f[1] = 1 / sqrt of the block's sums of a and b (in order: the same bits
 // for the same block).  terms: threads from this one on hold zeros; up to a
 // warp's worth need no second stage.

@@ -206,13 +206,40 @@ __device__ int float_sweeps(const Team &tm, cpx<float> *A32, int ell, cpx<float>
   return -1;
 }
 
+// Largest row sum of |M| (its leading parts), each row by a warp: the same on
+// teams of every size.  get(r, k): entry as cpx<float>.
+template <int NT, class FG>
+__device__ float team_row_sum(const Team &tm, int c, FG get, TeamWork &tw, int &slot, double *red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = NT / 32;
+  float most = 0.f;
+  for (int r = tm.rank * nw + warp; r < c; r += tm.size * nw) {
+    float s = 0.f;
+    for (int k = lane; k < c; k += 32) {
+      const cpx<float> v = get(r, k);
+      s += fabsf(v.x) + fabsf(v.y);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    most = s > most || s != s ? s : most;  // (NaN stays)
+  }
+  return team_max<NT>(tm, most, tw, slot, red);
+}
+
 // W (unit_entry) of S (c x c, Hermitian) in place of S, transposed: S[y][k] =
 // W[k][y], the rows that a product with W on the right takes.  The square from
-// 3 digits (a relative 2^-21 of |S1|^2 < 1e-8).  Scratch: the planes' memory.
+// 3 digits (a relative 2^-21 of its 1e-6 at the most), and where the square's
+// norm asks for it the next two terms, S1^2 (-5/16 S1 + 35/128 S1^2), too
+// (the matrices commute, so the product is Hermitian).  The norms are row sums
+// of S1^2, each by a warp: the same on teams of every size.  Returns false (S
+// spoilt) when the series does not reach: the terms left out are below 3/5 of
+// the norm of S1 to the third power (1e-15) or the fifth (5e-16).
+// Scratch: the planes' memory.
+constexpr float kTeamSquare = 1.2e-5f, kTeamMax = 1e-3f;
 template <int NT, typename S>
-__device__ void team_correction(const Team &tm, int c, TeamWork &tw, S &sm) {
+__device__ bool team_correction(const Team &tm, int c, TeamWork &tw, int &slot, S &sm) {
   const OzPlanes p = oz_planes(tw.plP, tw.exP, c, c, 3);
-  cpx<dd> *sq = reinterpret_cast<cpx<dd> *>(tw.plQ);
+  cpx<dd> *sq = reinterpret_cast<cpx<dd> *>(tw.plQ), *hi = sq;
+  float w2 = 0.375f;
   for (int k = tm.rank * NT + threadIdx.x; k < c; k += tm.size * NT) tw.dg[k] = dg_minus1(tw.S[size_t(k) * c + k].x);
   tm.sync();
   oz_split<NT, 3>(tm, p, c, [&](int r, int k) {
@@ -224,13 +251,45 @@ __device__ void team_correction(const Team &tm, int c, TeamWork &tw, S &sm) {
   tm.sync();
   oz_gemm<NT>(tm, p, p, true, 3, kOzHerm, sq, c, nullptr, sm);  // S1 S1^H
   tm.sync();
+  const float n2 = team_row_sum<NT>(
+      tm, c, [&](int r, int k) { return mkc<float>(sq[size_t(r) * c + k].x.hi, sq[size_t(r) * c + k].y.hi); }, tw, slot,
+      sm.red);
+  if (!(n2 <= kTeamMax * kTeamMax)) return false;
+  if (n2 > kTeamSquare * kTeamSquare) {
+    // planes of S1^2 behind it, those of the other factor and the result in the
+    // other buffer (each holds 8 planes of c rows; S1's own have served)
+    unsigned char *const after = reinterpret_cast<unsigned char *>(tw.plQ) + ((size_t(c) * c * sizeof(cpx<dd>) + 255) & ~size_t(255));
+    const OzPlanes a = oz_planes(after, tw.exQ, c, c, 3), b = oz_planes(tw.plP, tw.exP, c, c, 3);
+    hi = reinterpret_cast<cpx<dd> *>(reinterpret_cast<unsigned char *>(tw.plP) + ((3 * b.stride * 2 + 255) & ~size_t(255)));
+    w2 = 1.f;
+    oz_split<NT, 3>(tm, a, c, [&](int r, int k) { return sq[size_t(r) * c + k]; });
+    oz_split<NT, 3>(tm, b, c, [&](int r, int k) {
+      const cpx<dd> q = sq[size_t(r) * c + k];
+      cpx<float> v = mkc<float>(0.2734375f * q.x.hi, 0.2734375f * q.y.hi);
+      if (r != k) {
+        const cpx<dd> s = tw.S[size_t(r) * c + k];
+        const float g = -0.3125f * (1.f + tw.dg[r].hi) * (1.f + tw.dg[k].hi);
+        v = mkc<float>(fmaf(s.x.hi, g, v.x), fmaf(s.y.hi, g, v.y));
+      }
+      return mkc<dd>(dd(v.x), dd(v.y));
+    });
+    tm.sync();
+    oz_gemm<NT>(tm, a, b, true, 3, kOzHerm, hi, c, nullptr, sm);  // A B^H = S1^2 B
+    tm.sync();
+    for (int e = tm.rank * NT + threadIdx.x; e < c * c; e += tm.size * NT) {
+      const cpx<dd> q = sq[e], h = hi[e];
+      hi[e] = mkc<dd>(dd(fmaf(0.375f, q.x.hi, h.x.hi)), dd(fmaf(0.375f, q.y.hi, h.y.hi)));
+    }
+    tm.sync();
+  }
   // S[x][y] = conj(S[y][x]): entry (y, x) of W^T is W[x][y] with S[x][y] = conj of what is there
   for (int e = tm.rank * NT + threadIdx.x; e < c * c; e += tm.size * NT) {
     const int y = e / c, x = e - y * c;
     const cpx<dd> s = tw.S[e];
-    tw.S[e] = unit_entry(x == y, mkc<dd>(s.x, -s.y), tw.dg[x], tw.dg[y], mkc<float>(sq[e].x.hi, -sq[e].y.hi));
+    tw.S[e] = unit_entry(x == y, mkc<dd>(s.x, -s.y), tw.dg[x], tw.dg[y], mkc<float>(w2 * hi[e].x.hi, -w2 * hi[e].y.hi));
   }
   tm.sync();
+  return true;
 }
 
 // Powers of two near the norms of the columns of M (length ell): a product with
@@ -275,23 +334,14 @@ __device__ bool team_transform(const Team &tm, cpx<dd> *A, int ell, int c, bool 
   // S[p][q] = sum_k conj(X[k][p]) X[k][q]: planes by column serve both operands
   oz_gemm<NT>(tm, x, x, true, add ? 5 : 7, kOzHermT, tw.S, c, nullptr, sm);
   tm.sync();
-  float smax = 0.f, dmax = 0.f;
-  for (int e = tm.rank * NT + threadIdx.x; e < c * c; e += tm.size * NT) {
-    cpx<dd> v = tw.S[e];
-    if (e % (c + 1) == 0) {
-      if (!add) {
-        v.x = v.x - dd(1.f);
-        tw.S[e].x = v.x;
-      }
-      dmax = fmaxf(dmax, fabsf(v.x.hi));
-    } else {
-      smax = fmaxf(smax, fmaxf(fabsf(v.x.hi), fabsf(v.y.hi)));
-    }
-    if (!(v.x.hi == v.x.hi)) smax = __int_as_float(0x7f800000);
+  float dmax = 0.f;
+  for (int k = tm.rank * NT + threadIdx.x; k < c; k += tm.size * NT) {
+    dd &v = tw.S[size_t(k) * c + k].x;
+    if (!add) v = v - dd(1.f);
+    dmax = fabsf(v.hi) > dmax || v.hi != v.hi ? fabsf(v.hi) : dmax;
   }
-  smax = team_max<NT>(tm, smax, tw, slot, sm.red);
   dmax = team_max<NT>(tm, dmax, tw, slot, sm.red);
-  if (!(smax <= kOffMax && dmax <= kDiagMax)) return false;
+  if (!(dmax <= 0.1f)) return false;
   // B = A X (+ A): rows of A against the columns of X
   const OzPlanes pa = oz_planes(tw.plP, tw.exP, ell, c, add ? 6 : 8);
   if (add) {
@@ -305,7 +355,7 @@ __device__ bool team_transform(const Team &tm, cpx<dd> *A, int ell, int c, bool 
   tm.sync();
   oz_gemm<NT>(tm, pa, x, false, add ? 6 : 8, kOzTrans, tw.B, ell, add ? A : nullptr, sm);
   tm.sync();
-  team_correction<NT>(tm, c, tw, sm);
+  if (!team_correction<NT>(tm, c, tw, slot, sm)) return false;
   // A = B + B W; W below 1e-3, so six digits leave 1e-16 of every column
   team_scales<NT>(tm, tw.B, ell, c, tw);
   const OzPlanes pb = oz_planes(tw.plP, tw.exP, ell, c, 6), w = oz_planes(tw.plQ, tw.exQ, c, c, 6);
@@ -325,6 +375,7 @@ __device__ int svd_team(const Team &tm, cpx<dd> *A, int ell, int c, int max_swee
   const float floor_t = float(sweep_floor<dd>(ell));
   const float tol = float(4.0 * sqrt(double(ell)) * double(Eps<dd>::v));
   constexpr int kMaxStages = 3, kMaxSteps = 10;
+  constexpr float kSlight = 1e-7f;
   const int gthreads = tm.size * NT, gid = tm.rank * NT + threadIdx.x;
   int sweeps = 0, stages = 0, slot = 0;
   if (tm.rank == 0)
@@ -404,9 +455,14 @@ __device__ int svd_team(const Team &tm, cpx<dd> *A, int ell, int c, int max_swee
     ++sweeps;
     const float far = fmaxf(rmax, kmax);  // as svd_local
     const bool last = fine && rmax * far * 8.f <= tol;
-    if (far <= 1e-7f) {
+    // A += A K where the second order, which it leaves out, is below 2^-47
+    // (beyond, or where K's entries are not all small: with its unitary factor)
+    bool slight = far <= 1e-7f;
+    if (slight)
+      slight = team_row_sum<NT>(tm, c, [&](int r, int k) { return tw.V32[size_t(r) * c + k]; }, tw, slot, sm.red) <= kSlight;
+    if (slight) {
       team_scales<NT>(tm, A, ell, c, tw);
-      // A += A K: K below 1e-7, so four digits of both leave 1e-16
+      // K below 1e-7, so four digits of both leave 1e-16
       const OzPlanes k = oz_planes(tw.plQ, tw.exQ, c, c, 4), pa = oz_planes(tw.plP, tw.exP, ell, c, 4);
       oz_split<NT, 4>(tm, k, c, [&](int y, int p) {
         const cpx<float> v = tw.V32[size_t(y) * c + p];
