@@ -1593,10 +1593,8 @@ __device__ __forceinline__ int jacobi_svd_body(cpx<T> *__restrict__ A, int ell, 
   bool guided = kDD;
   const float tol_f = 4.f * sqrtf(float(ell)) * Eps<float>::v;
   constexpr float kGuidedDone = 1e-4f, kFinishDone = 1e-9f;
-  // Float: a sweep whose pairs were all below 3e-5 leaves ~1e-9 / gap, under
-  // the threshold (7e-7 to 1e-5) for relative gaps down to 1e-3, and is the last
-  // one.  Besides the confirming Gram pass this removes the sweep-limit hits:
-  // pairs whose rounding noise hovers about the threshold.
+  // Float: the last sweep is one by pair_far's rule; a further Gram pass would
+  // only confirm it.
   constexpr bool kFar = kDD || sizeof(T) == 4;
   // Columns with |a|^2 <= eps^2 ||A||_F^2 are rounding noise: rotating them
   // changes nothing above rounding and their relative off-diagonals never
@@ -1777,8 +1775,8 @@ __device__ __forceinline__ int jacobi_svd_body(cpx<T> *__restrict__ A, int ell, 
               act = pair_active<T>(sm.G[p * (W + 1) + p].x, sm.G[q * (W + 1) + q].x, sm.G[p * (W + 1) + q], tol,
                                    tiny2);
               if constexpr (sizeof(T) == 4)
-                farS |= int(pair_active<T>(sm.G[p * (W + 1) + p].x, sm.G[q * (W + 1) + q].x, sm.G[p * (W + 1) + q],
-                                           kFloatDone, tiny2));
+                farS |= int(pair_far(sm.G[p * (W + 1) + p].x, sm.G[q * (W + 1) + q].x, sm.G[p * (W + 1) + q], tol,
+                                     tiny2));
             }
           }
           if (act) {
@@ -2886,7 +2884,7 @@ __device__ __noinline__ void bond_team(const Team &tm, const TrajDev &tr, int k,
     if (tm.rank == 0)
       for (int i = tid; i < kTeamFlags; i += NT) tw.flag[i] = 0u;
     const long long t0 = clock64();
-    sw = float_sweeps<NT, W>(tm, wk.A, ell, nullptr, c, float(sweep_floor<float>(ell)), kFloatDone, max_sweeps, tw,
+    sw = float_sweeps<NT, W>(tm, wk.A, ell, nullptr, c, float(sweep_floor<float>(ell)), kLastWord, max_sweeps, tw,
                              slot, sm, cyc);
     cyc[1] += clock64() - t0;
   }

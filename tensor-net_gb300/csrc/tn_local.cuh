@@ -35,8 +35,21 @@
 
 namespace tn {
 
-// Float sweeps end after one whose pairs were all below this (see jacobi_svd).
+// Float sweeps that are the last word end after one whose pairs leave nothing
+// above the threshold (7e-7 to 1e-5): what a sweep leaves is of second order in
+// what it found, r r' between vectors of different size (below 1e-9 with every r
+// below kFloatDone) and r |t| between neighbours (r = |g| / (|a| |b|) before the
+// rotation by the angle t; in a cluster of nearly equal values t is near 1 however
+// small r is, and up to 2.6 times the threshold was left of a cluster of 128).
 constexpr float kFloatDone = 3e-5f;
+__device__ __forceinline__ bool pair_far(float a, float b, cpx<float> g, float tol, float tiny2) {
+  if (!(a > tiny2 && b > tiny2)) return false;
+  const float s = 1.f / (sqrtf(a) * sqrtf(b)), r = sqrtf(cabs2(g)) * s, d = fabsf(b - a) * s;
+  if (!(r > tol)) return false;
+  const float t = 2.f * r / (d + sqrtf(fmaf(d, d, 4.f * r * r)));
+  return r > kFloatDone || 8.f * r * t > tol;
+}
+constexpr float kLastWord = 0.f;  // `done` of such sweeps
 
 // ------------------------------------------------------------- arithmetic
 // Arithmetic of the sums that need more than float but not float64's
@@ -204,7 +217,7 @@ __device__ void gemm_exact_from(int M, int N, FK from, int K, FP P, FQ Q, FE E) 
 // (de Rijk); a pair belongs to LG lanes, which form the inner product and
 // apply the rotation to their elements.  Norms are carried by a' = a - t |g|,
 // b' = b + t |g| and recomputed each sweep.  Stops after a sweep without a
-// pair above `done` (before its rotation).  Returns the sweeps, -1 at the
+// pair above `done` (before its rotation), or by pair_far's rule (kLastWord).  Returns the sweeps, -1 at the
 // limit, -2 before a sweep whose sum of squared norms is below `least` or not
 // below kNormMax (a NaN or an infinity among them; the vectors are as the sweep
 // found them).
@@ -276,10 +289,14 @@ __device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<flo
             const float sc = __fdividef(1.f, a + b);
             const float hx = gx * sc, hy = gy * sc, as = a * sc, bs = b * sc;
             const float g2 = fmaf(hx, hx, hy * hy), ab = as * bs;
-            far |= int(g2 > done2 * ab);
+            if (done > kLastWord) far |= int(g2 > done2 * ab);
             if (g2 > tol2 * ab) {
               const float d = 0.5f * (bs - as), h2 = fmaf(d, d, g2), rh = rsqrt_near(h2);
               const float c2 = fmaf(0.5f * fabsf(d), rh, 0.5f), rc = rsqrt_near(c2), cs = c2 * rc;
+              if (done <= kLastWord) {  // pair_far, squared
+                const float r2 = __fdividef(g2, ab), t2 = (1.f - c2) * rc * rc;
+                far |= int(r2 > kFloatDone * kFloatDone || 64.f * r2 * t2 > tol2);
+              }
               const float w = copysignf(0.5f * rh * rc, d);
               const cpx<float> se = mkc<float>(hx * w, -hy * w);
               for (int i = l; i < ell; i += LG) {
@@ -692,7 +709,7 @@ __device__ __forceinline__ int svd_local_steps(cpx<T> *A, int ld, int ell, int c
     load();
     __syncthreads();
     const int sw = hestenes<NT>(As, pa, ell, nullptr, 0, c, nrm, ord, float(sweep_floor<float>(ell)), 0.f, tolf,
-                                fmaxf(tolf, kFloatDone), max_sweeps);
+                                kLastWord, max_sweeps);
     if (sw == -2) return -2;
     for (int idx = tid; idx < c * ell; idx += NT) {
       const int j = idx / ell, i = idx - j * ell;

@@ -83,7 +83,7 @@ __device__ float team_max(const Team &tm, float v, TeamWork &tw, int &slot, doub
 
 // One block-pair step of the float sweeps: the 32 columns cols of A32 (length
 // ell) are orthogonalised against each other, V32 (c rows, when set) follows.
-// rot / far: some pair was above the threshold / above kFloatDone.
+// rot / far: some pair was above the threshold / above `done` (kLastWord: by pair_far's rule).
 template <int NT, int W>
 __device__ void float_step(cpx<float> *A32, int ell, cpx<float> *V32, int c, const int *cols, float tol, float done,
                            float tiny2, int inner, int &rot, int &far, Smem<float, W> &sf) {
@@ -105,7 +105,7 @@ __device__ void float_step(cpx<float> *A32, int ell, cpx<float> *V32, int c, con
       const float a = sf.G[p * GP + p].x, b = sf.G[q * GP + q].x;
       const cpx<float> g = sf.G[p * GP + q];
       if (pair_active<float>(a, b, g, tol, tiny2)) need |= (p < B) != (q < B) ? 2 : 1;
-      if (pair_active<float>(a, b, g, done, tiny2)) need |= 4;
+      if (done > kLastWord ? pair_active<float>(a, b, g, done, tiny2) : pair_far(a, b, g, tol, tiny2)) need |= 4;
     }
   }
   const int w1 = __syncthreads_or(need & 1), w2 = __syncthreads_or(need & 2), w4 = __syncthreads_or(need & 4);
