@@ -3065,28 +3065,42 @@ __device__ __noinline__ void bond_team(const Team &tm, const TrajDev &tr, int k,
   tm.sync();
 }
 
-// local_probs (mps.rs:1079-1134): p_s = sum L_{k-1}[v]^2 |G[v,s,u]|^2 L_k[u]^2
+// Float states: a sum of probabilities within this of 1 differs from it by rounding.
+constexpr double kFloatSum = 1e-6;
+
+// local_probs (mps.rs:1079-1134): p_s = sum L_{k-1}[v]^2 |G[v,s,u]|^2 L_k[u]^2.
+// A float state's sum p_0 + p_1 differs from 1 by the rounding of its Gammas (a
+// certain outcome comes out at 1 +- 1e-7, and an impossible one could be drawn
+// when the other falls short of 1): the terms are summed in double-float there, and
+// a sum that close to 1 is divided out.  Reads, records and the projection take
+// the same values.  sum: p_0 + p_1 as it was.
 template <typename T, int NT, int W>
-__device__ void site_probs(const TrajDev &tr, int k, double &p0, double &p1, Smem<T, W> &sm) {
+__device__ void site_probs(const TrajDev &tr, int k, double &p0, double &p1, double &sum, Smem<T, W> &sm) {
+  using R = typename RedType<T>::type;
   const int cL = tr.chi[k], cR = tr.chi[k + 1];
   const cpx<T> *g = gamma_slot<T>(tr, k);
   const double *lamL = lam_slot(tr, k), *lamR = lam_slot(tr, k + 1);
-  // squared Lambdas in the working precision (shared scratch), per-thread
-  // partial sums in T, block reduction in float64
-  T *wl2 = reinterpret_cast<T *>(sm.r0), *wr2 = wl2 + cL;
+  // squared Lambdas (shared scratch) and per-thread partial sums in R, block
+  // reduction in float64
+  R *wl2 = reinterpret_cast<R *>(sm.r0), *wr2 = wl2 + cL;
   __syncthreads();
-  for (int v = threadIdx.x; v < cL; v += NT) wl2[v] = T(lamL[v] * lamL[v]);
-  for (int u = threadIdx.x; u < cR; u += NT) wr2[u] = T(lamR[u] * lamR[u]);
+  for (int v = threadIdx.x; v < cL; v += NT) wl2[v] = R(lamL[v] * lamL[v]);
+  for (int u = threadIdx.x; u < cR; u += NT) wr2[u] = R(lamR[u] * lamR[u]);
   __syncthreads();
-  T b0 = T(0), b1 = T(0);
+  R b0 = R(0), b1 = R(0);
   const int tot = cL * 2 * cR;
   for (int idx = threadIdx.x; idx < tot; idx += NT) {
     int u = idx % cR, s = (idx / cR) & 1, v = idx / (2 * cR);
-    T w = cabs2(g[idx]) * wl2[v] * wr2[u];
+    R w = cabs2(widen(g[idx])) * wl2[v] * wr2[u];
     if (s) b1 += w; else b0 += w;
   }
   double a0 = double(b0), a1 = double(b1);
   block_sum2<NT>(a0, a1, sm.red);
+  sum = a0 + a1;
+  if (sizeof(T) == 4 && fabs(sum - 1.0) <= kFloatSum) {
+    a0 /= sum;
+    a1 /= sum;
+  }
   p0 = a0;
   p1 = a1;
 }
@@ -3095,23 +3109,21 @@ __device__ void site_probs(const TrajDev &tr, int k, double &p0, double &p1, Sme
 template <typename T, int NT, int W>
 __device__ void measure_site(const TrajDev &tr, int k, double u, int post, int *out_outcome, double *out_prob,
                              Smem<T, W> &sm) {
-  double p0, p1;
-  site_probs<T, NT, W>(tr, k, p0, p1, sm);
+  double p0, p1, sum;
+  site_probs<T, NT, W>(tr, k, p0, p1, sum, sm);
   int outcome;
   if (post >= 0)
     outcome = post;
   else
     outcome = (u < p0) ? 0 : 1;
   const double prob = outcome ? p1 : p0;
-  const double sum = p0 + p1;
   if (threadIdx.x == 0) {
     if (tr.stats) {
       atomicAdd(tr.stats + STAT_MEAS, 1.0);
       atomicAdd(tr.stats + STAT_BYTES, double(sizeof(cpx<T>)) * 2.0 * 2.0 * tr.chi[k] * tr.chi[k + 1]);
     }
     if (out_outcome) *out_outcome = outcome;
-    // (a certain outcome's float sum can come out one unit above 1)
-    if (out_prob) *out_prob = sizeof(T) == 4 && prob > 1.0 && prob < 1.0 + 1e-6 ? 1.0 : prob;
+    if (out_prob) *out_prob = prob;
     const double ptol = (sizeof(T) == 8) ? 1e-9 : 1e-4;
     if (!(fabs(sum - 1.0) <= ptol)) atomicOr(tr.status, ST_PROB_SUM);
   }
@@ -3214,8 +3226,8 @@ __device__ void run_program(const Team &tm, const LaunchArgs &la, const Instr *p
         if (tm.size > 1) tm.sync();
         break;
       case OP_PROBS: {
-        double p0, p1;
-        site_probs<T, NT, W>(tr, in.k, p0, p1, sm);
+        double p0, p1, sum;
+        site_probs<T, NT, W>(tr, in.k, p0, p1, sum, sm);
         if (threadIdx.x == 0 && tm.rank == 0) {
           la.pout[2 * in.a] = p0;
           la.pout[2 * in.a + 1] = p1;

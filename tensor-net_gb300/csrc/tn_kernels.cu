@@ -340,8 +340,8 @@ __global__ void __launch_bounds__(kObserveThreads) k_observe(const TrajDev *traj
   Smem<T, kBlockW> sm(osm, 1);
   const TrajDev tr = *traj;
   if (op == OP_PROBS) {
-    double p0, p1;
-    site_probs<T, kObserveThreads, kBlockW>(tr, k, p0, p1, sm);
+    double p0, p1, sum;
+    site_probs<T, kObserveThreads, kBlockW>(tr, k, p0, p1, sum, sm);
     if (threadIdx.x == 0) {
       out[0] = p0;
       out[1] = p1;
@@ -375,14 +375,14 @@ __global__ void __launch_bounds__(kObserveThreads) k_unitary1(const TrajDev *tra
 template <typename T>
 static cudaError_t launch_observe_t(const TrajDev *traj, int cap, int op, int k, double alpha, double *out,
                                     cudaStream_t st) {
-  // site_probs keeps the squared Lambdas of both bonds in shared memory
-  const size_t smem = SmemLayout<T, kBlockW>::head_bytes + 2 * size_t(cap) * sizeof(T);
+  // site_probs keeps the squared Lambdas of both bonds in shared memory (8 bytes each)
+  const size_t smem = SmemLayout<T, kBlockW>::head_bytes + 2 * size_t(cap) * 8;
   if (smem > 48 * 1024) return cudaErrorInvalidValue;
   k_observe<T><<<1, kObserveThreads, smem, st>>>(traj, op, k, alpha, out);
   return cudaGetLastError();
 }
 
-bool observe_fits(int prec, int cap) { return 2048 + 2 * size_t(cap) * (prec == 1 ? 4 : 8) <= 48 * 1024; }
+bool observe_fits(int, int cap) { return 2048 + 2 * size_t(cap) * 8 <= 48 * 1024; }
 
 cudaError_t launch_observe(int prec, const TrajDev *traj, int cap, int op, int k, double alpha, double *out,
                            cudaStream_t st) {
