@@ -330,24 +330,26 @@ int run_blocks_per_sm(int prec, int sortP) {
 // its arguments arrive by value, so a read is one launch and one copy back
 // instead of four copies in, a launch of the whole executor and a copy back
 // (an entropy, a Renyi entropy and the site probabilities of one state: 99 us
-// through the executor, 78 us here).  Bound by launch and copy latency.
-constexpr int kObserveThreads = 256;
+// through the executor, 78 us here).  Bound by launch and copy latency; the
+// probabilities of a wide site by the loads that one SM has in flight (chi = 1024,
+// df: 735 us in the executor, 1160 us on 256 threads, 360 us on 1024), while an
+// entropy of a few hundred values takes longer on more threads.
+constexpr int kObserveThreads = 256, kProbsThreads = 1024;
 
-template <typename T>
-__global__ void __launch_bounds__(kObserveThreads) k_observe(const TrajDev *traj, int op, int k, double alpha,
-                                                             double *out) {
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT) k_observe(const TrajDev *traj, int op, int k, double alpha, double *out) {
   extern __shared__ __align__(256) unsigned char osm[];
   Smem<T, kBlockW> sm(osm, 1);
   const TrajDev tr = *traj;
   if (op == OP_PROBS) {
     double p0, p1, sum;
-    site_probs<T, kObserveThreads, kBlockW>(tr, k, p0, p1, sum, sm);
+    site_probs<T, NT, kBlockW>(tr, k, p0, p1, sum, sm);
     if (threadIdx.x == 0) {
       out[0] = p0;
       out[1] = p1;
     }
   } else {
-    const double e = bond_entropy<kObserveThreads>(tr, k, alpha, sm.red);
+    const double e = bond_entropy<NT>(tr, k, alpha, sm.red);
     if (threadIdx.x == 0) out[0] = e;
   }
 }
@@ -378,7 +380,10 @@ static cudaError_t launch_observe_t(const TrajDev *traj, int cap, int op, int k,
   // site_probs keeps the squared Lambdas of both bonds in shared memory (8 bytes each)
   const size_t smem = SmemLayout<T, kBlockW>::head_bytes + 2 * size_t(cap) * 8;
   if (smem > 48 * 1024) return cudaErrorInvalidValue;
-  k_observe<T><<<1, kObserveThreads, smem, st>>>(traj, op, k, alpha, out);
+  if (op == OP_PROBS)
+    k_observe<T, kProbsThreads><<<1, kProbsThreads, smem, st>>>(traj, op, k, alpha, out);
+  else
+    k_observe<T, kObserveThreads><<<1, kObserveThreads, smem, st>>>(traj, op, k, alpha, out);
   return cudaGetLastError();
 }
 

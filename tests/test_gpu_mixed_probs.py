@@ -52,3 +52,25 @@ def test_sum_far_from_one_is_reported_as_it_is(pkg):
     np.testing.assert_allclose(m.probs(1), [0.36, 0.81], atol=1e-7)
     m.measure_prob(1, 0.1)
     assert m.device_status() != 0
+
+
+@pytest.mark.parametrize("prec,tol", [("f64", 1e-13), ("df", 1e-12), ("mixed", 1e-5)])
+@pytest.mark.parametrize("dims", [(1, 1), (1, 2), (2, 3), (3, 1), (5, 17), (33, 16), (31, 32), (16, 33), (70, 65),
+                                  (128, 200), (300, 1)])
+def test_sums_over_every_shape_of_a_site(pkg, prec, dims, tol):
+    """Rows of 1 to 200 entries on groups of 1 to 32 lanes, in the read and in the
+    measurement, against numpy; the tolerance is the mode's rounding of a sum of
+    squares."""
+    cl, cr = dims
+    rng = np.random.default_rng(cl * 1000 + cr)
+    g = [rng.standard_normal((a, 2, b)) + 1j * rng.standard_normal((a, 2, b)) for a, b in ((1, cl), (cl, cr), (cr, 1))]
+    lam = [rng.random(cl) + 0.1, rng.random(cr) + 0.1]
+    w = np.abs(g[1]) ** 2 * (lam[0] ** 2)[:, None, None] * (lam[1] ** 2)[None, None, :]
+    g[1] /= np.sqrt(w.sum())
+    p = w.sum((0, 2)) / w.sum()
+    g += [np.eye(1, 2).reshape(1, 2, 1).astype(complex)] * 15  # (a chain long enough for such bonds)
+    lam += [np.ones(1)] * 15
+    m = pkg.MPS.from_parts(g, lam, None, prec, chi_cap=max(dims))
+    np.testing.assert_allclose(m.probs(1), p, atol=tol)
+    o, pr = m.clone().measure_prob(1, 0.3)
+    assert o == (0 if 0.3 < p[0] else 1) and abs(pr - p[o]) < tol
