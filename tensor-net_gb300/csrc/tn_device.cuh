@@ -3146,22 +3146,6 @@ __device__ void measure_site(const TrajDev &tr, int k, double u, int post, int *
   __syncthreads();
 }
 
-// apply_unitary1 (mps.rs:1298-1314): Gamma_k[v,:,u] <- op Gamma_k[v,:,u]
-template <typename T, int NT, int W>
-__device__ void unitary1(const TrajDev &tr, int k, const double *op) {
-  const int cL = tr.chi[k], cR = tr.chi[k + 1];
-  cpx<T> *g = gamma_slot<T>(tr, k);
-  cpx<T> o00 = mkc<T>(T(op[0]), T(op[1])), o01 = mkc<T>(T(op[2]), T(op[3]));
-  cpx<T> o10 = mkc<T>(T(op[4]), T(op[5])), o11 = mkc<T>(T(op[6]), T(op[7]));
-  for (int idx = threadIdx.x; idx < cL * cR; idx += NT) {
-    int v = idx / cR, u = idx % cR;
-    cpx<T> a = g[(v * 2 + 0) * cR + u], b = g[(v * 2 + 1) * cR + u];
-    g[(v * 2 + 0) * cR + u] = cfma(o01, b, cmul(o00, a));
-    g[(v * 2 + 1) * cR + u] = cfma(o11, b, cmul(o10, a));
-  }
-  __syncthreads();
-}
-
 // entropy_vn (mps.rs:1251-1261) / entropy_ry_schmidt (1268-1282), float64
 template <int NT>
 __device__ double bond_entropy(const TrajDev &tr, int b, double alpha, double *red) {
@@ -3229,10 +3213,6 @@ __device__ void run_program(const Team &tm, const LaunchArgs &la, const Instr *p
         __syncthreads();
         break;
       }
-      case OP_UNI1:
-        if (tm.rank == 0) unitary1<T, NT, W>(tr, in.k, la.gates + size_t(in.a) * 32);
-        if (tm.size > 1) tm.sync();
-        break;
       case OP_PROBS: {
         double p0, p1, sum;
         site_probs<T, NT, W>(tr, in.k, p0, p1, sum, sm);

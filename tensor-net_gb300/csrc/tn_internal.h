@@ -18,9 +18,8 @@ enum Opcode : int {
   OP_REFACTOR = 2,  // k                          local_refactor (mps.rs:846)
   OP_MEAS = 3,      // k, a = slot, b = post|-1   sample_state+project (mps.rs:1427-1465)
   OP_ENTROPY = 4,   // k = bond, a = slot         entropy_vn (mps.rs:1251)
-  OP_UNI1 = 5,      // k, a = gate index          apply_unitary1 (mps.rs:1298)
-  OP_PROBS = 6,     // k, a = slot                local_probs (mps.rs:1079)
-  OP_RENYI = 7      // k = bond, a = slot, b = index of alpha in us[]  entropy_ry_schmidt (mps.rs:1268)
+  OP_PROBS = 5,     // k, a = slot                local_probs (mps.rs:1079)
+  OP_RENYI = 6      // k = bond, a = slot, b = index of alpha in us[]  entropy_ry_schmidt (mps.rs:1268)
 };
 
 struct Instr {

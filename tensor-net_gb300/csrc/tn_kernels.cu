@@ -354,6 +354,7 @@ __global__ void __launch_bounds__(NT) k_observe(const TrajDev *traj, int op, int
   }
 }
 
+// apply_unitary1 (mps.rs:1298-1314): Gamma_k[v,:,u] <- op Gamma_k[v,:,u]
 struct Op1 {
   double v[8];
 };
