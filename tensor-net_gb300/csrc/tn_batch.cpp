@@ -336,9 +336,10 @@ int launch_step(tn_batch *b, uint32_t nt, const StepPtrs &P0, bool timed = true)
     // A layer lasts as long as its heaviest trajectory's refactor chain. With at
     // most one trajectory an SM, and bonds wide enough for operations that a
     // cluster shares (beyond chi = 64), clusters of CTAs shorten that chain by
-    // more than the idle members cost on narrow bonds: 152 trajectories at n =
-    // 16, chi = 128, two layers: 210 -> 105 ms.  Beyond that the SMs have trajectories of their own.
-    // The results have the same bits either way.
+    // more than the idle members cost on narrow bonds (152 trajectories at n =
+    // 16, chi = 128, two layers: 110 ms, and 210 ms on single CTAs).  With more
+    // trajectories the SMs have chains of their own.  The results have the same
+    // bits either way.
     int grid = gmax;
     if (b->prec == TN_PREC_DF && b->grid_limit == 0 && P.chi_hint > 64 && nt <= uint32_t(b->sms)) {
       const int size = nt <= uint32_t(b->sms) / 8 ? 8 : 4;

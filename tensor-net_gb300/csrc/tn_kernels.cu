@@ -294,11 +294,17 @@ size_t run_team_bytes(int prec, int cap) {
   return prec == 0 ? run_team_f64(cap) : (prec == 2 ? run_team_df(cap) : run_team_f32(cap));
 }
 
-int DeviceMem::alloc(void **p, size_t bytes) {
+namespace {
+struct OutsideCaptures {
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  cudaThreadExchangeStreamCaptureMode(&mode);
+  OutsideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~OutsideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+}  // namespace
+
+int DeviceMem::alloc(void **p, size_t bytes) {
+  OutsideCaptures relaxed;
   const cudaError_t e = cudaMalloc(p, bytes);
-  cudaThreadExchangeStreamCaptureMode(&mode);
   if (e != cudaSuccess) {
     *p = nullptr;
     (void)cudaGetLastError();
@@ -306,7 +312,10 @@ int DeviceMem::alloc(void **p, size_t bytes) {
   return int(e);
 }
 
-void DeviceMem::free(void *p) { (void)cudaFree(p); }
+void DeviceMem::free(void *p) {
+  OutsideCaptures relaxed;
+  (void)cudaFree(p);
+}
 
 size_t DeviceMem::available() {
   size_t avail = 0, total = 0;

@@ -15,8 +15,9 @@
 //  3. refinement: the Gram matrix of A in the working precision gives every
 //     remaining rotation at once, tan(theta) = t for each pair as in a Jacobi
 //     rotation; I + K with K_qp = -t e, K_pq = t conj(e) is made unitary (by a
-//     short series while t is small, unitary_step; else as in 2) and applied.  The off-diagonals fall quadratically; two steps
-//     usually reach the working precision's threshold.
+//     short series while K is small, unitary_step; else as in 2) and applied.
+//     The off-diagonals fall quadratically; two steps usually reach the working
+//     precision's threshold.
 //
 // The sweeps of 1 are the many, cheap ones; the working precision pays for two
 // or three products instead of every rotation of every sweep.  Pairs that are
@@ -24,13 +25,13 @@
 // small); svd_local then reports so and the caller goes on with the block
 // Jacobi on the (already unitarily transformed) vectors.
 //
-// Code size counts: an operation of a few vectors runs most of its code once,
-// and with the sums unrolled four or eight times and one copy per call the warps
-// waited for instructions a third of the time that they were not at a barrier
-// (46 % of the instruction cache's requests missed).  So one copy of every
-// product, rolled loops where a loop is short, and unrolling only inside the
-// float sweeps: 304 trajectories at n = 64 101 -> 84 ms, with the counters by
-// one warp and shorter butterflies 76 ms; bonds of 16 and more vectors as before.
+// Code size counts: an operation of a few vectors runs most of its code once.
+// Sums unrolled four or eight times, with a copy per call, leave the warps
+// waiting for instructions a third of the time that they are not at a barrier
+// (46 % of the instruction cache's requests miss) and cost a quarter of such
+// batches' time (304 trajectories at n = 64: 101 against 84 ms).  So one copy of
+// every product, rolled loops where a loop is short, and unrolling only inside
+// the float sweeps, where bonds of 16 and more vectors need it (5 %).
 #pragma once
 
 namespace tn {
