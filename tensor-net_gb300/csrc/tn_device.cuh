@@ -3072,8 +3072,8 @@ constexpr double kFloatSum = 1e-6;
 // A float state's sum p_0 + p_1 differs from 1 by the rounding of its Gammas (a
 // certain outcome comes out at 1 +- 1e-7, and an impossible one could be drawn
 // when the other falls short of 1): a sum that close to 1 is divided out.  (Its
-// rows are summed in double-float, a lane's part of a row in float.)  Reads, records and the
-// projection take the same values.  sum: p_0 + p_1 as it was.
+// rows are summed in double-float, a lane's part of a row in float.)  Reads,
+// records and the projection take the same values.  sum: p_0 + p_1 as it was.
 // A row (v, s) belongs to as many lanes as it has entries, up to a warp: no
 // division per entry, which is what one CTA's time on a wide bond went to.
 template <typename T, int NT, int W>
@@ -3082,12 +3082,12 @@ __device__ void site_probs(const TrajDev &tr, int k, double &p0, double &p1, dou
   const int cL = tr.chi[k], cR = tr.chi[k + 1];
   const cpx<T> *g = gamma_slot<T>(tr, k);
   const double *lamL = lam_slot(tr, k), *lamR = lam_slot(tr, k + 1);
-  // squared Lambdas (shared scratch) and partial sums in R, block reduction in
-  // float64
-  R *wl2 = reinterpret_cast<R *>(sm.r0), *wr2 = wl2 + cL;
+  // squared Lambdas in the working precision (shared scratch), sums of rows in
+  // R, block reduction in float64
+  T *wl2 = reinterpret_cast<T *>(sm.r0), *wr2 = wl2 + cL;
   __syncthreads();
-  for (int v = threadIdx.x; v < cL; v += NT) wl2[v] = R(lamL[v] * lamL[v]);
-  for (int u = threadIdx.x; u < cR; u += NT) wr2[u] = R(lamR[u] * lamR[u]);
+  for (int v = threadIdx.x; v < cL; v += NT) wl2[v] = T(lamL[v] * lamL[v]);
+  for (int u = threadIdx.x; u < cR; u += NT) wr2[u] = T(lamR[u] * lamR[u]);
   __syncthreads();
   R b0 = R(0), b1 = R(0);
   const int lb = cR > 16 ? 5 : (cR > 1 ? 32 - __clz(cR - 1) : 0);
@@ -3095,8 +3095,8 @@ __device__ void site_probs(const TrajDev &tr, int k, double &p0, double &p1, dou
     const cpx<T> *gr = g + size_t(row) * cR;
     T s = T(0);
 #pragma unroll 8
-    for (int u = threadIdx.x & ((1 << lb) - 1); u < cR; u += 1 << lb) s += cabs2(gr[u]) * T(wr2[u]);
-    const R w = R(s) * wl2[row >> 1];
+    for (int u = threadIdx.x & ((1 << lb) - 1); u < cR; u += 1 << lb) s += cabs2(gr[u]) * wr2[u];
+    const R w = R(s) * R(wl2[row >> 1]);
     if (row & 1)
       b1 += w;
     else

@@ -387,8 +387,8 @@ __global__ void __launch_bounds__(kObserveThreads) k_unitary1(const TrajDev *tra
 template <typename T>
 static cudaError_t launch_observe_t(const TrajDev *traj, int cap, int op, int k, double alpha, double *out,
                                     cudaStream_t st) {
-  // site_probs keeps the squared Lambdas of both bonds in shared memory (8 bytes each)
-  const size_t smem = SmemLayout<T, kBlockW>::head_bytes + 2 * size_t(cap) * 8;
+  // site_probs keeps the squared Lambdas of both bonds in shared memory
+  const size_t smem = SmemLayout<T, kBlockW>::head_bytes + 2 * size_t(cap) * sizeof(T);
   if (smem > 48 * 1024) return cudaErrorInvalidValue;
   if (op == OP_PROBS)
     k_observe<T, kProbsThreads><<<1, kProbsThreads, smem, st>>>(traj, op, k, alpha, out);
@@ -397,7 +397,7 @@ static cudaError_t launch_observe_t(const TrajDev *traj, int cap, int op, int k,
   return cudaGetLastError();
 }
 
-bool observe_fits(int, int cap) { return 2048 + 2 * size_t(cap) * 8 <= 48 * 1024; }
+bool observe_fits(int prec, int cap) { return 2048 + 2 * size_t(cap) * (prec == 1 ? 4 : 8) <= 48 * 1024; }
 
 cudaError_t launch_observe(int prec, const TrajDev *traj, int cap, int op, int k, double alpha, double *out,
                            cudaStream_t st) {

@@ -218,10 +218,10 @@ __device__ void gemm_exact_from(int M, int N, FK from, int K, FP P, FQ Q, FE E) 
 // (de Rijk); a pair belongs to LG lanes, which form the inner product and
 // apply the rotation to their elements.  Norms are carried by a' = a - t |g|,
 // b' = b + t |g| and recomputed each sweep.  Stops after a sweep without a
-// pair above `done` (before its rotation), or by pair_far's rule (kLastWord).  Returns the sweeps, -1 at the
-// limit, -2 before a sweep whose sum of squared norms is below `least` or not
-// below kNormMax (a NaN or an infinity among them; the vectors are as the sweep
-// found them).
+// pair above `done` (before its rotation), or by pair_far's rule (kLastWord).
+// Returns the sweeps, -1 at the limit, -2 before a sweep whose sum of squared
+// norms is below `least` or not below kNormMax (a NaN or an infinity among them;
+// the vectors are as the sweep found them).
 constexpr float kNormMax = 1e30f, kNormTiny = 1e-37f;
 template <int NT>
 __device__ __forceinline__ int hestenes(cpx<float> *As, int pa, int ell, cpx<float> *Vs, int pv, int c, float *nrm, int *ord,
@@ -499,8 +499,9 @@ __device__ __noinline__ bool unitarise(cpx<float> *Vs, int pv, int c, cpx<dd> *S
 // float, K[x][y] = Vs[y * pv + x] off the diagonal, of Frobenius norm at most
 // kStepMax.  (I + K)(I - K^2)^(-1/2) = I + K + K^2 / 2 + K^3 / 2 + 3/8 K^4 +
 // 3/8 K^5 ...: K is exact, K^2 is summed in double-float, what follows is below
-// 5e-10, so floats do, and what is left out is below 4e-16.  Two passes instead of unitarise's five and its maxima: a third of
-// its time.  Y: c x c of scratch for K^2.
+// 5e-10, so floats do, and what is left out is below 4e-16.  Two passes instead
+// of unitarise's five and its sums: a third of its time.  Y: c x c of scratch
+// for K^2.
 constexpr float kStepMax = 1e-3f;
 template <typename T, int NT>
 __device__ __noinline__ void unitary_step(const cpx<float> *Vs, int pv, int c, cpx<dd> *Y, int py, cpx<T> *Q, int pq) {
