@@ -148,9 +148,11 @@ int tn_mps_apply_unitary2(tn_mps *m, uint32_t k, const double *op,
 /* apply_unitary2 without any device allocation.  No counterpart in the
  * reference: for callers that cannot allocate device memory when they apply
  * a gate (a fixed memory plan that forbids allocation after start-up, or
- * work around a CUDA graph capture).  Same arguments and result as
- * tn_mps_apply_unitary2 (a non-finite gate entry is TN_ERR_INVALID_ARG);
- * the bond operation's scratch is a fixed 4.5 MiB device array shared by
+ * work around a CUDA graph capture).  Same arguments as
+ * tn_mps_apply_unitary2 (a non-finite gate entry is TN_ERR_INVALID_ARG) and
+ * the same result to the mode's rounding, on one CTA: several times slower
+ * on double-float bonds wider than 32.
+ * The bond operation's scratch is a fixed 4.5 MiB device array shared by
  * every call: handles with a chi capacity above 270 in mixed precision or
  * above 191 in float64 / double-float are rejected with TN_ERR_CAPACITY.
  * Calls that overlap on the GPU race on that array: order them on one
